@@ -112,9 +112,10 @@ struct MetadataParams {
   // the dispatch into an empty one and records kStatusOverflow / kStatusRegionMismatch.
   int region_id;                 // -1: exact mode
   int tiles_cap, recv_cap;
-  int* dev_sizes;                // [4] device: total_tiles, num_recv_tokens, overflow flag, reserved (capacity mode)
+  int* dev_sizes;                // [4] device: total_tiles, num_recv_tokens, overflow flag, pairs of row tiles (capacity mode)
   int* tile_id_to_expert;        // [tiles_cap] filled by the materialise launch in capacity mode
   int* pool_arrival_target;      // [tiles_cap]
+  int* pair_tiles;               // [tiles_cap] row tiles two by two, see GemmParams::pair_tiles; dev_sizes[3] counts the live pairs
   HostOverflow* host_overflow;   // mapped pinned memory: where the host learns of an overflow without a sync
 };
 void launch_dispatch_metadata(const MetadataParams& p, cudaStream_t stream);
@@ -125,6 +126,7 @@ struct FillParams {
   const int* expert_pool_block_offset;
   int* tile_id_to_expert;
   int* pool_arrival_target;
+  int* pair_tiles;             // (exact mode) row tiles two by two, see GemmParams::pair_tiles
   int* pool_arrival_count;
   int* pool_recv_token;        // -> -1
   int* pool_k_slot;            // -> -1
@@ -230,6 +232,11 @@ void launch_pool_compress(const void* pool, void* recv, const int* pool_recv_tok
 void launch_pool_expand(const void* recv, void* pool, const int* pool_recv_token, int tk_padded,
                         int hidden, cudaStream_t stream);
 
+// Zeroes the rows of both pools between an expert's length and the next multiple of 64: the weight-gradient GEMM of CTA
+// pairs multiplies whole 64-row blocks.
+void launch_zero_pool_padding(void* pool_a, void* pool_b, const int* expert_frequency, const int* expert_pool_block_offset,
+                              int num_experts, int hidden, cudaStream_t stream);
+
 // out[t, :] += sum over the pairs (t, k) owned by OTHER ranks of rows[t * K + k, :], accumulated in fp32.
 // Second half of the fused combine: expert ranks store one bf16 row per remote (token, k) pair into the
 // source rank's `rows`; pairs owned by the source rank itself were already reduced into `out`.
@@ -280,6 +287,10 @@ struct GemmParams {
   int mode, epilogue;
   int block_n;                   // 128 or 256
   int a_mn_major, b_mn_major;
+  int pair_ctas;                 // 1: a cluster of two CTAs per pair of row tiles (block_n 256 only).  VarlenM: num_m_tiles and
+                                 // num_m_tiles_dev then count pairs; VarlenK: num_m_tiles counts 256-row units, and the rows of
+                                 // both operands past an expert's length, up to a multiple of 64, must hold zeros
+  const int* pair_tiles;         // VarlenM, pair_ctas: [pairs] first row tile * 2 + (1: the next tile is the same expert's too)
   int N;                         // output columns (per expert)
   int K;                         // reduction length (VarlenM)
   int M_out;                     // output rows per expert (VarlenK)
@@ -353,6 +364,5 @@ constexpr int kTimingCols = 12;
 bool launch_grouped_gemm(const GemmParams& p, const void* tmap_a, const void* tmap_b, const void* tmap_o0,
                          const void* tmap_o1, const PushParams* fused_push, int num_ctas, cudaStream_t stream,
                          cudaError_t* setup_error = nullptr, const void* maps2 = nullptr);
-size_t grouped_gemm_smem_bytes(int block_n);
 
 }  // namespace sep

@@ -60,6 +60,16 @@ __device__ __forceinline__ int warp_excl_scan(int v, int lane, int& total) {
   return x - v;
 }
 
+// Pairs of row tiles (units of the CTA-pair GEMM): tiles 2i and 2i + 1 of an expert, an odd last tile on its own.  Tile `t`
+// of expert `e` writes its pair when it is the first of it; pairs are numbered in pool order.
+__device__ __forceinline__ void store_pair(int* pair_tiles, const int* block_offset, int e, int t) {
+  const int j = t - block_offset[e];
+  if (j & 1) return;
+  int before = 0;
+  for (int i = 0; i < e; ++i) before += (block_offset[i + 1] - block_offset[i] + 1) / 2;
+  pair_tiles[before + j / 2] = t * 2 + (t + 1 < block_offset[e + 1] ? 1 : 0);
+}
+
 __global__ void __launch_bounds__(kMetaThreads, 1) dispatch_metadata_kernel(const MetadataParams p) {
   __shared__ int s_hist[kMaxExperts];          // phase A: running per-expert count; phase B: freq
   __shared__ int s_off[kMaxExperts];           // phase B: tile offset of each expert inside its owner
@@ -95,6 +105,7 @@ __global__ void __launch_bounds__(kMetaThreads, 1) dispatch_metadata_kernel(cons
         }
         p.tile_id_to_expert[t] = e;
         p.pool_arrival_target[t] = target;
+        if (static_cast<int>(t) < live) store_pair(p.pair_tiles, p.expert_pool_block_offset, e, static_cast<int>(t));
       }
       if (p.dev_sizes[2] != 0) {   // the dispatch was turned into an empty one: nothing is sent anywhere
         for (size_t i = gid; i < static_cast<size_t>(T) * K; i += gsz) p.pair_slot[i] = -1;
@@ -283,7 +294,7 @@ __global__ void __launch_bounds__(kMetaThreads, 1) dispatch_metadata_kernel(cons
       report_note(p.status, (s_bad & 2) ? kStatusRegionMismatch : kStatusOverflow, kKernelMetadata, 1, p.rank,
                   p.region_id, (s_bad & 2) ? p.region_id : p.tiles_cap, need_tiles);
       *p.num_send = 0;
-      if (p.dev_sizes != nullptr) { p.dev_sizes[0] = 0; p.dev_sizes[1] = 0; p.dev_sizes[2] = 1; }
+      if (p.dev_sizes != nullptr) { p.dev_sizes[0] = 0; p.dev_sizes[1] = 0; p.dev_sizes[2] = 1; p.dev_sizes[3] = 0; }
       if (p.host_overflow != nullptr) {
         p.host_overflow->needed_tiles = need_tiles;
         p.host_overflow->needed_recv = need_recv;
@@ -314,7 +325,11 @@ __global__ void __launch_bounds__(kMetaThreads, 1) dispatch_metadata_kernel(cons
     int recv = 0;
     for (int s = 0; s < R; ++s) recv += s_U[s][p.rank];
     if (host_polls) { p.host->total_tiles = s_total_tiles[p.rank]; p.host->num_recv_tokens = recv; }
-    if (p.dev_sizes != nullptr) { p.dev_sizes[0] = s_total_tiles[p.rank]; p.dev_sizes[1] = recv; p.dev_sizes[2] = 0; }
+    if (p.dev_sizes != nullptr) {
+      int pairs = 0;
+      for (int el = 0; el < EL; ++el) pairs += ((s_hist[p.rank * EL + el] + p.tile_m - 1) / p.tile_m + 1) / 2;
+      p.dev_sizes[0] = s_total_tiles[p.rank]; p.dev_sizes[1] = recv; p.dev_sizes[2] = 0; p.dev_sizes[3] = pairs;
+    }
   }
   __syncthreads();
   if (tid == 0 && host_polls) {
@@ -494,6 +509,7 @@ __global__ void fill_tile_metadata_kernel(const FillParams p) {
       const int j = t - p.expert_pool_block_offset[e];
       p.tile_id_to_expert[t] = e;
       p.pool_arrival_target[t] = min(p.tile_m, p.expert_frequency[e] - j * p.tile_m);
+      store_pair(p.pair_tiles, p.expert_pool_block_offset, e, t);
     }
     p.pool_arrival_count[t] = 0;
   }
@@ -776,6 +792,19 @@ void launch_pool_expand(const void* recv, void* pool, const int* pool_recv_token
   const int grid = min((tk_padded + 7) / 8, sm_count() * 8);
   pool_rows_kernel<false><<<grid, 256, 0, stream>>>(static_cast<const char*>(recv), static_cast<char*>(pool),
                                                     pool_recv_token, tk_padded, hidden);
+}
+
+__global__ void zero_pool_padding_kernel(char* a, char* b, const int* freq, const int* block_offset, int vecs) {
+  const int e = blockIdx.x, n = freq[e], rows = ((n + 63) / 64) * 64 - n;
+  char* base = blockIdx.y == 0 ? a : b;
+  const size_t first = (static_cast<size_t>(block_offset[e]) * kTileM + n) * vecs;
+  for (int i = threadIdx.x; i < rows * vecs; i += blockDim.x)
+    st_na_v4(base + (first + i) * 16, make_uint4(0, 0, 0, 0));
+}
+void launch_zero_pool_padding(void* pool_a, void* pool_b, const int* expert_frequency, const int* expert_pool_block_offset,
+                              int num_experts, int hidden, cudaStream_t stream) {
+  zero_pool_padding_kernel<<<dim3(num_experts, 2), 1024, 0, stream>>>(static_cast<char*>(pool_a), static_cast<char*>(pool_b),
+                                                                     expert_frequency, expert_pool_block_offset, hidden / 8);
 }
 
 // =============================================================================================

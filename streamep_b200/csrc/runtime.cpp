@@ -299,19 +299,20 @@ struct DispatchState {
       num_send;
   // receiver side metadata (regular device memory)
   at::Tensor expert_frequency, expert_pool_block_offset, base_pool, seen_per_substream, rank_prefix_matrix,
-      recv_channel_prefix_matrix, tile_id_to_expert, pool_arrival_target;
+      recv_channel_prefix_matrix, tile_id_to_expert, pool_arrival_target, pair_tiles;
   // receiver side, written by peers (symmetric arena)
   at::Tensor meta_slab;
   at::Tensor pool, pool_topk_weight, pool_recv_token, pool_k_slot, pool_src, recv_token_to_slots, k_local_total,
       k_local_remaining, pool_arrival_count, recv_src, y_done_per_token, o;
   int total_tiles = 0, num_recv_tokens = 0;
+  int num_pairs = 0;                   // pairs of row tiles the GEMMs of this dispatch work on (capacity mode: a bound); 0 = single tiles
   std::vector<int> recv_per_expert;
   std::optional<EventHandle> metadata_done_event;
   BufferRecord record{};
   std::vector<at::Tensor> aux_keepalive;
   // capacity mode (no host read of the sizes): the receive buffers are a fixed region of the arena
   int region_id = -1;                  // -1: exact mode
-  at::Tensor dev_sizes;                // int32 [4] device: live total_tiles, live num_recv_tokens, overflow flag
+  at::Tensor dev_sizes;                // int32 [4] device: live total_tiles, live num_recv_tokens, overflow flag, live pairs
   std::shared_ptr<void> region_guard;  // keeps the region claimed while this state (or a view of the region) lives
 
   void release_o() { o = at::Tensor(); }
@@ -354,7 +355,11 @@ struct GemmArgs {
   std::vector<int> remote_dw;
   // capacity mode: the buffer sits at this arena offset on every rank (no record look-up); -1 = use the record
   int64_t remote_out_offset = -1, remote_dw_offset = -1;
-  std::optional<at::Tensor> num_m_tiles_dev;        // VarlenM: live tile count in device memory (capacity mode)
+  std::optional<at::Tensor> num_m_tiles_dev;        // VarlenM: the dispatch's dev_sizes (live counts, capacity mode)
+  // VarlenM on CTA pairs: the dispatch's list of row-tile pairs and how many there are (at most, in capacity mode)
+  std::optional<at::Tensor> pair_tiles;
+  int num_pairs = 0;
+  bool padding_is_zero = false;                     // VarlenK: rows past an expert's length, up to a multiple of 64, hold zeros
   int num_topk = 0;
   int64_t seq = 0;
   int num_m_tiles = -1;                             // VarlenM: total tiles (defaults to len(tile_id_to_expert))
@@ -749,7 +754,7 @@ class Runtime {
     const int64_t tiles_cap = capacity_mode ? static_->tiles_cap : 0;
     if (capacity_mode) SEP_ASSERT(static_fits(T, st->hidden, st->num_topk), "this dispatch does not fit the capacity-mode regions (tokens, hidden or top-k differ)");
     const int64_t n_i32 = T * K * 3 + T * R * 3 + (T * R + 3) / 4 + R * C + 2 * C * E + C * R + 2 * R + EL + (EL + 1) +
-                          2 * C * R * EL + R * R + R * C + 2 * tiles_cap + 104;
+                          2 * C * R * EL + R * R + R * C + 3 * tiles_cap + 108;
     st->sender_slab = at::empty({n_i32}, x.options().dtype(at::kInt));
     int64_t off = 0;
     auto take = [&](std::vector<int64_t> shape) {
@@ -768,7 +773,8 @@ class Runtime {
     st->base_pool = take({C, R, EL}); st->seen_per_substream = take({C, R, EL});
     st->rank_prefix_matrix = take({R, R}); st->recv_channel_prefix_matrix = take({R, C});
     if (capacity_mode) {
-      st->tile_id_to_expert = take({tiles_cap}); st->pool_arrival_target = take({tiles_cap});
+      st->tile_id_to_expert = take({tiles_cap}); st->pool_arrival_target = take({tiles_cap}); st->pair_tiles = take({tiles_cap});
+      st->num_pairs = pairs_pay(T * K * R, E) ? static_cast<int>(tiles_cap) : 0;
       st->dev_sizes = take({4});
       // claim the lowest free region: ranks that run the same program pick the same one (the metadata kernel checks)
       std::shared_ptr<StaticPlan> pl = static_;
@@ -815,6 +821,7 @@ class Runtime {
       p.tiles_cap = static_cast<int>(pl.tiles_cap); p.recv_cap = static_cast<int>(pl.recv_cap);
       p.dev_sizes = st->dev_sizes.data_ptr<int>();
       p.tile_id_to_expert = st->tile_id_to_expert.data_ptr<int>(); p.pool_arrival_target = st->pool_arrival_target.data_ptr<int>();
+      p.pair_tiles = st->pair_tiles.data_ptr<int>();
       p.host_overflow = host_overflow_dev_;
       if (phase_mask & 1) {
         // Defaults of everything peers write into this region, for the whole capacity (a few MB of small arrays),
@@ -871,8 +878,12 @@ class Runtime {
 
     const int64_t tiles = st->total_tiles, TKp = tiles * st->tile_m, Tr = st->num_recv_tokens, K = st->num_topk, H = st->hidden;
     auto opts = st->x.options();
-    st->tile_id_to_expert = at::empty({tiles * 2}, opts.dtype(at::kInt));
+    st->tile_id_to_expert = at::empty({tiles * 3}, opts.dtype(at::kInt));
     st->pool_arrival_target = st->tile_id_to_expert.narrow(0, tiles, tiles);
+    st->pair_tiles = st->tile_id_to_expert.narrow(0, tiles * 2, tiles);
+    int pairs = 0;
+    for (int e = 0; e < EL; ++e) pairs += ((st->recv_per_expert[e] + st->tile_m - 1) / st->tile_m + 1) / 2;
+    st->num_pairs = 2.0 * pairs <= kPairWaste * tiles ? pairs : 0;
     st->tile_id_to_expert = st->tile_id_to_expert.narrow(0, 0, tiles);
     size_t off_pool = 0, off_slab = 0;   // empty tensors report a null data pointer, so offsets are tracked here
     st->pool = alloc_symmetric({TKp, H}, at::kBFloat16, false, &off_pool);
@@ -897,6 +908,7 @@ class Runtime {
     f.expert_frequency = st->expert_frequency.data_ptr<int>();
     f.expert_pool_block_offset = st->expert_pool_block_offset.data_ptr<int>();
     f.tile_id_to_expert = st->tile_id_to_expert.data_ptr<int>(); f.pool_arrival_target = st->pool_arrival_target.data_ptr<int>();
+    f.pair_tiles = st->pair_tiles.data_ptr<int>();
     f.pool_topk_weight = reinterpret_cast<float*>(at_off(0));
     f.pool_recv_token = reinterpret_cast<int*>(at_off(1)); f.pool_k_slot = reinterpret_cast<int*>(at_off(2));
     f.pool_src = reinterpret_cast<int2*>(at_off(3));
@@ -1154,15 +1166,19 @@ class Runtime {
       SEP_ASSERT(K % 8 == 0 && N % 8 == 0, "K and N must be multiples of 8");
       p.N = N; p.K = K; p.num_experts = E; p.total_rows = rows;
       p.num_m_tiles = a.num_m_tiles >= 0 ? a.num_m_tiles : a.tile_id_to_expert->numel();
+      if (a.num_pairs > 0 && BN == 256) {
+        p.pair_ctas = 1; p.pair_tiles = a.pair_tiles->data_ptr<int>();
+        if (a.num_m_tiles != 0) p.num_m_tiles = a.num_pairs;
+      }
       // (the fp32-store epilogue guards rows itself: its last tile may hang over the end of A, TMA zero-fills it)
       SEP_ASSERT(static_cast<int64_t>(p.num_m_tiles) * BM_ <= rows || a.epilogue == kEpiStoreF32, "tile list longer than A");
       p.num_n_tiles = (N + BN - 1) / BN;
       p.tile_id_to_expert = a.tile_id_to_expert->data_ptr<int>();
-      if (a.num_m_tiles_dev.has_value()) p.num_m_tiles_dev = a.num_m_tiles_dev->data_ptr<int>();
+      if (a.num_m_tiles_dev.has_value()) p.num_m_tiles_dev = a.num_m_tiles_dev->data_ptr<int>() + (p.pair_ctas ? 3 : 0);
       if (rows == 0) { launch_without_tiles(a); return; }
       ta = make_tmap(a.a.data_ptr(), K, rows, 1, K, rows * K, 64, BM_);
       if (a.b_mn_major) tb = make_tmap(a.b.data_ptr(), N, K, E, N, K * N, 64, 64);
-      else tb = make_tmap(a.b.data_ptr(), K, N, E, K, N * K, 64, BN);
+      else tb = make_tmap(a.b.data_ptr(), K, N, E, K, N * K, 64, p.pair_ctas ? BN / 2 : BN);
     } else {
       // dW: A [rows, M], B [rows, N] row-major; out [E, M, N]
       SEP_ASSERT(a.a.dim() == 2 && a.b.dim() == 2 && a.a.size(0) == a.b.size(0), "varlen-K GEMM needs A [rows, M] and B [rows, N]");
@@ -1171,7 +1187,13 @@ class Runtime {
       const int64_t rows = a.a.size(0), M = a.a.size(1), N = a.b.size(1), E = a.expert_frequency->numel();
       SEP_ASSERT(M % 8 == 0 && N % 8 == 0, "M and N must be multiples of 8");
       p.N = N; p.M_out = M; p.num_experts = E; p.total_rows = rows;
-      p.num_m_tiles = (M + BM_ - 1) / BM_; p.num_n_tiles = (N + BN - 1) / BN;
+      const int64_t M2_ = a.a2.has_value() ? a.a2->size(1) : 0;
+      // Pairs of 128-row tiles of the output, unless too many of them would have no second tile.
+      auto units = [](int64_t m, int64_t rows_per_unit) { return (m + rows_per_unit - 1) / rows_per_unit; };
+      p.pair_ctas = a.padding_is_zero && BN == 256 &&
+                    2.0 * (units(M, 2 * BM_) + units(M2_, 2 * BM_)) <= kPairWaste * (units(M, BM_) + units(M2_, BM_));
+      const int64_t unit_m = p.pair_ctas ? 2 * BM_ : BM_;
+      p.num_m_tiles = units(M, unit_m); p.num_n_tiles = (N + BN - 1) / BN;
       p.expert_pool_block_offset = a.expert_pool_block_offset->data_ptr<int>();
       p.expert_frequency = a.expert_frequency->data_ptr<int>();
       p.out_expert_stride = M * N;
@@ -1182,7 +1204,7 @@ class Runtime {
                    "the second varlen-K problem needs contiguous bf16 A2 [rows, M2], B2 [rows, N2] over the same rows, and an output");
         const int64_t M2 = a.a2->size(1), N2 = a.b2->size(1);
         SEP_ASSERT(M2 % 8 == 0 && N2 % 8 == 0, "M2 and N2 must be multiples of 8");
-        p.N2 = N2; p.M_out2 = M2; p.num_m_tiles2 = (M2 + BM_ - 1) / BM_; p.num_n_tiles2 = (N2 + BN - 1) / BN;
+        p.N2 = N2; p.M_out2 = M2; p.num_m_tiles2 = units(M2, unit_m); p.num_n_tiles2 = (N2 + BN - 1) / BN;
       }
       if (rows == 0) { a.out0->zero_(); if (a.out2.has_value()) a.out2->zero_(); return; }
       ta = make_tmap(a.a.data_ptr(), M, rows, 1, M, rows * M, 64, 64);
@@ -1271,6 +1293,7 @@ class Runtime {
       to1 = out_map(*a.out1, p.N, p.total_rows, 1, 32, CU_TENSOR_MAP_SWIZZLE_64B); have_o1 = true;
     }
     int n_ctas = a.num_ctas > 0 ? a.num_ctas : num_sms();
+    const int ctas_per_unit = p.pair_ctas ? 2 : 1;
     const int64_t total = a.mode == kVarlenM ? static_cast<int64_t>(p.num_m_tiles) * p.num_n_tiles
         : static_cast<int64_t>(p.num_experts) * (static_cast<int64_t>(p.num_m_tiles) * p.num_n_tiles + static_cast<int64_t>(p.num_m_tiles2) * p.num_n_tiles2);
     PushParams pp{};
@@ -1287,7 +1310,8 @@ class Runtime {
       pp.started_flag = nullptr;
       ppp = &pp;
     }
-    if (ppp == nullptr) n_ctas = static_cast<int>(std::min<int64_t>(n_ctas, std::max<int64_t>(total, 1)));
+    if (ppp == nullptr) n_ctas = static_cast<int>(std::min<int64_t>(n_ctas, std::max<int64_t>(total, 1) * ctas_per_unit));
+    n_ctas = std::max(n_ctas / ctas_per_unit, 1) * ctas_per_unit;
     if (n_ctas > num_sms()) p.timing = nullptr;   // the stamp tensor has one row per SM
     ++launches_;
     cudaError_t setup_error = cudaSuccess;
@@ -1353,6 +1377,7 @@ class Runtime {
     a.arrival_count = st->pool_arrival_count; a.arrival_target = st->pool_arrival_target;
     a.fused_push = st; a.push_flags = 3;
     if (cap) a.num_m_tiles_dev = st->dev_sizes;
+    use_pairs(a, *st);
     grouped_gemm(a);
     if (!cap) dispatch_finish_views(st);          // host work in the shadow of kernel A
     GemmArgs y;
@@ -1363,6 +1388,7 @@ class Runtime {
     else y.remote_out = {kKindDispatch, st->push_epoch, 10};
     y.row_src = st->pool_src; y.row_k_slot = st->pool_k_slot; y.num_topk = st->num_topk;
     y.tail = true; y.tail_kind = kKindGemmYTail; y.tail_wait = true;
+    use_pairs(y, *st);
     grouped_gemm(y);
     combine_reduce(out, landing, st->topk_idx, st->num_experts, std::nullopt, std::nullopt,
                    cap ? std::optional<at::Tensor>(st->dev_sizes) : std::nullopt);
@@ -1400,6 +1426,7 @@ class Runtime {
         r.mode = kVarlenM; r.epilogue = kEpiStore; r.block_n = tile_n_a;
         r.a = pool; r.b = w1; r.tile_id_to_expert = st->tile_id_to_expert; r.out0 = preact;
         if (cap) r.num_m_tiles_dev = st->dev_sizes;
+        use_pairs(r, *st);
         grouped_gemm(r);
       }
     }
@@ -1413,6 +1440,7 @@ class Runtime {
     else y.remote_dw = {kKindDispatchGrads, g->epoch, 11};
     y.row_src = st->pool_src; y.row_k_slot = st->pool_k_slot; y.num_topk = static_cast<int>(K); y.tile_stripes_done = stripes;
     y.fused_push_grads = g; y.fused_push_routing = st; y.fused_push_rows = dl_dy; y.push_flags = 3;
+    use_pairs(y, *st);
     grouped_gemm(y);
     GemmArgs a;
     a.mode = kVarlenM; a.epilogue = kEpiScatter; a.block_n = tile_n_a_bwd; a.b_mn_major = true; a.num_ctas = num_sms_a_bwd;
@@ -1422,6 +1450,7 @@ class Runtime {
     else a.remote_out = {kKindDispatchGrads, g->epoch, 10};
     a.row_src = st->pool_src; a.row_k_slot = st->pool_k_slot; a.num_topk = static_cast<int>(K);
     a.tail = true; a.tail_kind = kKindGemmABwdTail; a.tail_wait = true;
+    use_pairs(a, *st);
     grouped_gemm(a);
     at::Tensor dwt = g->dwt;
     if (cap) {
@@ -1440,6 +1469,10 @@ class Runtime {
       GemmArgs d;
       d.mode = kVarlenK; d.epilogue = kEpiStore; d.a_mn_major = d.b_mn_major = true; d.dynamic_tiles = true;
       d.expert_pool_block_offset = st->expert_pool_block_offset; d.expert_frequency = st->expert_frequency;
+      // Y_bwd wrote zeros into the padding rows of its two outputs; the pools get theirs here
+      ++launches_; launch_zero_pool_padding(pool.data_ptr(), g->dl_do_pool.data_ptr(), st->expert_frequency.data_ptr<int>(),
+                                            st->expert_pool_block_offset.data_ptr<int>(), st->num_experts / num_ranks_, H, stream());
+      d.padding_is_zero = true;
       if (tile_n_dw1 == tile_n_dw2) {
         d.block_n = tile_n_dw1;
         d.a = dswiglu_in; d.b = pool; d.out0 = dW1;
@@ -1455,6 +1488,19 @@ class Runtime {
       dW1.zero_(); dW2.zero_();
     }
     return {dx, dwt, dW1, dW2};
+  }
+
+  // Work on pairs of row tiles with CTA pairs (see gemm_kernel.cuh) when the dispatch has a pair list worth using.
+  static void use_pairs(GemmArgs& a, const DispatchState& st) {
+    if (st.num_pairs > 0) { a.pair_tiles = st.pair_tiles; a.num_pairs = st.num_pairs; }
+  }
+  // An expert with an odd number of row tiles leaves half of its last pair idle, half a tile per expert on average.
+  // Pairs pay as long as they have at most this many times as many tile slots as there are tiles.
+  static constexpr double kPairWaste = 1.15;
+  // The same decision from the mean load, for a dispatch whose counts the host does not read.
+  static bool pairs_pay(int64_t pairs, int64_t experts) {
+    const double tiles = static_cast<double>(pairs) / static_cast<double>(experts) / kTileM;      // per expert
+    return tiles + 1.0 <= kPairWaste * (tiles + 0.5);
   }
 
   // ---- small ops ---------------------------------------------------------------------------------------
@@ -1716,6 +1762,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
       RW(tile_id_to_expert) RW(expert_pool_block_offset) RW(expert_frequency) RW(arrival_count) RW(arrival_target)
       RW(out0) RW(out1) RW(preact) RW(row_weight) RW(row_token) RW(dl_dweight) RW(scatter_local) RW(row_src) RW(row_k_slot)
       RW(tile_stripes_done) RW(k_remaining) RW(done_per_token) RW(remote_out) RW(remote_dw) RW(remote_out_offset) RW(remote_dw_offset) RW(num_m_tiles_dev)
+      RW(pair_tiles) RW(num_pairs) RW(padding_is_zero)
       RW(num_topk) RW(seq) RW(num_m_tiles) RW(started_flag)
       RW(tail) RW(tail_kind) RW(tail_wait) RW(fused_push) RW(fused_push_grads) RW(fused_push_routing) RW(fused_push_rows)
       RW(push_flags);
