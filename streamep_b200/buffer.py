@@ -375,7 +375,9 @@ class Buffer:
         torch.cuda.synchronize()
         self.runtime.poll_status(True)
         mine = self.runtime.get_epochs()
-        if self._local is not None:
+        if self.group_size == 1:
+            every = [mine]
+        elif self._local is not None:
             every = [b.runtime.get_epochs() for b in self._local[0].buffers]
         else:
             every = [None] * self.group_size
@@ -665,6 +667,21 @@ class Buffer:
         self.runtime.barrier()
 
 
+class _OneRank:
+    """The group of a buffer that is on its own.  It does not point back at the buffer: the buffer's memory is
+    returned when its last reference goes, not at some later garbage collection in the middle of other work."""
+    num_ranks = 1
+
+    def __init__(self):
+        self._static_bases = [None]
+
+    def size(self):
+        return 1
+
+    def _barrier_wait(self):
+        pass
+
+
 class LocalWorld:
     """Several ranks emulated in ONE process on ONE device.
 
@@ -686,7 +703,8 @@ class LocalWorld:
         self._in_run = threading.local()
         self._static_bases = [None] * num_ranks
         self.buffers: List[Buffer] = [
-            Buffer(None, arena_bytes, _local=(self, r), timeout_ms=timeout_ms, allocator=allocator) for r in range(num_ranks)]
+            Buffer(None, arena_bytes, _local=(self if num_ranks > 1 else _OneRank(), r), timeout_ms=timeout_ms, allocator=allocator)
+            for r in range(num_ranks)]
         ptrs = [b.runtime.get_local_base_ptr() for b in self.buffers]
         for b in self.buffers:
             b.runtime.sync_local(ptrs)

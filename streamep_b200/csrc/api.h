@@ -183,6 +183,51 @@ struct PushParams {
 void launch_dispatch_push(const PushParams& p, int num_blocks, cudaStream_t stream);
 
 // ---------------------------------------------------------------------------------------------
+// Dispatch of a single rank (local_kernels.cu): slots by a counting sort, rows copied into the pool, no exchange
+// ---------------------------------------------------------------------------------------------
+struct LocalGrid {
+  int blocks, tokens_per_block;
+  bool fused_count;              // no count launch: every block counts all pairs
+  size_t count_ints;             // scratch for the counts
+};
+LocalGrid local_grid(int num_tokens, int num_topk, int num_experts);
+struct LocalPlaceParams {
+  const void* x;                 // [T, H] bf16
+  const long long* topk_idx;     // [T, K], -1 = skip
+  const float* topk_weights;     // [T, K]
+  int num_tokens, hidden, num_topk, num_experts;
+  int tokens_per_block, token_blocks;   // set by the launcher
+  int* counts;                   // [E][token_blocks] scratch
+  int* pair_slot;                // [T, K] pool slot of every pair (-1 = skipped)
+  int* row_token;                // [slots] token of the slot (-1 = padding)
+  int* row_pair;                 // [slots] t * K + k (-1 = padding)
+  float* row_weight;             // [slots]
+  int* expert_frequency;         // [E]
+  int* expert_pool_block_offset; // [E + 1]
+  int* tile_id_to_expert;        // [tiles_cap]
+  int* pair_tiles;               // [tiles_cap]
+  int* sizes;                    // [4] live tiles, tokens, overflow flag, live pairs of tiles
+  int tiles_cap;                 // a layout with more tiles runs as an empty dispatch and is reported
+  void* pool;                    // [slots, H]
+  void* x_saved;                 // optional [T, H]: a copy of x
+  void* zero; size_t zero_bytes; // memory to zero on the side (the layer's output)
+  int region_id, epoch;
+  HostOverflow* host_overflow;
+  StatusBlock* status;
+};
+void launch_local_place(const LocalPlaceParams& p, const LocalGrid& g, cudaStream_t stream);
+struct LocalRowsParams {
+  const void* rows[2];           // [T, H] each; pool[i] == nullptr: none
+  void* pool[2];
+  const int* pair_slot;
+  const int* expert_frequency;
+  const int* expert_pool_block_offset;
+  int num_tokens, hidden, num_topk, num_experts;
+  void* zero[2]; size_t zero_bytes[2];
+};
+void launch_local_rows(const LocalRowsParams& p, cudaStream_t stream);
+
+// ---------------------------------------------------------------------------------------------
 // Pull combine: each source rank gathers its tokens' partial rows from the expert ranks
 // ---------------------------------------------------------------------------------------------
 struct CombineParams {
@@ -315,6 +360,7 @@ struct GemmParams {
   const float* row_weight;       // pool_topk_weight, may be null (unweighted scatter)
   const int* row_token;          // pool_recv_token (-1 = padding row)
   float* dl_dweight;             // [rows] fp32, red.add per (row, n-tile)
+  const int* row_pair;           // optional: dl_dweight is indexed by row_pair[row] instead of the row
   // scatter targets
   void* scatter_local;           // [T_recv, N] bf16 (local variant)
   const int2* row_src;           // per-slot (src_rank, src_token) (remote variant)

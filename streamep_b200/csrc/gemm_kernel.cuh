@@ -786,7 +786,7 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
       }
       if (!t.rows_valid) continue;
       if (EPI == kEpiDswiglu) {
-        if (tok >= 0 && p.dl_dweight != nullptr) red_add_f32(p.dl_dweight + grow, dw_acc);
+        if (tok >= 0 && p.dl_dweight != nullptr) red_add_f32(p.dl_dweight + (p.row_pair != nullptr ? p.row_pair[grow] : grow), dw_acc);
       }
       if ((EPI == kEpiScatter && !p.remote_out.enabled && p.tile_stripes_done != nullptr) ||
           (EPI == kEpiDswiglu && p.remote_dw.enabled)) {

@@ -393,7 +393,31 @@ struct StaticPlan {
   uint64_t landing_calls = 0, bwd_calls = 0;
 };
 
-class Runtime {
+class Runtime;
+
+// Tile widths and grid limits of a layer's GEMMs (0 = every SM), from the caller's TileConfig.
+struct LayerConfig {
+  int tile_n_a, tile_n_y, tile_n_y_bwd, tile_n_a_bwd, tile_n_dw1, tile_n_dw2;
+  int num_sms_a, num_sms_y, num_sms_y_bwd, num_sms_a_bwd;
+};
+
+// What the forward of a single-rank layer keeps for its backward.
+struct LocalState : torch::CustomClassHolder {
+  std::shared_ptr<Runtime> runtime;
+  LayerConfig cfg{};
+  int level = 0, tokens = 0, hidden = 0, ffn = 0, experts = 0, topk = 0;
+  int tiles = 0;                       // row tiles the buffers hold (a bound: the live count is in device memory)
+  int pairs = 0;                       // bound on pairs of row tiles; 0 = the GEMMs work on single tiles
+  at::Tensor slab;                     // the int32 arrays below
+  int *pair_slot = nullptr, *row_token = nullptr, *row_pair = nullptr, *frequency = nullptr, *block_offset = nullptr,
+      *tile_expert = nullptr, *pair_tiles = nullptr, *sizes = nullptr;
+  float* row_weight = nullptr;
+  at::Tensor rows;                     // the pool (levels 0 and 1) or a copy of x (level 2)
+  at::Tensor preact, w1, w2;
+  std::shared_ptr<void> region_guard;  // capacity mode
+};
+
+class Runtime : public std::enable_shared_from_this<Runtime> {
  public:
   // `use_vmm`: take the arena from the virtual-memory-management API (shareable by file descriptor) instead of
   // cudaMalloc + CUDA IPC.
@@ -550,12 +574,19 @@ class Runtime {
   int rank() const { return rank_; }
   int num_ranks() const { return num_ranks_; }
   int num_channels() const { return num_channels_; }
-  int64_t launch_count() const { return launches_; }
+  int64_t launch_count() const { return launches_.load(std::memory_order_relaxed); }
   // Event at the point of the current stream where the most recent backward left its last kernel that talks to
   // peers: what follows (the dW GEMMs) is local.  A host-to-device prefetch that waits on it stays clear of the
   // kernels that synchronise at system scope, which measured markedly slower while a PCIe copy was in flight.
-  void mark_local_phase() { local_phase_ = std::make_shared<EventHandle>(stream()); }
-  std::optional<EventHandle> local_phase_event() const { return local_phase_ ? std::optional<EventHandle>(*local_phase_) : std::nullopt; }
+  void mark_local_phase() {
+    auto e = std::make_shared<EventHandle>(stream());
+    std::lock_guard<std::mutex> g(phase_mu_);
+    local_phase_ = std::move(e);
+  }
+  std::optional<EventHandle> local_phase_event() {
+    std::lock_guard<std::mutex> g(phase_mu_);
+    return local_phase_ ? std::optional<EventHandle>(*local_phase_) : std::nullopt;
+  }
   // Per-CTA time stamps of the GEMM kernels (see GemmParams::timing).  Returns the tensor the launches that follow
   // fill: int64 [10, num_sms, 8], first index = epilogue kind (0 store, 1 SwiGLU, 2 scatter, 3 dSwiGLU, 4 fp32 store),
   // + 5 for the launches with a fused push.  Each launch overwrites the rows of its kind.  `on = false` stops it.
@@ -776,19 +807,23 @@ class Runtime {
       st->tile_id_to_expert = take({tiles_cap}); st->pool_arrival_target = take({tiles_cap}); st->pair_tiles = take({tiles_cap});
       st->num_pairs = pairs_pay(T * K * R, E) ? static_cast<int>(tiles_cap) : 0;
       st->dev_sizes = take({4});
-      // claim the lowest free region: ranks that run the same program pick the same one (the metadata kernel checks)
-      std::shared_ptr<StaticPlan> pl = static_;
-      int id = -1;
-      {
-        std::lock_guard<std::mutex> g(pl->mu);
-        for (int i = 0; i < pl->num_regions && id < 0; ++i) if (!pl->busy[i]) { pl->busy[i] = 1; id = i; }
-      }
-      SEP_ASSERT(id >= 0, "every capacity-mode region is in use: enable capacity mode with as many regions as layers keep forward state alive");
-      st->region_id = id;
-      st->region_guard = std::shared_ptr<void>(nullptr, [pl, id](void*) { std::lock_guard<std::mutex> g(pl->mu); pl->busy[id] = 0; });
+      st->region_id = claim_region(st->region_guard);
     }
     SEP_ASSERT(off <= n_i32, "sender slab overflow");
     return st;
+  }
+
+  // Claims the lowest free region: ranks that run the same program pick the same one (the metadata kernel checks).
+  int claim_region(std::shared_ptr<void>& guard) {
+    std::shared_ptr<StaticPlan> pl = static_;
+    int id = -1;
+    {
+      std::lock_guard<std::mutex> g(pl->mu);
+      for (int i = 0; i < pl->num_regions && id < 0; ++i) if (!pl->busy[i]) { pl->busy[i] = 1; id = i; }
+    }
+    SEP_ASSERT(id >= 0, "every capacity-mode region is in use: enable capacity mode with as many regions as layers keep forward state alive");
+    guard = std::shared_ptr<void>(nullptr, [pl, id](void*) { std::lock_guard<std::mutex> g(pl->mu); pl->busy[id] = 0; });
+    return id;
   }
 
   // ---- dispatch: phase 1, metadata kernel ------------------------------------------------------
@@ -1490,6 +1525,239 @@ class Runtime {
     return {dx, dwt, dW1, dW2};
   }
 
+  // ---- the layer of a single rank -------------------------------------------------------------------------------
+  // Nothing is exchanged, so the pairs are sorted and the rows copied by the kernels of local_kernels.cu and the GEMM
+  // kernels run without gates or pushes.  Buffers are sized by a bound (pairs / 128 + one tile per expert) and the live
+  // counts stay on the device: the host reads nothing.  Backward adds dL/dweight directly into its [T, K] result.
+  // In capacity mode the pools are the fixed regions, as in the general path.
+  std::pair<at::Tensor, c10::intrusive_ptr<LocalState>> local_forward(const at::Tensor& x_in, const at::Tensor& idx_in, const at::Tensor& weights_in,
+                                                                      const at::Tensor& w1_in, const at::Tensor& w2_in, int num_experts, int level,
+                                                                      const LayerConfig& cfg, bool for_backward, c10::cuda::CUDAStream comp) {
+    SEP_ASSERT(available_ && num_ranks_ == 1, "Buffer.sync has not completed");
+    SEP_ASSERT(x_in.is_cuda() && x_in.dim() == 2 && x_in.scalar_type() == at::kBFloat16, "x must be a [T, H] bf16 CUDA tensor");
+    SEP_ASSERT(idx_in.is_cuda() && idx_in.dim() == 2 && weights_in.is_cuda() && weights_in.sizes() == idx_in.sizes() && x_in.size(0) == idx_in.size(0),
+               "topk_idx and topk_weights must be [T, K] CUDA tensors over the tokens of x");
+    SEP_ASSERT(num_experts <= ctl_.num_experts_cap, "num_experts must fit the Buffer's expert capacity");
+    SEP_ASSERT(x_in.size(1) % 8 == 0 && w2_in.size(2) % 8 == 0, "hidden and ffn must be multiples of 8");
+    SEP_ASSERT(idx_in.size(1) >= 1 && idx_in.size(1) <= kMaxTopK, "num_topk out of range");
+    SEP_ASSERT(w1_in.is_cuda() && w2_in.is_cuda() && w1_in.dim() == 3 && w1_in.size(0) == num_experts && w1_in.size(2) == x_in.size(1) &&
+               w2_in.size(1) == x_in.size(1) && w1_in.size(1) == 2 * w2_in.size(2), "expert weights do not match x and num_experts");
+    const c10::cuda::CUDAStream caller = at::cuda::getCurrentCUDAStream();
+    at::Tensor x = x_in.contiguous(), w1 = w1_in.contiguous(), w2 = w2_in.contiguous(), idx = idx_in, weights = weights_in;
+    if (idx.scalar_type() != at::kLong) idx = idx.to(at::kLong);
+    if (weights.scalar_type() != at::kFloat) weights = weights.to(at::kFloat);
+    idx = idx.contiguous(); weights = weights.contiguous();
+    stream_wait(comp, caller);
+    c10::cuda::CUDAStreamGuard guard(comp);
+    const int64_t T = x.size(0), H = x.size(1), K = idx.size(1), I = w2.size(2), E = num_experts, P = T * K;
+    auto st = c10::make_intrusive<LocalState>();
+    st->cfg = cfg; st->level = level; st->tokens = T; st->hidden = H; st->ffn = I; st->experts = E; st->topk = K;
+    const bool cap = static_fits(T, H, K);
+    int64_t tiles = P / kTileM + std::min<int64_t>(E, P);
+    int region = -1;
+    if (cap) {
+      region = claim_region(st->region_guard);
+      tiles = std::min<int64_t>(tiles, static_->tiles_cap);
+    }
+    st->tiles = tiles;
+    st->pairs = pairs_pay(P, E) ? static_cast<int>(std::min<int64_t>(tiles, P / (2 * kTileM) + std::min<int64_t>(E, P))) : 0;
+    const int64_t R = tiles * kTileM;
+    const LocalGrid grid = local_grid(T, K, E);
+    const int64_t counts[] = {static_cast<int64_t>(grid.count_ints), P, R, R, R, E, E + 1, tiles, tiles, 4};
+    int64_t off[11] = {0};
+    for (int i = 0; i < 10; ++i) off[i + 1] = off[i] + (counts[i] + 3) / 4 * 4;
+    auto opts = x.options();
+    st->slab = at::empty({off[10]}, opts.dtype(at::kInt));
+    int* base = st->slab.data_ptr<int>();
+    st->pair_slot = base + off[1]; st->row_token = base + off[2]; st->row_pair = base + off[3];
+    st->row_weight = reinterpret_cast<float*>(base + off[4]); st->frequency = base + off[5]; st->block_offset = base + off[6];
+    st->tile_expert = base + off[7]; st->pair_tiles = base + off[8]; st->sizes = base + off[9];
+    at::Tensor pool = cap ? region_view(static_->region_off[region] + static_->o_pool, {R, H}, at::kBFloat16, st->region_guard)
+                          : at::empty({R, H}, opts);
+    at::Tensor out = at::empty({T, H}, opts), postact = at::empty({R, I}, opts);
+    if (for_backward) {
+      st->w1 = w1; st->w2 = w2;
+      if (level == 0) st->preact = at::empty({R, 2 * I}, opts);
+      st->rows = level < 2 ? pool : at::empty({T, H}, opts);
+    }
+    LocalPlaceParams p{};
+    p.x = x.data_ptr(); p.topk_idx = reinterpret_cast<const long long*>(idx.data_ptr<int64_t>()); p.topk_weights = weights.data_ptr<float>();
+    p.num_tokens = T; p.hidden = H; p.num_topk = K; p.num_experts = E;
+    p.counts = base; p.pair_slot = st->pair_slot; p.row_token = st->row_token; p.row_pair = st->row_pair; p.row_weight = st->row_weight;
+    p.expert_frequency = st->frequency; p.expert_pool_block_offset = st->block_offset;
+    p.tile_id_to_expert = st->tile_expert; p.pair_tiles = st->pair_tiles; p.sizes = st->sizes;
+    p.tiles_cap = cap ? static_cast<int>(static_->tiles_cap) : static_cast<int>(tiles);
+    p.pool = pool.data_ptr(); p.x_saved = for_backward && level == 2 ? st->rows.data_ptr() : nullptr;
+    p.zero = out.data_ptr(); p.zero_bytes = out.nbytes();
+    p.region_id = region; p.epoch = ++epochs_[kKindMetadata];
+    p.host_overflow = cap ? host_overflow_dev_ : nullptr; p.status = status_;
+    launches_ += grid.fused_count ? 1 : 2;
+    launch_local_place(p, grid, stream());
+    SEP_CUDA_CHECK(cudaGetLastError());
+    if (tiles > 0) {
+      LocalGemm a(*this, *st, kEpiSwiglu, cfg.tile_n_a);
+      a.operands(pool, w1, false);
+      a.output0(postact, 16, CU_TENSOR_MAP_SWIZZLE_32B);
+      if (st->preact.defined()) a.output1(st->preact, 32, CU_TENSOR_MAP_SWIZZLE_64B);
+      a.launch(cfg.num_sms_a, 1);
+      LocalGemm y(*this, *st, kEpiScatter, cfg.tile_n_y);
+      y.operands(postact, w2, false);
+      y.p.row_token = st->row_token; y.p.row_weight = st->row_weight; y.p.scatter_local = out.data_ptr();
+      y.launch(cfg.num_sms_y, 2);
+    }
+    stream_wait(caller, comp);
+    return {out, st};
+  }
+
+  // Returns {dL_dx, dL_dtopk_weights, dW1, dW2}.
+  std::vector<at::Tensor> local_backward(LocalState& st, const at::Tensor& dl_dy_in, c10::cuda::CUDAStream comp) {
+    const c10::cuda::CUDAStream caller = at::cuda::getCurrentCUDAStream();
+    SEP_ASSERT(st.w1.defined(), "the forward of this layer kept nothing for a backward");
+    at::Tensor dy = dl_dy_in.contiguous();
+    if (dy.scalar_type() != at::kBFloat16) dy = dy.to(at::kBFloat16);
+    SEP_ASSERT(dy.is_cuda() && dy.dim() == 2 && dy.size(0) == st.tokens && dy.size(1) == st.hidden, "dL_dy must be [T, H]");
+    stream_wait(comp, caller);
+    c10::cuda::CUDAStreamGuard guard(comp);
+    const int64_t T = st.tokens, H = st.hidden, I = st.ffn, K = st.topk, R = static_cast<int64_t>(st.tiles) * kTileM;
+    auto opts = dy.options();
+    const LayerConfig& cfg = st.cfg;
+    at::Tensor dx = at::empty({T, H}, opts), dwt = at::empty({T, K}, opts.dtype(at::kFloat));
+    at::Tensor dW1 = at::empty_like(st.w1), dW2 = at::empty_like(st.w2);
+    at::Tensor dl_pool;
+    if (st.region_guard) {            // two fixed gradient regions alternate, as in grads_begin
+      const int par = static_cast<int>(static_->bwd_calls++ & 1);
+      dl_pool = region_view(static_->bwd_pool_off[par], {R, H}, at::kBFloat16, nullptr);
+    } else {
+      dl_pool = at::empty({R, H}, opts);
+    }
+    at::Tensor pool = st.level == 2 ? at::empty({R, H}, opts) : st.rows;
+    LocalRowsParams p{};
+    p.rows[0] = dy.data_ptr(); p.pool[0] = dl_pool.data_ptr();
+    if (st.level == 2) { p.rows[1] = st.rows.data_ptr(); p.pool[1] = pool.data_ptr(); }
+    p.pair_slot = st.pair_slot; p.expert_frequency = st.frequency; p.expert_pool_block_offset = st.block_offset;
+    p.num_tokens = T; p.hidden = H; p.num_topk = K; p.num_experts = st.experts;
+    p.zero[0] = dx.data_ptr(); p.zero_bytes[0] = dx.nbytes(); p.zero[1] = dwt.data_ptr(); p.zero_bytes[1] = dwt.nbytes();
+    ++launches_; launch_local_rows(p, stream());
+    SEP_CUDA_CHECK(cudaGetLastError());
+    if (st.tiles > 0) {
+      at::Tensor preact = st.preact;
+      if (!preact.defined()) {
+        preact = at::empty({R, 2 * I}, opts);
+        LocalGemm r(*this, st, kEpiStore, cfg.tile_n_a);
+        r.operands(pool, st.w1, false);
+        r.output0(preact, 32, CU_TENSOR_MAP_SWIZZLE_64B);
+        r.launch(0, 5);
+      }
+      at::Tensor dswiglu_in = at::empty({R, 2 * I}, opts), postact_dw2 = at::empty({R, I}, opts);
+      LocalGemm y(*this, st, kEpiDswiglu, cfg.tile_n_y_bwd);
+      y.operands(dl_pool, st.w2, true);
+      y.output0(dswiglu_in, 64, CU_TENSOR_MAP_SWIZZLE_128B);
+      y.output1(postact_dw2, 32, CU_TENSOR_MAP_SWIZZLE_64B);
+      y.p.preact = preact.data_ptr(); y.p.ld_preact = 2 * I;
+      y.p.row_token = st.row_token; y.p.row_weight = st.row_weight; y.p.dl_dweight = dwt.data_ptr<float>(); y.p.row_pair = st.row_pair;
+      y.launch(cfg.num_sms_y_bwd, 3);
+      LocalGemm a(*this, st, kEpiScatter, cfg.tile_n_a_bwd);
+      a.operands(dswiglu_in, st.w1, true);
+      a.p.row_token = st.row_token; a.p.scatter_local = dx.data_ptr();
+      a.launch(cfg.num_sms_a_bwd, 7);
+      mark_local_phase();
+      // dW1 and dW2 in one launch, tiles claimed dynamically: one tail instead of two, and experts of unequal row counts
+      // (tiles of unequal length) balance out.  dW1 first: its tiles are the longer ones.
+      if (cfg.tile_n_dw1 == cfg.tile_n_dw2) {
+        LocalGemm d(*this, st, kEpiStore, cfg.tile_n_dw1, /*varlen_k=*/true);
+        d.dw_operands(dswiglu_in, pool, dW1, dl_pool, postact_dw2, &dW2);
+        d.launch(0, 0);
+      } else {
+        LocalGemm d2(*this, st, kEpiStore, cfg.tile_n_dw2, true);
+        d2.dw_operands(dl_pool, postact_dw2, dW2, dl_pool, postact_dw2, nullptr);
+        d2.launch(0, 0);
+        LocalGemm d1(*this, st, kEpiStore, cfg.tile_n_dw1, true);
+        d1.dw_operands(dswiglu_in, pool, dW1, dl_pool, postact_dw2, nullptr);
+        d1.launch(0, 0);
+      }
+    } else {
+      mark_local_phase();
+      dW1.zero_(); dW2.zero_();
+    }
+    stream_wait(caller, comp);
+    return {dx, dwt, dW1, dW2};
+  }
+
+  // One grouped GEMM of the single-rank layer: parameters straight from the state's pointers.
+  struct LocalGemm {
+    Runtime& rt;
+    const LocalState& st;
+    GemmParams p{};
+    CUtensorMap ta, tb, to0, to1, second[3];
+    bool have_o0 = false, have_o1 = false, have_second = false;
+
+    LocalGemm(Runtime& r, const LocalState& s, int epilogue, int block_n, bool varlen_k = false) : rt(r), st(s) {
+      SEP_ASSERT(block_n == 128 || block_n == 256, "block_n must be 128 or 256");
+      p.mode = varlen_k ? kVarlenK : kVarlenM; p.epilogue = epilogue; p.block_n = block_n;
+      p.status = rt.status_; p.wait_budget_ns = rt.budget_ns_; p.num_ranks = 1;
+      p.num_experts = st.experts; p.total_rows = st.tiles * kTileM;
+      p.tile_id_to_expert = st.tile_expert; p.expert_pool_block_offset = st.block_offset; p.expert_frequency = st.frequency;
+    }
+    // A [rows, K], weights [E, N, K] or (b_mn) [E, K, N]
+    void operands(const at::Tensor& a, const at::Tensor& w, bool b_mn) {
+      const int64_t rows = a.size(0), K = a.size(1), N = b_mn ? w.size(2) : w.size(1), E = w.size(0);
+      p.N = N; p.K = K; p.b_mn_major = b_mn;
+      p.pair_ctas = st.pairs > 0 && p.block_n == 256; p.pair_tiles = st.pair_tiles;
+      p.num_m_tiles = p.pair_ctas ? st.pairs : st.tiles; p.num_m_tiles_dev = st.sizes + (p.pair_ctas ? 3 : 0);
+      p.num_n_tiles = (N + p.block_n - 1) / p.block_n;
+      ta = make_tmap(a.data_ptr(), K, rows, 1, K, rows * K, 64, BM_);
+      tb = b_mn ? make_tmap(w.data_ptr(), N, K, E, N, K * N, 64, 64)
+                : make_tmap(w.data_ptr(), K, N, E, K, N * K, 64, p.pair_ctas ? p.block_n / 2 : p.block_n);
+    }
+    // out[e] = a[rows_e]^T @ b[rows_e] and, optionally, out2[e] = a2[rows_e]^T @ b2[rows_e]
+    void dw_operands(const at::Tensor& a, const at::Tensor& b, const at::Tensor& out, const at::Tensor& a2, const at::Tensor& b2, const at::Tensor* out2) {
+      const int64_t rows = a.size(0), M = a.size(1), N = b.size(1), M2 = out2 ? a2.size(1) : 0, E = st.experts;
+      auto units = [](int64_t m, int64_t rows_per_unit) { return (m + rows_per_unit - 1) / rows_per_unit; };
+      p.a_mn_major = p.b_mn_major = 1;
+      p.pair_ctas = p.block_n == 256 && 2.0 * (units(M, 2 * BM_) + units(M2, 2 * BM_)) <= kPairWaste * (units(M, BM_) + units(M2, BM_));
+      const int64_t unit_m = p.pair_ctas ? 2 * BM_ : BM_;
+      p.N = N; p.M_out = M; p.out_expert_stride = M * N;
+      p.num_m_tiles = units(M, unit_m); p.num_n_tiles = (N + p.block_n - 1) / p.block_n;
+      ta = make_tmap(a.data_ptr(), M, rows, 1, M, rows * M, 64, 64);
+      tb = make_tmap(b.data_ptr(), N, rows, 1, N, rows * N, 64, 64);
+      to0 = make_tmap(out.data_ptr(), N, M, E, N, M * N, 32, 32, CU_TENSOR_MAP_SWIZZLE_64B); have_o0 = true;
+      if (out2) {
+        const int64_t N2 = b2.size(1);
+        p.N2 = N2; p.M_out2 = M2; p.num_m_tiles2 = units(M2, unit_m); p.num_n_tiles2 = (N2 + p.block_n - 1) / p.block_n;
+        second[0] = make_tmap(a2.data_ptr(), M2, rows, 1, M2, rows * M2, 64, 64);
+        second[1] = make_tmap(b2.data_ptr(), N2, rows, 1, N2, rows * N2, 64, 64);
+        second[2] = make_tmap(out2->data_ptr(), N2, M2, E, N2, M2 * N2, 32, 32, CU_TENSOR_MAP_SWIZZLE_64B);
+        have_second = true;
+      }
+      p.tile_counter = rt.counters_ + 10;
+    }
+    void output0(const at::Tensor& t, uint32_t box, CUtensorMapSwizzle sw) {
+      to0 = make_tmap(t.data_ptr(), t.size(1), t.size(0), 1, t.size(1), t.numel(), box, 32, sw); have_o0 = true;
+      p.out0 = t.data_ptr(); p.ld0 = t.size(1);
+    }
+    void output1(const at::Tensor& t, uint32_t box, CUtensorMapSwizzle sw) {
+      to1 = make_tmap(t.data_ptr(), t.size(1), t.size(0), 1, t.size(1), t.numel(), box, 32, sw); have_o1 = true;
+      p.out1 = t.data_ptr(); p.ld1 = t.size(1);
+    }
+    // `kind`: row block of the time-stamp tensor (see set_kernel_timing)
+    void launch(int num_sms, int kind) {
+      const int unit = p.pair_ctas ? 2 : 1;
+      const int64_t total = p.mode == kVarlenM ? static_cast<int64_t>(p.num_m_tiles) * p.num_n_tiles
+          : static_cast<int64_t>(p.num_experts) * (static_cast<int64_t>(p.num_m_tiles) * p.num_n_tiles + static_cast<int64_t>(p.num_m_tiles2) * p.num_n_tiles2);
+      int64_t ctas = std::min<int64_t>(num_sms > 0 ? num_sms : rt.num_sms(), std::max<int64_t>(total, 1) * unit);
+      ctas = std::max<int64_t>(ctas / unit, 1) * unit;
+      if (rt.timing_.defined() && ctas <= rt.num_sms())
+        p.timing = reinterpret_cast<long long*>(rt.timing_.data_ptr<int64_t>()) + static_cast<int64_t>(kind) * rt.num_sms() * kTimingCols;
+      ++rt.launches_;
+      cudaError_t setup_error = cudaSuccess;
+      const bool launched = launch_grouped_gemm(p, &ta, &tb, have_o0 ? &to0 : nullptr, have_o1 ? &to1 : nullptr, nullptr, static_cast<int>(ctas),
+                                                rt.stream(), &setup_error, have_second ? second : nullptr);
+      SEP_ASSERT(launched, "no grouped GEMM kernel for this combination of mode, operand layouts and epilogue");
+      SEP_CUDA_CHECK(setup_error);
+      SEP_CUDA_CHECK(cudaGetLastError());
+    }
+  };
+
   // Work on pairs of row tiles with CTA pairs (see gemm_kernel.cuh) when the dispatch has a pair list worth using.
   static void use_pairs(GemmArgs& a, const DispatchState& st) {
     if (st.num_pairs > 0) { a.pair_tiles = st.pair_tiles; a.num_pairs = st.num_pairs; }
@@ -1590,8 +1858,22 @@ class Runtime {
   // The current torch stream; remembered so that released arena blocks wait for the work queued on it.
   at::cuda::CUDAStream stream() {
     auto s = at::cuda::getCurrentCUDAStream();
-    if (s.stream() != last_stream_) { release_ctx_->note_stream(s.stream()); last_stream_ = s.stream(); }
+    if (s.stream() != last_stream_.load(std::memory_order_relaxed)) {
+      release_ctx_->note_stream(s.stream());
+      last_stream_.store(s.stream(), std::memory_order_relaxed);
+    }
     return s;
+  }
+  // `waiter` goes on only after everything queued on `on` so far.  (One event per thread and device is enough: a wait
+  // refers to the record that was last made when the wait is issued.)
+  static void stream_wait(c10::cuda::CUDAStream waiter, c10::cuda::CUDAStream on) {
+    if (waiter.stream() == on.stream()) return;
+    thread_local cudaEvent_t events[64] = {};
+    cudaEvent_t& e = events[on.device_index()];
+    c10::cuda::CUDAGuard guard(on.device_index());
+    if (e == nullptr) SEP_CUDA_CHECK(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+    SEP_CUDA_CHECK(cudaEventRecord(e, on.stream()));
+    SEP_CUDA_CHECK(cudaStreamWaitEvent(waiter.stream(), e, 0));
   }
   void fill_peers(void** dst) const { for (int i = 0; i < kMaxRanks; ++i) dst[i] = peer_base_[i]; }
   void finish_sync() {
@@ -1621,7 +1903,7 @@ class Runtime {
   std::shared_ptr<Arena> arena_;
   std::shared_ptr<void> arena_guard_;
   std::shared_ptr<ReleaseCtx> release_ctx_;
-  cudaStream_t last_stream_ = reinterpret_cast<cudaStream_t>(-1);
+  std::atomic<cudaStream_t> last_stream_{reinterpret_cast<cudaStream_t>(-1)};   // (a backward may run on another host thread)
   void* peer_base_[kMaxRanks];
   bool opened_[kMaxRanks] = {false, false, false, false, false, false, false, false};
   bool use_vmm_ = false;
@@ -1639,7 +1921,7 @@ class Runtime {
   unsigned long long budget_ns_ = 0;
   int64_t timeout_ms_ = 0;
   int epochs_[kNumKinds];
-  int64_t launches_ = 0;
+  std::atomic<int64_t> launches_{0};
   int pairs_per_chunk_ = 8;
   int head_pairs_per_chunk_ = 2, head_chunks_ = 0;
   int push_ctas_ = 0;
@@ -1650,9 +1932,39 @@ class Runtime {
   at::Tensor router_tiles_;            // zeros: every M tile of the router GEMM belongs to "expert" 0
   int push_order_ = 0;
   std::shared_ptr<EventHandle> local_phase_;
+  std::mutex phase_mu_;
   at::Tensor timing_;
   int gate_issued_[8];
   bool available_ = false, destroyed_ = false;
+};
+
+// The single-rank layer as an autograd node of its own: neither direction goes through the interpreter.
+struct LocalLayerCall {
+  std::shared_ptr<Runtime> runtime;
+  int num_experts, level;
+  LayerConfig cfg;
+  c10::cuda::CUDAStream comp;
+};
+class LocalLayerFunction : public torch::autograd::Function<LocalLayerFunction> {
+ public:
+  static at::Tensor forward(torch::autograd::AutogradContext* ctx, const at::Tensor& x, const at::Tensor& weights, const at::Tensor& w1,
+                            const at::Tensor& w2, const at::Tensor& idx, const LocalLayerCall& call) {
+    auto r = call.runtime->local_forward(x, idx, weights, w1, w2, call.num_experts, call.level, call.cfg, true, call.comp);
+    r.second->runtime = call.runtime;
+    ctx->saved_data["state"] = c10::IValue::make_capsule(r.second);
+    ctx->saved_data["stream"] = static_cast<int64_t>(call.comp.id());
+    ctx->saved_data["device"] = static_cast<int64_t>(call.comp.device_index());
+    return r.first;
+  }
+  static torch::autograd::variable_list backward(torch::autograd::AutogradContext* ctx, torch::autograd::variable_list grads) {
+    SEP_ASSERT(ctx->saved_data.count("state"), "the backward of this layer has already run (its forward state is gone)");
+    auto st = c10::static_intrusive_pointer_cast<LocalState>(ctx->saved_data["state"].toCapsule());
+    const auto comp = c10::cuda::CUDAStream::unpack3(ctx->saved_data["stream"].toInt(),
+                                                     static_cast<c10::DeviceIndex>(ctx->saved_data["device"].toInt()), c10::DeviceType::CUDA);
+    ctx->saved_data.clear();
+    auto g = st->runtime->local_backward(*st, grads[0], comp);
+    return {g[0], g[1], g[2], g[3], at::Tensor(), at::Tensor()};
+  }
 };
 
 }  // namespace sep
@@ -1768,7 +2080,13 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
       RW(push_flags);
 #undef RW
 
-  py::class_<Runtime>(m, "Runtime")
+  py::class_<LayerConfig>(m, "LayerConfig")
+      .def(py::init([](int a, int y, int yb, int ab, int d1, int d2, int sa, int sy, int syb, int sab) {
+        return LayerConfig{a, y, yb, ab, d1, d2, sa, sy, syb, sab};
+      }));
+  py::class_<LocalState, c10::intrusive_ptr<LocalState>>(m, "LocalState");
+
+  py::class_<Runtime, std::shared_ptr<Runtime>>(m, "Runtime")
       .def(py::init<int, int, int64_t, int, int, int64_t, bool>(), py::arg("rank"), py::arg("num_ranks"), py::arg("arena_bytes"),
            py::arg("num_channels"), py::arg("num_experts_cap"), py::arg("timeout_ms"), py::arg("use_vmm") = false)
       .def("uses_vmm", &Runtime::uses_vmm)
@@ -1838,6 +2156,23 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
       .def("grouped_gemm", &Runtime::grouped_gemm)
       .def("mark_local_phase", &Runtime::mark_local_phase)
       .def("local_phase_event", &Runtime::local_phase_event)
+      // x, topk_idx, topk_weights, w1, w2, num_experts, level, config, stream id and device of the compute stream
+      .def("local_layer", [](const std::shared_ptr<Runtime>& r, const at::Tensor& x, const at::Tensor& idx, const at::Tensor& weights, const at::Tensor& w1,
+                             const at::Tensor& w2, int num_experts, int level, const LayerConfig& cfg, int64_t stream_id, int device) {
+        const auto comp = c10::cuda::CUDAStream::unpack3(stream_id, static_cast<c10::DeviceIndex>(device), c10::DeviceType::CUDA);
+        const bool differentiable = at::GradMode::is_enabled() &&
+                                    (x.requires_grad() || weights.requires_grad() || w1.requires_grad() || w2.requires_grad());
+        if (!differentiable) return r->local_forward(x, idx, weights, w1, w2, num_experts, level, cfg, false, comp).first;
+        return LocalLayerFunction::apply(x, weights, w1, w2, idx, LocalLayerCall{r, num_experts, level, cfg, comp});
+      })
+      .def("local_forward", [](const std::shared_ptr<Runtime>& r, const at::Tensor& x, const at::Tensor& idx, const at::Tensor& weights, const at::Tensor& w1,
+                               const at::Tensor& w2, int num_experts, int level, const LayerConfig& cfg, int64_t stream_id, int device) {
+        return r->local_forward(x, idx, weights, w1, w2, num_experts, level, cfg, true,
+                                c10::cuda::CUDAStream::unpack3(stream_id, static_cast<c10::DeviceIndex>(device), c10::DeviceType::CUDA));
+      })
+      .def("local_backward", [](const std::shared_ptr<Runtime>& r, LocalState& st, const at::Tensor& dy, int64_t stream_id, int device) {
+        return r->local_backward(st, dy, c10::cuda::CUDAStream::unpack3(stream_id, static_cast<c10::DeviceIndex>(device), c10::DeviceType::CUDA));
+      })
       .def("fused_forward", &Runtime::fused_forward)
       .def("fused_backward", &Runtime::fused_backward)
       .def("tile_producer", &Runtime::tile_producer)

@@ -24,6 +24,10 @@ default on):
               GEMM-A_bwd (+) combine_grads (remote red.add into the source's dL/dx)
               dW2, dW1 grouped GEMMs (true-length varlen-K)
 
+With a single rank nothing is exchanged and the fused plan is the native single-rank layer (``Runtime.local_layer``, an
+autograd node of its own): pairs sorted and rows copied into the pool by one or two kernels, then the same GEMM kernels
+without gates or pushes.
+
 *unfused* (the reference's plan, stream_ep/stream_moe/stream_moe.py:447-1175) -
 dispatch and combine are stand-alone kernels on the communicate stream, GEMMs on
 the compute stream, overlapped per tile / per token through ``pool_arrival_count``
@@ -38,6 +42,7 @@ from typing import Optional
 
 import torch
 
+from .. import _ext
 from ..ops import grouped_gemm as gg
 from .tile_config import TileConfig, _resolve_tile_config, default_tile_config  # noqa: F401
 
@@ -100,9 +105,17 @@ def moe_forward(ctx, streams, buffer, x, topk_idx, topk_weights, is_token_in_ran
     rt = buffer.runtime
     caller = torch.cuda.current_stream()
     comm, comp = streams.communicate, streams.compute
+    if fused and buffer.group_size == 1:
+        _nvtx_push(f"fwd_fused_{_NVTX_FWD}")
+        buffer._next_seq += 1
+        out, ctx.local = rt.local_forward(x, topk_idx, topk_weights, w1, w2, num_experts, level, _native_config(cfg),
+                                          comp.stream_id, comp.device_index)
+        ctx.buffer, ctx.streams, ctx.fused = buffer, streams, fused
+        _nvtx_pop()
+        _nvtx_pop()
+        return out
     x = x.contiguous()
     w1c, w2c = w1.contiguous(), w2.contiguous()
-
     comm.wait_stream(caller)
     comp.wait_stream(caller)
     if fused and not buffer._emulated:
@@ -253,6 +266,12 @@ def moe_backward(ctx, dL_dy):
     global _NVTX_BWD
     _NVTX_BWD += 1
     _nvtx_push(f"moe_bwd_{_NVTX_BWD}")
+    if ctx.fused and ctx.buffer.group_size == 1:
+        comp = ctx.streams.compute
+        grads = ctx.buffer.runtime.local_backward(ctx.local, dL_dy, comp.stream_id, comp.device_index)
+        ctx.local = None
+        _nvtx_pop()
+        return tuple(grads)
     buffer, streams, handle, cfg, level, fused = ctx.buffer, ctx.streams, ctx.handle, ctx.cfg, ctx.level, ctx.fused
     T, H, I, E_local = ctx.shapes
     sv = ctx.saved
@@ -397,6 +416,21 @@ def _launch_dw(buffer, handle, cfg, dl_do_pool, postact_dw2, dswiglu_in, pool, d
         dW2.zero_()
 
 
+def _native_config(cfg: TileConfig):
+    """The native form of a resolved tile configuration (kept: a program uses few)."""
+    native = _NATIVE_CONFIGS.get(cfg)
+    if native is None:
+        native = _ext.load().LayerConfig(cfg.tile_n_a, cfg.tile_n_y, cfg.tile_n_y_bwd, cfg.tile_n_a_bwd, cfg.tile_n_dW1, cfg.tile_n_dW2,
+                                         cfg.num_sms_a or 0, cfg.num_sms_y or 0, cfg.num_sms_y_bwd or 0, cfg.num_sms_a_bwd or 0)
+        if len(_NATIVE_CONFIGS) >= 256:
+            _NATIVE_CONFIGS.clear()
+        _NATIVE_CONFIGS[cfg] = native
+    return native
+
+
+_NATIVE_CONFIGS: dict = {}
+
+
 class StreamMoEFunc(torch.autograd.Function):
     """Autograd boundary of the layer (stream_ep/stream_moe/stream_moe.py:432-1175)."""
 
@@ -427,9 +461,20 @@ def stream_moe_func(buffer, x: torch.Tensor, topk_idx: torch.Tensor, topk_weight
     recomputes ``preact_a`` in backward; 2 keeps one compact row per recv token and re-expands the
     pool in backward.
     """
-    _, two_i, H = w1_local.shape
-    cfg = _resolve_tile_config(tile_config, two_i // 2, H)
+    E_local, two_i, H = w1_local.shape
+    I = two_i // 2
+    cfg = _resolve_tile_config(tile_config, I, H)
     if fused is None:
         fused = _fused_default()
+    if fused and buffer.group_size == 1 and not _NVTX_ENABLED:
+        level = activation_checkpoint_level
+        assert level in (0, 1, 2), "activation_checkpoint_level must be 0, 1 or 2"
+        assert x.dtype == torch.bfloat16 and w1_local.dtype == torch.bfloat16 and w2_local.dtype == torch.bfloat16, "bf16 only"
+        assert w2_local.shape == (E_local, H, I), f"w2_local must be [E_local, H, I], got {tuple(w2_local.shape)}"
+        assert num_experts == E_local
+        buffer._next_seq += 1
+        comp = streams.compute
+        return buffer.runtime.local_layer(x, topk_idx, topk_weights, w1_local, w2_local, num_experts, level, _native_config(cfg),
+                                          comp.stream_id, comp.device_index)
     return StreamMoEFunc.apply(streams, buffer, x, topk_idx, topk_weights, is_token_in_rank, w1_local, w2_local,
                                num_experts, cfg, activation_checkpoint_level, fused)

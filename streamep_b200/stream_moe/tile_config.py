@@ -19,6 +19,7 @@ memory, so
 from __future__ import annotations
 
 from dataclasses import dataclass, fields, replace
+from functools import lru_cache
 from typing import Optional
 
 _VALID_TILE_N = (128, 256)
@@ -91,8 +92,10 @@ def default_tile_config(I: int, H: int) -> TileConfig:
     )
 
 
+@lru_cache(maxsize=256)
 def _resolve_tile_config(tile_config: Optional[TileConfig], I: int, H: int) -> TileConfig:
-    """Overlay the caller's non-``None`` fields on the baseline and validate."""
+    """Overlay the caller's non-``None`` fields on the baseline and validate (once per configuration and shape: the layer
+    asks on every call)."""
     cfg = default_tile_config(I, H)
     if tile_config is not None:
         over = {f.name: getattr(tile_config, f.name) for f in fields(tile_config)
