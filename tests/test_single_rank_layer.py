@@ -29,7 +29,8 @@ def _run(T, H, I, E, K, seed, skip, level=0, capacity_factor=None):
     with torch.no_grad():
         plain = stream_moe_func(*args, streams=make_streams(), num_experts=E)
     torch.cuda.synchronize()
-    return buf, out, grads, plain, moe_reference_grads(x, idx, w, w1, w2, dy)
+    want = moe_reference_grads(x, idx, w, w1, w2, dy) if bool((idx >= 0).any()) else [torch.zeros_like(t) for t in (x, *leaves)]
+    return buf, out, grads, plain, want
 
 
 @pytest.mark.parametrize("T,H,I,E,K,skip,level", [
@@ -44,14 +45,17 @@ def _run(T, H, I, E, K, seed, skip, level=0, capacity_factor=None):
 def test_single_rank_layer(native, T, H, I, E, K, skip, level):
     buf, out, grads, plain, (want_out, *want) = _run(T, H, I, E, K, T + E, skip, level)
     buf.check_status()
+    # out and dx are sums of K rows, added one by one in bf16: every addition rounds by at most 2^-9 of the partial sum, which
+    # the largest result bounds (statistically; inputs are N(0, 1)), so K * 2^-9 once that exceeds the layer tolerance
+    sums = max(2e-2, K * 2.0 ** -9)
     for name, got, ref, tol in zip(("out", "dx", "dtopk_weights", "dW1", "dW2", "out without gradients"), (out, *grads, plain),
-                                   (want_out, *want, want_out), (2e-2, 2e-2, 2e-2, 3e-2, 3e-2, 2e-2)):
+                                   (want_out, *want, want_out), (sums, sums, 2e-2, 3e-2, 3e-2, sums)):
         check_close(name, got, ref, atol=tol * max(float(ref.abs().max()), 1e-6), rtol=tol)
 
 
 def test_single_rank_capacity_overflow_runs_empty(native):
-    buf, out, grads, _, _ = _run(500, 128, 64, 4, 2, 3, 0.0, capacity_factor=0.5)
-    assert float(out.abs().max()) == 0.0 and all(float(g.abs().max()) == 0.0 for g in grads)
+    buf, out, grads, _, _ = _run(2000, 128, 64, 4, 2, 3, 0.0, capacity_factor=0.5)
+    assert float(out.detach().abs().max()) == 0.0 and all(float(g.abs().max()) == 0.0 for g in grads)
     assert buf.overflow_info()["count"] == 2
     with pytest.raises(StreamEPOverflow, match="capacity overflow"):
         buf.check_status()
