@@ -26,7 +26,7 @@ _NAME = "_C"
 _lock = threading.Lock()
 _module = None
 
-SOURCES = ["runtime.cpp", "comm_kernels.cu", "local_kernels.cu", "gemm_kernels.cu", "gemm_inst_swiglu.cu", "gemm_inst_dswiglu.cu",
+SOURCES = ["runtime.cpp", "comm_kernels.cu", "local_kernels.cu", "router_kernels.cu", "gemm_kernels.cu", "gemm_inst_swiglu.cu", "gemm_inst_dswiglu.cu",
            "gemm_inst_scatter.cu", "gemm_inst_store.cu", "gemm_inst_dw.cu"]
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a",

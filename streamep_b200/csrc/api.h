@@ -302,15 +302,17 @@ struct RouterParams {
   float* probs;         // optional [T, E] softmax output (for the backward), may be null
 };
 void launch_router(const RouterParams& p, cudaStream_t stream);
-// Second half of the tensor-core router: softmax / top-k / rank bitmap from fp32 logits [T, ld_logits] that the
-// grouped GEMM wrote with its fp32 store epilogue (p.x / p.w_gate are not read).
-void launch_router_finish(const RouterParams& p, const float* logits, int ld_logits, cudaStream_t stream);
+// The tensor-core router in one launch: `map_w` [E, H] with boxes of 128 x 64 and `map_x` [T, H] with boxes of
+// router_tile_tokens() x 64 elements, both bf16 with 128-byte swizzle (p.x / p.w_gate are not read).
+int router_tile_tokens(const RouterParams& p, int sms);
+cudaError_t launch_router_mma(const RouterParams& p, const void* map_w, const void* map_x, int sms, StatusBlock* status,
+                              unsigned long long wait_budget_ns, cudaStream_t stream);
 
 // ---------------------------------------------------------------------------------------------
 // Grouped GEMM on tcgen05 / TMEM
 // ---------------------------------------------------------------------------------------------
 enum GemmMode : int { kVarlenM = 0, kVarlenK = 1 };
-enum GemmEpilogue : int { kEpiStore = 0, kEpiSwiglu = 1, kEpiScatter = 2, kEpiDswiglu = 3, kEpiStoreF32 = 4 };
+enum GemmEpilogue : int { kEpiStore = 0, kEpiSwiglu = 1, kEpiScatter = 2, kEpiDswiglu = 3 };
 
 struct TailSignal {              // end-of-kernel "all my remote writes are done" handshake
   int enabled;

@@ -858,213 +858,4 @@ void launch_combine_reduce(void* out, const void* rows, const long long* topk_id
                                                   dw_src, dw_dst, skip_rows);
 }
 
-// =============================================================================================
-// Router: logits = x @ w_gate^T, softmax, top-k, renormalise, rank bitmap.  One warp per token.
-// The reference has no router; its harnesses build routing with torch ops
-// (stream_ep/stream_moe/profile_pipeline.py:102-139).
-// =============================================================================================
-constexpr int kRouterMaxExpertsPerLane = 16;   // up to 512 experts
-constexpr int kRouterKChunk = 64;              // hidden elements per shared-memory step (128 bytes of a row)
-constexpr int kRouterLd = kRouterKChunk + 4;   // padded row: float4 reads of 8 consecutive rows hit 32 different banks
-
-// One warp finishes one token from its fp32 logits (shared or global memory): softmax over all experts, top-k by
-// repeated arg-max (ties -> lowest expert id), renormalise, rank bitmap.  EPL = experts per lane.
-template <int EPL>
-__device__ __forceinline__ void route_token(const RouterParams& p, const float* row, int t, int lane) {
-  const int E = p.num_experts, K = p.num_topk;
-  const int e_local = E / p.num_ranks;
-  float logit[EPL];
-  float mx = -INFINITY;
-#pragma unroll
-  for (int j = 0; j < EPL; ++j) {
-    const int e = j * 32 + lane;
-    logit[j] = (e < E) ? row[e] : -INFINITY;
-    mx = fmaxf(mx, logit[j]);
-  }
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
-  float sum = 0.f;
-#pragma unroll
-  for (int j = 0; j < EPL; ++j) {
-    const int e = j * 32 + lane;
-    logit[j] = (e < E) ? __expf(logit[j] - mx) : 0.f;
-    sum += logit[j];
-  }
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
-  const float inv = 1.f / sum;
-#pragma unroll
-  for (int j = 0; j < EPL; ++j) {
-    logit[j] *= inv;
-    const int e = j * 32 + lane;
-    if (p.probs != nullptr && e < E) p.probs[static_cast<size_t>(t) * E + e] = logit[j];
-  }
-  // top-k by repeated arg-max (ties -> lowest expert id)
-  float wsum = 0.f, my_w = 0.f;
-  int my_e = -1;
-  unsigned rank_mask = 0;
-  for (int k = 0; k < K; ++k) {
-    float best = -1.f; int best_e = 0x7fffffff;
-#pragma unroll
-    for (int j = 0; j < EPL; ++j) {
-      const int e = j * 32 + lane;
-      if (e < E && logit[j] > best) { best = logit[j]; best_e = e; }
-    }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-      const float ob = __shfl_xor_sync(0xffffffffu, best, o);
-      const int oe = __shfl_xor_sync(0xffffffffu, best_e, o);
-      if (ob > best || (ob == best && oe < best_e)) { best = ob; best_e = oe; }
-    }
-#pragma unroll
-    for (int j = 0; j < EPL; ++j)
-      if (j * 32 + lane == best_e) logit[j] = -2.f;
-    if (lane == k) { my_w = best; my_e = best_e; }
-    wsum += best;
-    rank_mask |= 1u << (best_e / e_local);
-  }
-  if (lane < K) {
-    p.topk_idx[static_cast<size_t>(t) * K + lane] = my_e;
-    p.topk_weights[static_cast<size_t>(t) * K + lane] = p.renormalize ? my_w / wsum : my_w;
-  }
-  if (lane < p.num_ranks && p.is_token_in_rank != nullptr)
-    p.is_token_in_rank[static_cast<size_t>(t) * p.num_ranks + lane] = (rank_mask >> lane) & 1u;
-}
-
-// One CTA routes TOK tokens with TOK * 4 threads.  Logits: a register-tiled fp32 GEMM, (TOK / 4) x 16 threads
-// with 4 tokens x JE experts each, so one pass covers 16 * JE experts (16 / 32 / 64; wider expert counts loop).
-// Operands are fetched 128 contiguous bytes per row (8 lanes per row), converted to fp32 and kept row-major in
-// shared memory; the global loads of the next two chunks are in flight while the current one is multiplied.
-// Few experts make the kernel latency-bound, so those instances use 32 tokens per CTA (twice the CTAs); 64
-// experts per pass are FMA-bound and use 64 tokens for operand reuse.  Then each warp finishes 8 tokens:
-// softmax over all experts, top-k by repeated arg-max, renormalise, rank bitmap.
-template <int JE, int TOK>
-__global__ void __launch_bounds__(TOK * 4) router_kernel(const RouterParams p) {
-  constexpr int THREADS = TOK * 4;
-  constexpr int NE = 16 * JE;                                      // experts per pass
-  constexpr int EPL = JE == 4 ? kRouterMaxExpertsPerLane : 1;      // experts per lane in the softmax / top-k part
-  constexpr int XV = TOK * 8 / THREADS;                            // 16-byte loads of x per thread and chunk (2)
-  constexpr int WV = (NE * 8 + THREADS - 1) / THREADS;             // ... of the gate weights (1 or 2)
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  float* xs = reinterpret_cast<float*>(smem_raw);                 // [TOK tokens][kRouterLd]
-  float* ws = xs + TOK * kRouterLd;                               // [NE experts][kRouterLd]
-  float* logits = ws + NE * kRouterLd;                            // [TOK tokens][e_pad]
-  const int E = p.num_experts, H = p.hidden;
-  const int e_pad = (E + NE - 1) / NE * NE + 1;                   // +1: rows start in different banks
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int ty = tid >> 4, tx = tid & 15;
-  const __nv_bfloat16* xg = static_cast<const __nv_bfloat16*>(p.x);
-  const __nv_bfloat16* wg = static_cast<const __nv_bfloat16*>(p.w_gate);
-  const int t0 = blockIdx.x * TOK;
-
-  for (int e0 = 0; e0 < E; e0 += NE) {
-    float acc[4][JE];
-#pragma unroll
-    for (int i = 0; i < 4; ++i)
-#pragma unroll
-      for (int j = 0; j < JE; ++j) acc[i][j] = 0.f;
-    uint4 xv0[XV], wv0[WV], xv1[XV], wv1[WV];
-    auto fetch = [&](int k0, uint4 (&xv)[XV], uint4 (&wv)[WV]) {
-#pragma unroll
-      for (int i = 0; i < XV; ++i) {
-        const int idx = tid + THREADS * i, row = idx >> 3, kk = k0 + (idx & 7) * 8;
-        xv[i] = (t0 + row < p.num_tokens && kk < H) ? ld_nc_v4(xg + static_cast<size_t>(t0 + row) * H + kk)
-                                                    : make_uint4(0, 0, 0, 0);
-      }
-#pragma unroll
-      for (int i = 0; i < WV; ++i) {
-        const int idx = tid + THREADS * i, row = idx >> 3, kk = k0 + (idx & 7) * 8;
-        wv[i] = (row < NE && e0 + row < E && kk < H)
-                    ? __ldg(reinterpret_cast<const uint4*>(wg + static_cast<size_t>(e0 + row) * H + kk))
-                    : make_uint4(0, 0, 0, 0);
-      }
-    };
-    auto stash1 = [&](float* dst, const uint4& v, int idx) {
-      const float2 a = unpack_bf16x2(v.x), b = unpack_bf16x2(v.y), c = unpack_bf16x2(v.z), d = unpack_bf16x2(v.w);
-      float4* o = reinterpret_cast<float4*>(dst + (idx >> 3) * kRouterLd + (idx & 7) * 8);
-      o[0] = make_float4(a.x, a.y, b.x, b.y);
-      o[1] = make_float4(c.x, c.y, d.x, d.y);
-    };
-    // one chunk: registers -> shared memory, refill the registers two chunks ahead, multiply
-    auto chunk = [&](int k_next, uint4 (&xv)[XV], uint4 (&wv)[WV]) {
-      __syncthreads();   // the previous chunk's tiles are no longer read
-#pragma unroll
-      for (int i = 0; i < XV; ++i) stash1(xs, xv[i], tid + THREADS * i);
-#pragma unroll
-      for (int i = 0; i < WV; ++i)
-        if (tid + THREADS * i < NE * 8) stash1(ws, wv[i], tid + THREADS * i);
-      __syncthreads();
-      if (k_next < H) fetch(k_next, xv, wv);                       // in flight during this and the next multiply
-#pragma unroll 4
-      for (int k = 0; k < kRouterKChunk; k += 4) {
-        float4 a[4], b[JE];
-#pragma unroll
-        for (int i = 0; i < 4; ++i) a[i] = *reinterpret_cast<const float4*>(xs + (ty * 4 + i) * kRouterLd + k);
-#pragma unroll
-        for (int j = 0; j < JE; ++j) b[j] = *reinterpret_cast<const float4*>(ws + (j * 16 + tx) * kRouterLd + k);   // lanes on consecutive rows: no bank conflict
-#pragma unroll
-        for (int i = 0; i < 4; ++i)
-#pragma unroll
-          for (int j = 0; j < JE; ++j) {
-            acc[i][j] = fmaf(a[i].x, b[j].x, acc[i][j]);
-            acc[i][j] = fmaf(a[i].y, b[j].y, acc[i][j]);
-            acc[i][j] = fmaf(a[i].z, b[j].z, acc[i][j]);
-            acc[i][j] = fmaf(a[i].w, b[j].w, acc[i][j]);
-          }
-      }
-    };
-    fetch(0, xv0, wv0);
-    if (kRouterKChunk < H) fetch(kRouterKChunk, xv1, wv1);
-    for (int k0 = 0; k0 < H; k0 += 2 * kRouterKChunk) {
-      chunk(k0 + 2 * kRouterKChunk, xv0, wv0);
-      if (k0 + kRouterKChunk >= H) break;
-      chunk(k0 + 3 * kRouterKChunk, xv1, wv1);
-    }
-#pragma unroll
-    for (int i = 0; i < 4; ++i)
-#pragma unroll
-      for (int j = 0; j < JE; ++j) logits[(ty * 4 + i) * e_pad + e0 + j * 16 + tx] = acc[i][j];
-  }
-  __syncthreads();
-
-  for (int tt = warp; tt < TOK; tt += THREADS / 32) {
-    const int t = t0 + tt;
-    if (t >= p.num_tokens) break;
-    route_token<EPL>(p, logits + tt * e_pad, t, lane);
-  }
-}
-
-// Second half of the tensor-core router: one warp per token reads the fp32 logits the grouped GEMM stored.
-template <int EPL>
-__global__ void __launch_bounds__(256) router_finish_kernel(const RouterParams p, const float* __restrict__ logits, int ld) {
-  const int lane = threadIdx.x & 31;
-  const int t = blockIdx.x * 8 + (threadIdx.x >> 5);
-  if (t >= p.num_tokens) return;
-  route_token<EPL>(p, logits + static_cast<size_t>(t) * ld, t, lane);
-}
-
-void launch_router_finish(const RouterParams& p, const float* logits, int ld_logits, cudaStream_t stream) {
-  const int grid = (p.num_tokens + 7) / 8;
-  if (p.num_experts <= 32) router_finish_kernel<1><<<grid, 256, 0, stream>>>(p, logits, ld_logits);
-  else if (p.num_experts <= 128) router_finish_kernel<4><<<grid, 256, 0, stream>>>(p, logits, ld_logits);
-  else router_finish_kernel<kRouterMaxExpertsPerLane><<<grid, 256, 0, stream>>>(p, logits, ld_logits);
-}
-
-template <int JE, int TOK>
-static void launch_router_je(const RouterParams& p, cudaStream_t stream) {
-  constexpr int NE = 16 * JE;
-  const int e_pad = (p.num_experts + NE - 1) / NE * NE + 1;
-  const size_t smem = sizeof(float) * (static_cast<size_t>(TOK + NE) * kRouterLd + static_cast<size_t>(TOK) * e_pad);
-  const int grid = (p.num_tokens + TOK - 1) / TOK;
-  if (smem > 48 * 1024)
-    cudaFuncSetAttribute(router_kernel<JE, TOK>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
-  router_kernel<JE, TOK><<<grid, TOK * 4, smem, stream>>>(p);
-}
-
-void launch_router(const RouterParams& p, cudaStream_t stream) {
-  if (p.num_experts <= 16) launch_router_je<1, 32>(p, stream);
-  else if (p.num_experts <= 32) launch_router_je<2, 32>(p, stream);
-  else launch_router_je<4, 64>(p, stream);
-}
-
 }  // namespace sep

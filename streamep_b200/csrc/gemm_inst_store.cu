@@ -1,4 +1,4 @@
-// Instances of the grouped GEMM with the store epilogues over row tiles: preact recompute (bf16) and router logits (fp32).
+// Instances of the grouped GEMM with the plain store epilogue over row tiles (preact recompute).
 #include "gemm_kernel.cuh"
 
 namespace sep {
@@ -10,12 +10,8 @@ static cudaError_t launch_width(const GemmParams& p, const LaunchMaps& m, int n,
 }
 
 cudaError_t launch_store(const GemmParams& p, const LaunchMaps& m, const PushParams* push, int n, cudaStream_t s, bool& handled) {
-  handled = p.mode == kVarlenM && !p.a_mn_major && push == nullptr && (p.epilogue == kEpiStore || (!p.b_mn_major && !p.pair_ctas));
+  handled = p.mode == kVarlenM && !p.a_mn_major && push == nullptr;
   if (!handled) return cudaSuccess;
-  if (p.epilogue == kEpiStoreF32) {
-    return p.block_n == 128 ? launch_instance<128, false, false, kEpiStoreF32, false, 1>(p, m, PushParams{}, n, s)
-                            : launch_instance<256, false, false, kEpiStoreF32, false, 1>(p, m, PushParams{}, n, s);
-  }
   if (p.block_n == 128) return launch_width<128, 1>(p, m, n, s);
   return p.pair_ctas ? launch_width<256, 2>(p, m, n, s) : launch_width<256, 1>(p, m, n, s);
 }

@@ -675,15 +675,6 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
             }
             __syncwarp();
           }
-        } else if (EPI == kEpiStoreF32) {
-          // fp32 accumulator values as they are (router logits): a thread owns a row, so its 32 columns are
-          // one full 128-byte line of the output row.  Rows past the end of A are TMA zero fill: not stored.
-          if (grow < p.total_rows) {
-            float* dst = static_cast<float*>(p.out0) + grow * p.ld0 + n;
-#pragma unroll
-            for (int q = 0; q < 8; ++q)
-              if (n + q * 4 < p.N) st_global_v4(dst + q * 4, r[q * 4], r[q * 4 + 1], r[q * 4 + 2], r[q * 4 + 3]);
-          }
         } else {   // kEpiDswiglu: r = g[row, n..n+32) = dL/d(postact) before the topk weight
           uint32_t o_pw[16];
           unsigned char* sb = epi_stage + (warp - 2) * Cfg::kEpiStageBytes;

@@ -244,6 +244,11 @@ __device__ __forceinline__ void st_cluster(uint32_t cluster_addr, int v) {
 __device__ __forceinline__ void st_release_cluster(uint32_t cluster_addr, int v) {
   asm volatile("st.release.cluster.shared::cluster.s32 [%0], %1;" :: "r"(cluster_addr), "r"(v) : "memory");
 }
+__device__ __forceinline__ float ld_cluster_f32(uint32_t cluster_addr) {
+  float v;
+  asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(cluster_addr) : "memory");
+  return v;
+}
 __device__ __forceinline__ int ld_acquire_cluster_shared(const int* p) {
   int v;
   asm volatile("ld.acquire.cluster.shared::cta.s32 %0, [%1];" : "=r"(v) : "r"(smem_u32(p)) : "memory");

@@ -1205,8 +1205,7 @@ class Runtime : public std::enable_shared_from_this<Runtime> {
         p.pair_ctas = 1; p.pair_tiles = a.pair_tiles->data_ptr<int>();
         if (a.num_m_tiles != 0) p.num_m_tiles = a.num_pairs;
       }
-      // (the fp32-store epilogue guards rows itself: its last tile may hang over the end of A, TMA zero-fills it)
-      SEP_ASSERT(static_cast<int64_t>(p.num_m_tiles) * BM_ <= rows || a.epilogue == kEpiStoreF32, "tile list longer than A");
+      SEP_ASSERT(static_cast<int64_t>(p.num_m_tiles) * BM_ <= rows, "tile list longer than A");
       p.num_n_tiles = (N + BN - 1) / BN;
       p.tile_id_to_expert = a.tile_id_to_expert->data_ptr<int>();
       if (a.num_m_tiles_dev.has_value()) p.num_m_tiles_dev = a.num_m_tiles_dev->data_ptr<int>() + (p.pair_ctas ? 3 : 0);
@@ -1300,8 +1299,7 @@ class Runtime : public std::enable_shared_from_this<Runtime> {
         SEP_ASSERT(p.row_src != nullptr && p.row_k_slot != nullptr && p.tile_stripes_done != nullptr && p.dl_dweight != nullptr,
                    "dL/dweight return needs pool_src, pool_k_slot, stripe counters and dl_dweight");
     }
-    if (a.epilogue == kEpiSwiglu || a.epilogue == kEpiStore || a.epilogue == kEpiStoreF32) SEP_ASSERT(p.out0 != nullptr, "this epilogue needs out0");
-    if (a.epilogue == kEpiStoreF32) SEP_ASSERT(a.out0->scalar_type() == at::kFloat && p.ld0 % 4 == 0, "the fp32 store epilogue writes float rows of a multiple of 4 elements");
+    if (a.epilogue == kEpiSwiglu || a.epilogue == kEpiStore) SEP_ASSERT(p.out0 != nullptr, "this epilogue needs out0");
     if (a.tail) {
       p.tail.enabled = 1; p.tail.kind = a.tail_kind; p.tail.epoch = ++epochs_[a.tail_kind];
       p.tail.wait = a.tail_wait ? 1 : 0;
@@ -1829,28 +1827,20 @@ class Runtime : public std::enable_shared_from_this<Runtime> {
     p.is_token_in_rank = reinterpret_cast<unsigned char*>(in_rank.data_ptr<bool>());
     p.probs = want_probs ? probs.data_ptr<float>() : nullptr;
     if (p.num_tokens > 0) {
-      const int64_t T = x.size(0), E = w_gate.size(0);
-      if (router_on_tensor_cores_ && E % 8 == 0 && E <= 256 && x.size(1) % 64 == 0) {
-        // Logits on the tensor cores: the grouped GEMM with x as the only "expert group" and W_gate as its weight,
-        // fp32 accumulators stored as they are (bf16 x bf16 products are exact in fp32, so this matches an fp32
-        // GEMM up to summation order); then one warp per token for softmax / top-k.
-        const int64_t tiles = (T + BM_ - 1) / BM_;
-        if (!router_tiles_.defined() || router_tiles_.numel() < tiles)
-          router_tiles_ = at::zeros({std::max<int64_t>(tiles, 64)}, x.options().dtype(at::kInt));
-        at::Tensor logits = at::empty({T, E}, x.options().dtype(at::kFloat));
-        GemmArgs g;
-        g.mode = kVarlenM; g.epilogue = kEpiStoreF32; g.block_n = E > 128 ? 256 : 128;
-        g.a = x; g.b = w_gate.unsqueeze(0); g.tile_id_to_expert = router_tiles_.narrow(0, 0, tiles); g.out0 = logits;
-        grouped_gemm(g);
-        ++launches_; launch_router_finish(p, logits.data_ptr<float>(), static_cast<int>(E), stream());
+      ++launches_;
+      if (router_on_tensor_cores_) {
+        const int64_t T = x.size(0), H = x.size(1), E = w_gate.size(0);
+        const CUtensorMap mw = make_tmap(w_gate.data_ptr(), H, E, 1, H, E * H, 64, 128);
+        const CUtensorMap mx = make_tmap(x.data_ptr(), H, T, 1, H, T * H, 64, router_tile_tokens(p, num_sms()));
+        SEP_CUDA_CHECK(launch_router_mma(p, &mw, &mx, num_sms(), status_, budget_ns_, stream()));
       } else {
-        ++launches_; launch_router(p, stream());
+        launch_router(p, stream());
       }
     }
     SEP_CUDA_CHECK(cudaGetLastError());
     return {idx, w, in_rank, probs};
   }
-  // false: always the SIMT router kernel (also used for expert counts the GEMM path does not take)
+  // false: the SIMT router kernel
   void set_router_on_tensor_cores(bool on) { router_on_tensor_cores_ = on; }
 
  private:
@@ -1889,9 +1879,8 @@ class Runtime : public std::enable_shared_from_this<Runtime> {
   }
   int num_sms() {
     if (num_sms_ == 0) {
-      cudaDeviceProp prop;
-      SEP_CUDA_CHECK(cudaGetDeviceProperties(&prop, device_));
-      num_sms_ = prop.multiProcessorCount;
+      // (not cudaGetDeviceProperties: it takes milliseconds, in the first call on every new buffer)
+      SEP_CUDA_CHECK(cudaDeviceGetAttribute(&num_sms_, cudaDevAttrMultiProcessorCount, device_));
     }
     return num_sms_;
   }
@@ -1929,7 +1918,6 @@ class Runtime : public std::enable_shared_from_this<Runtime> {
   bool split_local_ = false;
   int active_push_warps_ = 0;
   bool router_on_tensor_cores_ = true;
-  at::Tensor router_tiles_;            // zeros: every M tile of the router GEMM belongs to "expert" 0
   int push_order_ = 0;
   std::shared_ptr<EventHandle> local_phase_;
   std::mutex phase_mu_;
