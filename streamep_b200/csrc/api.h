@@ -272,8 +272,9 @@ void launch_tile_producer(int* count, const int* target, int num_tiles, long lon
 
 // Row gather/scatter between the padded pool and the compact per-recv-token matrix
 // (reference: stream_ep/stream_moe/recv_pool_compress.py:29-78).
-void launch_pool_compress(const void* pool, void* recv, const int* pool_recv_token, int tk_padded,
-                          int hidden, cudaStream_t stream);
+// `owner`: scratch of num_recv ints.
+void launch_pool_compress(const void* pool, void* recv, const int* pool_recv_token, int* owner, int tk_padded,
+                          int num_recv, int hidden, cudaStream_t stream);
 void launch_pool_expand(const void* recv, void* pool, const int* pool_recv_token, int tk_padded,
                         int hidden, cudaStream_t stream);
 

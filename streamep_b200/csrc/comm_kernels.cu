@@ -256,11 +256,12 @@ __global__ void __launch_bounds__(kMetaThreads, 1) dispatch_metadata_kernel(cons
     if (lane == 0) s_hist[e] = acc;
   }
   // tokens from s to d
-  if (tid < R * R) {
-    const int s = tid / R, d = tid % R;
+  for (int i = warp; i < R * R; i += num_warps) {     // (a warp each: one thread would wait for one load per channel)
+    const int s = i / R, d = i % R;
     int acc = 0;
-    for (int c = 0; c < C; ++c) acc += ctl_inbox_tokens(own, p.ctl, parity, s, c)[d];
-    s_U[s][d] = acc;
+    for (int c = lane; c < C; c += 32) acc += ctl_inbox_tokens(own, p.ctl, parity, s, c)[d];
+    acc = __reduce_add_sync(0xffffffffu, acc);
+    if (lane == 0) s_U[s][d] = acc;
   }
   __syncthreads();
   // 2. per-owner tile offsets
@@ -399,7 +400,13 @@ __global__ void __launch_bounds__(kMetaThreads, 1) dispatch_metadata_kernel(cons
     __syncthreads();
     for (int e = tid; e < E; e += blockDim.x) {
       int cnt = 0;
-      for (int c = 0; c < C; ++c) cnt += ctl_inbox_counts(own, p.ctl, parity, p.rank, c)[e];
+      for (int c0 = 0; c0 < C; c0 += 8) {     // eight loads in flight
+        int v[8];
+#pragma unroll
+        for (int j = 0; j < 8; ++j) v[j] = (c0 + j < C) ? ctl_inbox_counts(own, p.ctl, parity, p.rank, c0 + j)[e] : 0;
+#pragma unroll
+        for (int j = 0; j < 8; ++j) cnt += v[j];
+      }
       const int d = e / EL, el = e - d * EL;
       s_hist[el * R + ((d - p.rank + R) % R)] = cnt;     // keyed by push order
     }
@@ -602,20 +609,77 @@ __global__ void __launch_bounds__(kPushThreads, 1) dispatch_push_kernel(const Pu
   }
 }
 
+// The push of a single rank: every pair of a token lands in this rank's pool, so a warp takes whole tokens, reads each row
+// once and stores it once per pair, where the general kernel reads a row per pair.  Bound by the pool's writes to HBM; the
+// caller's SM budget (80 blocks by default) asks for as many bytes in flight per SM as it can hold: 32 warps, 4 KB each.
+// 4096 tokens x 8 pairs, hidden 7168, 80 blocks: 173 -> 135 us.
+constexpr int kLocalPushThreads = 1024;
+constexpr int kLocalPushPairs = 16;     // pairs a warp copies between two releases of their tiles
+
+__global__ void __launch_bounds__(kLocalPushThreads, 1) dispatch_push_local_kernel(const PushParams p) {
+  __shared__ PushTargets tg;
+  const int tid = threadIdx.x, lane = tid & 31, K = p.num_topk;
+  if (blockIdx.x == 0 && tid == 0 && p.started_flag != nullptr) atomicAdd(p.started_flag, 1);
+  if ((p.flags & 1) && !p.static_targets && blockIdx.x == 0 && tid == 0)
+    publish_record(p.own, p.peer_base, p.ctl, p.kind, p.epoch, p.rank, 0);
+  if (tid == 0) resolve_push_targets(tg, 0, p.peer_base[0], reinterpret_cast<const unsigned long long*>(&p.own));
+  __syncthreads();
+  if (!(p.flags & 2) || *p.num_send <= 0) return;       // (no pair, or the metadata kernel gave up)
+  const int vecs = p.hidden / 8;
+  const size_t row_bytes = static_cast<size_t>(p.hidden) * 2;
+  const int chunk = max(1, kLocalPushPairs / K);        // tokens
+  const int warps = gridDim.x * (kLocalPushThreads / 32);
+  for (int t0 = (blockIdx.x * (kLocalPushThreads / 32) + (tid >> 5)) * chunk; t0 < p.num_tokens; t0 += warps * chunk) {
+    const int t1 = min(t0 + chunk, p.num_tokens);
+    for (int t = t0; t < t1; ++t) {
+      const int slot = lane < K ? p.pair_slot[static_cast<size_t>(t) * K + lane] : -1;
+      const char* src = static_cast<const char*>(p.x) + t * row_bytes;
+      for (int v0 = 0; v0 < vecs; v0 += 256) copy_row_piece<8>(src, tg.pool[0], nullptr, v0, vecs, K, slot, lane);
+      const unsigned valid = __ballot_sync(0xffffffffu, slot >= 0);
+      if (!p.is_grads && valid != 0) {
+        const int r = p.send_recv_token[t];
+        if (slot >= 0) {
+          tg.pool_topk_weight[0][slot] = p.topk_weights[static_cast<size_t>(t) * K + lane];
+          tg.pool_recv_token[0][slot] = r;
+          tg.pool_k_slot[0][slot] = lane;
+          tg.pool_src[0][slot] = make_int2(p.rank, t);
+          tg.recv_token_to_slots[0][static_cast<size_t>(r) * K + lane] = slot;     // skipped k stay -1
+        }
+        if (lane == 0) {
+          tg.k_local_total[0][r] = __popc(valid);
+          tg.k_local_remaining[0][r] = __popc(valid);
+          tg.recv_src[0][r] = make_int2(p.rank, t);
+        }
+      }
+    }
+    __syncwarp();
+    for (int i = lane; i < (t1 - t0) * K; i += 32) {    // release the chunk's pairs (same GPU: device scope)
+      const int slot = p.pair_slot[static_cast<size_t>(t0) * K + i];
+      if (slot >= 0) red_release_gpu_add(tg.arrival_count[0] + slot / p.tile_m, 1);
+    }
+  }
+}
+
 void launch_dispatch_push(const PushParams& p, int num_blocks, cudaStream_t stream) {
-  dispatch_push_kernel<<<num_blocks, kPushThreads, 0, stream>>>(p);
+  if (p.num_ranks == 1) dispatch_push_local_kernel<<<num_blocks, kLocalPushThreads, 0, stream>>>(p);
+  else dispatch_push_kernel<<<num_blocks, kPushThreads, 0, stream>>>(p);
 }
 
 // =============================================================================================
 // Pull combine
 // =============================================================================================
-constexpr int kCombineThreads = 512;
-constexpr int kPullUnroll = 2;          // 16-byte loads in flight per lane and contributing rank
+// 16-byte loads in flight per lane and contributing rank, and threads of a block: one rank alone has no round trip over
+// NVLink to hide behind the other ranks' loads, so it takes a row in larger pieces and twice the warps (the caller's SM
+// budget sets the blocks).  4096 tokens, hidden 7168, 80 blocks, one rank: 84 -> 39 us.
+constexpr int pull_unroll(int ranks) { return ranks == 1 ? 4 : 2; }
+constexpr int combine_threads(int ranks) { return ranks == 1 ? 1024 : 512; }
 
-__global__ void __launch_bounds__(kCombineThreads, 1) combine_pull_kernel(const CombineParams p) {
-  __shared__ const char* s_x[kMaxRanks];
-  __shared__ const long long* s_done[kMaxRanks];
-  __shared__ const float* s_w[kMaxRanks];
+template <int NR>      // 1, or kMaxRanks for any number
+__global__ void __launch_bounds__(combine_threads(NR), 1) combine_pull_kernel(const CombineParams p) {
+  constexpr int U = pull_unroll(NR);
+  __shared__ const char* s_x[NR];
+  __shared__ const long long* s_done[NR];
+  __shared__ const float* s_w[NR];
   __shared__ int s_ok;
   __shared__ int s_is_last;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -646,7 +710,11 @@ __global__ void __launch_bounds__(kCombineThreads, 1) combine_pull_kernel(const 
     const size_t row_bytes = static_cast<size_t>(p.hidden) * 2;
     const int vec_per_row = p.hidden / 8;
     if (s_ok) {
-      for (int t = blockIdx.x * warps_per_block + warp; t < p.num_tokens; t += gridDim.x * warps_per_block) {
+      // a warp takes a piece of one token's row
+      const int pieces = NR == 1 ? max(1, (vec_per_row + 32 * U - 1) / (32 * U)) : 1;
+      const long long items = static_cast<long long>(p.num_tokens) * pieces;
+      for (long long item = blockIdx.x * warps_per_block + warp; item < items; item += gridDim.x * warps_per_block) {
+        const int t = static_cast<int>(item / pieces), piece = static_cast<int>(item - static_cast<long long>(t) * pieces);
         int my_r = -1;
         if (lane < R) my_r = p.send_recv_token[static_cast<size_t>(t) * R + lane];
         // gate: every contributing rank must have stamped its row
@@ -658,33 +726,33 @@ __global__ void __launch_bounds__(kCombineThreads, 1) combine_pull_kernel(const 
                                   static_cast<int>(p.seq), static_cast<int>(ld_acquire_sys(g)));
         }
         if (!__all_sync(0xffffffffu, ok)) break;
-        // Every contributing rank's row address, warp-uniform; a lane then keeps kPullUnroll x R
+        // Every contributing rank's row address, warp-uniform; a lane then keeps U x R
         // predicated 16-byte loads in flight so that the NVLink round trip is paid once per batch,
         // not once per load.
-        const char* src[kMaxRanks];
+        const char* src[NR];
 #pragma unroll
-        for (int d = 0; d < kMaxRanks; ++d) {
+        for (int d = 0; d < NR; ++d) {
           const int r = __shfl_sync(0xffffffffu, my_r, d);
           src[d] = (d < R && r >= 0) ? s_x[d] + static_cast<size_t>(r) * row_bytes : nullptr;
         }
         char* out_row = static_cast<char*>(p.out) + static_cast<size_t>(t) * row_bytes;
-        for (int v0 = lane; v0 < vec_per_row; v0 += 32 * kPullUnroll) {
-          uint4 q[kPullUnroll][kMaxRanks];
+        for (int v0 = piece * 32 * U + lane; v0 < vec_per_row; v0 += pieces * 32 * U) {
+          uint4 q[U][NR];
 #pragma unroll
-          for (int j = 0; j < kPullUnroll; ++j) {
+          for (int j = 0; j < U; ++j) {
             const int v = v0 + 32 * j;
 #pragma unroll
-            for (int d = 0; d < kMaxRanks; ++d)
+            for (int d = 0; d < NR; ++d)
               q[j][d] = (src[d] != nullptr && v < vec_per_row) ? ld_relaxed_sys_v4(src[d] + static_cast<size_t>(v) * 16)
                                                               : make_uint4(0, 0, 0, 0);
           }
 #pragma unroll
-          for (int j = 0; j < kPullUnroll; ++j) {
+          for (int j = 0; j < U; ++j) {
             const int v = v0 + 32 * j;
             if (v >= vec_per_row) break;
             float acc[8] = {0, 0, 0, 0, 0, 0, 0, 0};
 #pragma unroll
-            for (int d = 0; d < kMaxRanks; ++d) {
+            for (int d = 0; d < NR; ++d) {
               const float2 a = unpack_bf16x2(q[j][d].x), b = unpack_bf16x2(q[j][d].y), c = unpack_bf16x2(q[j][d].z),
                            e = unpack_bf16x2(q[j][d].w);
               acc[0] += a.x; acc[1] += a.y; acc[2] += b.x; acc[3] += b.y;
@@ -696,7 +764,7 @@ __global__ void __launch_bounds__(kCombineThreads, 1) combine_pull_kernel(const 
             st_na_v4(out_row + static_cast<size_t>(v) * 16, o);
           }
         }
-        if (!p.is_fwd && lane < K) {
+        if (!p.is_fwd && piece == 0 && lane < K) {
           const long long e = p.topk_idx[static_cast<size_t>(t) * K + lane];
           const int slot = p.pair_slot[static_cast<size_t>(t) * K + lane];
           float g = 0.f;
@@ -729,7 +797,8 @@ __global__ void __launch_bounds__(kCombineThreads, 1) combine_pull_kernel(const 
 }
 
 void launch_combine_pull(const CombineParams& p, int num_blocks, cudaStream_t stream) {
-  combine_pull_kernel<<<num_blocks, kCombineThreads, 0, stream>>>(p);
+  if (p.num_ranks == 1) combine_pull_kernel<1><<<num_blocks, combine_threads(1), 0, stream>>>(p);
+  else combine_pull_kernel<kMaxRanks><<<num_blocks, combine_threads(kMaxRanks), 0, stream>>>(p);
 }
 
 // =============================================================================================
@@ -760,38 +829,68 @@ void launch_tile_producer(int* count, const int* target, int num_tiles, long lon
   tile_producer_kernel<<<1, 1, 0, stream>>>(count, target, num_tiles, delay_ns);
 }
 
-template <bool kCompress>
-__global__ void pool_rows_kernel(const char* src, char* dst, const int* pool_recv_token, int tk_padded, int hidden) {
-  const int warps_per_block = blockDim.x >> 5;
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const size_t row_bytes = static_cast<size_t>(hidden) * 2;
-  const int vecs = hidden / 8;
-  for (int slot = blockIdx.x * warps_per_block + warp; slot < tk_padded; slot += gridDim.x * warps_per_block) {
+// Row copies between the padded pool and the compact per-recv-token matrix.  Both are bound by HBM.
+//
+// A received token has one pool row per (token, k) pair of this rank, all of them equal, and its compact row needs one of
+// them.  Compressing therefore goes by received token: pool_owner_kernel notes one slot of every token, and the copy
+// reads and writes each row once.  (Going by slot copied every pair's row onto the same compact row: 32768 pairs of 4096
+// tokens, hidden 7168, moved 940 MB in 120 us; the two launches now move 117 MB in 23 us.)
+constexpr int kRowVecs = 4;      // 16-byte loads in flight per lane
+
+__global__ void __launch_bounds__(256) pool_owner_kernel(const int* pool_recv_token, int tk_padded, int* owner, int num_recv) {
+  for (int slot = blockIdx.x * blockDim.x + threadIdx.x; slot < tk_padded; slot += gridDim.x * blockDim.x) {
     const int r = pool_recv_token[slot];
-    if (r < 0) {
-      if (!kCompress)   // padding rows of a re-expanded pool are zero
-        for (int v = lane; v < vecs; v += 32)
-          st_na_v4(dst + static_cast<size_t>(slot) * row_bytes + static_cast<size_t>(v) * 16, make_uint4(0, 0, 0, 0));
-      continue;
-    }
-    const char* s = kCompress ? src + static_cast<size_t>(slot) * row_bytes : src + static_cast<size_t>(r) * row_bytes;
-    char* d = kCompress ? dst + static_cast<size_t>(r) * row_bytes : dst + static_cast<size_t>(slot) * row_bytes;
-    for (int v = lane; v < vecs; v += 32) st_na_v4(d + static_cast<size_t>(v) * 16, ld_nc_v4(s + static_cast<size_t>(v) * 16));
+    if (r >= 0 && r < num_recv) owner[r] = slot;      // (any of the token's slots)
   }
 }
-void launch_pool_compress(const void* pool, void* recv, const int* pool_recv_token, int tk_padded, int hidden,
-                          cudaStream_t stream) {
-  if (tk_padded == 0) return;
-  const int grid = min((tk_padded + 7) / 8, sm_count() * 8);
-  pool_rows_kernel<true><<<grid, 256, 0, stream>>>(static_cast<const char*>(pool), static_cast<char*>(recv),
-                                                   pool_recv_token, tk_padded, hidden);
+
+// A warp copies a piece of 32 x kRowVecs vectors of one destination row.
+template <bool kCompress>
+__global__ void __launch_bounds__(256) pool_rows_kernel(const char* src, char* dst, const int* pool_recv_token, const int* owner,
+                                                        int tk_padded, int num_rows, int vecs, int pieces) {
+  const int lane = threadIdx.x & 31;
+  const long long items = static_cast<long long>(num_rows) * pieces, warps = static_cast<long long>(gridDim.x) * (blockDim.x >> 5);
+  for (long long item = static_cast<long long>(blockIdx.x) * (blockDim.x >> 5) + (threadIdx.x >> 5); item < items; item += warps) {
+    const int row = static_cast<int>(item / pieces), v0 = static_cast<int>(item - static_cast<long long>(row) * pieces) * 32 * kRowVecs + lane;
+    int from;
+    if (kCompress) {
+      // `owner` is not initialised: a token without a slot holds anything, and its row is left alone
+      from = owner[row];
+      if (from < 0 || from >= tk_padded || pool_recv_token[from] != row) continue;
+    } else {
+      from = pool_recv_token[row];                    // padding rows of a re-expanded pool are zero
+    }
+    const char* s = src + static_cast<size_t>(from) * vecs * 16;
+    char* d = dst + static_cast<size_t>(row) * vecs * 16;
+    uint4 q[kRowVecs];
+#pragma unroll
+    for (int u = 0; u < kRowVecs; ++u)
+      q[u] = from >= 0 && v0 + u * 32 < vecs ? ld_nc_v4(s + static_cast<size_t>(v0 + u * 32) * 16) : make_uint4(0, 0, 0, 0);
+#pragma unroll
+    for (int u = 0; u < kRowVecs; ++u)
+      if (v0 + u * 32 < vecs) st_na_v4(d + static_cast<size_t>(v0 + u * 32) * 16, q[u]);
+  }
+}
+
+template <bool kCompress>
+static void launch_pool_rows(const void* src, void* dst, const int* pool_recv_token, const int* owner, int tk_padded, int num_rows,
+                             int hidden, cudaStream_t stream) {
+  const int vecs = hidden / 8, pieces = (vecs + 32 * kRowVecs - 1) / (32 * kRowVecs);
+  const long long blocks = (static_cast<long long>(num_rows) * pieces + 7) / 8, most = 8LL * sm_count();
+  pool_rows_kernel<kCompress><<<static_cast<int>(blocks < most ? blocks : most), 256, 0, stream>>>(
+      static_cast<const char*>(src), static_cast<char*>(dst), pool_recv_token, owner, tk_padded, num_rows, vecs, pieces);
+}
+void launch_pool_compress(const void* pool, void* recv, const int* pool_recv_token, int* owner, int tk_padded, int num_recv,
+                          int hidden, cudaStream_t stream) {
+  if (tk_padded == 0 || num_recv == 0 || hidden == 0) return;
+  const int blocks = (tk_padded + 255) / 256, most = 8 * sm_count();
+  pool_owner_kernel<<<blocks < most ? blocks : most, 256, 0, stream>>>(pool_recv_token, tk_padded, owner, num_recv);
+  launch_pool_rows<true>(pool, recv, pool_recv_token, owner, tk_padded, num_recv, hidden, stream);
 }
 void launch_pool_expand(const void* recv, void* pool, const int* pool_recv_token, int tk_padded, int hidden,
                         cudaStream_t stream) {
-  if (tk_padded == 0) return;
-  const int grid = min((tk_padded + 7) / 8, sm_count() * 8);
-  pool_rows_kernel<false><<<grid, 256, 0, stream>>>(static_cast<const char*>(recv), static_cast<char*>(pool),
-                                                    pool_recv_token, tk_padded, hidden);
+  if (tk_padded == 0 || hidden == 0) return;
+  launch_pool_rows<false>(recv, pool, pool_recv_token, nullptr, tk_padded, tk_padded, hidden, stream);
 }
 
 __global__ void zero_pool_padding_kernel(char* a, char* b, const int* freq, const int* block_offset, int vecs) {

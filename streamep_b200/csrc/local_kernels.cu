@@ -71,35 +71,6 @@ __global__ void __launch_bounds__(kLocalThreads) local_count_kernel(const long l
   for (int e = threadIdx.x; e < num_experts; e += kLocalThreads) counts[static_cast<size_t>(e) * gridDim.x + blockIdx.x] = s_hist[e];
 }
 
-// Copies piece `v0` .. of token row `src` (16-byte vectors, V per lane) to the pool row of each of the token's pairs: one
-// read, `num_topk` writes.  `slot`: lane k holds the slot of pair k (-1: skipped).
-template <int V>
-__device__ __forceinline__ void copy_row_piece(const char* src, char* pool, char* also, int v0, int vecs, int num_topk, int slot, int lane) {
-  uint4 q[V];
-#pragma unroll
-  for (int u = 0; u < V; ++u) {
-    const int v = v0 + u * 32 + lane;
-    q[u] = v < vecs ? ld_nc_v4(src + static_cast<size_t>(v) * 16) : make_uint4(0, 0, 0, 0);
-  }
-  for (int k = 0; k < num_topk; ++k) {
-    const int s = __shfl_sync(0xffffffffu, slot, k);
-    if (s < 0) continue;
-    char* d = pool + static_cast<size_t>(s) * vecs * 16;
-#pragma unroll
-    for (int u = 0; u < V; ++u) {
-      const int v = v0 + u * 32 + lane;
-      if (v < vecs) *reinterpret_cast<uint4*>(d + static_cast<size_t>(v) * 16) = q[u];
-    }
-  }
-  if (also != nullptr) {
-#pragma unroll
-    for (int u = 0; u < V; ++u) {
-      const int v = v0 + u * 32 + lane;
-      if (v < vecs) st_na_v4(also + static_cast<size_t>(v) * 16, q[u]);
-    }
-  }
-}
-
 __device__ __forceinline__ void zero_slice(void* ptr, size_t bytes, size_t part, size_t parts) {
   const size_t vecs = bytes / 16;
   for (size_t i = part; i < vecs; i += parts) reinterpret_cast<uint4*>(ptr)[i] = make_uint4(0, 0, 0, 0);

@@ -1799,7 +1799,10 @@ class Runtime : public std::enable_shared_from_this<Runtime> {
   at::Tensor pool_compress(const at::Tensor& pool, const at::Tensor& pool_recv_token, int64_t num_recv) {
     SEP_ASSERT(pool.is_contiguous() && pool.scalar_type() == at::kBFloat16 && pool.size(1) % 8 == 0, "pool must be contiguous bf16 with hidden % 8 == 0");
     auto out = at::empty({num_recv, pool.size(1)}, pool.options());
-    ++launches_; launch_pool_compress(pool.data_ptr(), out.data_ptr(), pool_recv_token.data_ptr<int>(), pool.size(0), pool.size(1), stream());
+    auto owner = at::empty({num_recv}, pool_recv_token.options());
+    launches_ += 2;
+    launch_pool_compress(pool.data_ptr(), out.data_ptr(), pool_recv_token.data_ptr<int>(), owner.data_ptr<int>(), pool.size(0), num_recv,
+                         pool.size(1), stream());
     SEP_CUDA_CHECK(cudaGetLastError());
     return out;
   }
