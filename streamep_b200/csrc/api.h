@@ -215,7 +215,7 @@ struct LocalPlaceParams {
   HostOverflow* host_overflow;
   StatusBlock* status;
 };
-void launch_local_place(const LocalPlaceParams& p, const LocalGrid& g, cudaStream_t stream);
+cudaError_t launch_local_place(const LocalPlaceParams& p, const LocalGrid& g, cudaStream_t stream);
 struct LocalRowsParams {
   const void* rows[2];           // [T, H] each; pool[i] == nullptr: none
   void* pool[2];
@@ -393,6 +393,7 @@ struct GemmParams {
   // tiles of unequal length (experts of unequal row counts) and the last wave balance out.  Two ints, zero on
   // entry, reset by the kernel: [0] next tile, [1] CTAs done.
   int* tile_counter;
+  int early_start;               // 1: prepare (barriers, TMEM) while the kernel before this one in the stream still runs
   // Optional per-CTA time stamps, [gridDim.x][kTimingCols] int64 of %globaltimer nanoseconds (null = off):
   // 0 kernel start, 1 ns the operand pipeline stood still for tile gates, 2 first tile ready, 3 tiles this CTA had
   // finished when its push ended, 4 first push chunk

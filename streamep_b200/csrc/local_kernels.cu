@@ -59,6 +59,7 @@ LocalGrid local_grid(int num_tokens, int num_topk, int num_experts) {
 __global__ void __launch_bounds__(kLocalThreads) local_count_kernel(const long long* topk_idx, int num_tokens, int num_topk, int num_experts,
                                                                     int tokens_per_block, int* counts) {
   extern __shared__ int s_hist[];
+  grid_release();
   for (int e = threadIdx.x; e < num_experts; e += kLocalThreads) s_hist[e] = 0;
   __syncthreads();
   const int t0 = blockIdx.x * tokens_per_block, t1 = min(t0 + tokens_per_block, num_tokens);
@@ -99,6 +100,8 @@ __global__ void __launch_bounds__(kLocalThreads, 2) local_place_kernel(const Loc
   const int t0 = min(static_cast<int>(blockIdx.x) * p.tokens_per_block, p.num_tokens), t1 = min(t0 + p.tokens_per_block, p.num_tokens);
   const int n = has_tokens ? (t1 - t0) * K : 0;
   const long long* idx = p.topk_idx + static_cast<size_t>(t0) * K;
+  if (!FUSED_COUNT) grid_wait();
+  grid_release();
 
   // 1. pairs of every expert: in all, and in the blocks before this one
   if (FUSED_COUNT) {
@@ -249,7 +252,7 @@ __global__ void __launch_bounds__(kLocalThreads, 2) local_place_kernel(const Loc
   }
 }
 
-void launch_local_place(const LocalPlaceParams& q, const LocalGrid& g, cudaStream_t stream) {
+cudaError_t launch_local_place(const LocalPlaceParams& q, const LocalGrid& g, cudaStream_t stream) {
   LocalPlaceParams p = q;
   p.tokens_per_block = g.tokens_per_block;
   p.token_blocks = g.blocks;
@@ -258,11 +261,21 @@ void launch_local_place(const LocalPlaceParams& q, const LocalGrid& g, cudaStrea
                                                                                       g.tokens_per_block, p.counts);
   const size_t smem = sizeof(int) * (3 * static_cast<size_t>(p.num_experts) + 1 + static_cast<size_t>(g.tokens_per_block) * p.num_topk);
   if (g.fused_count) local_place_kernel<true><<<g.blocks, kLocalThreads, smem, stream>>>(p);
-  else local_place_kernel<false><<<g.blocks, kLocalThreads, smem, stream>>>(p);
+  else {
+    cudaLaunchAttribute early;          // sets up while the counts are being made
+    early.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    early.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(static_cast<unsigned>(g.blocks)); cfg.blockDim = dim3(kLocalThreads);
+    cfg.dynamicSmemBytes = smem; cfg.stream = stream; cfg.attrs = &early; cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, local_place_kernel<false>, p);
+  }
+  return cudaGetLastError();
 }
 
 // Rows of up to two matrices into their pools along the stored slots, the pools' padding rows, and two zero fills.
 __global__ void __launch_bounds__(256, 4) local_rows_kernel(const LocalRowsParams p) {
+  grid_release();
   const int tid = threadIdx.x, lane = tid & 31;
   const int K = p.num_topk, vecs = p.hidden / 8;
   const size_t row_bytes = static_cast<size_t>(p.hidden) * 2;

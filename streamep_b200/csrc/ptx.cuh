@@ -166,6 +166,14 @@ __device__ __forceinline__ bool spin_until(Pred pred, unsigned long long budget_
   }
 }
 
+// Programmatic dependent launch.  A kernel launched with the attribute may start before the kernel ahead of it in the
+// stream has finished: everything before grid_wait() must not touch memory that kernel reads or writes.  grid_wait()
+// returns once that kernel has completed and its writes are visible (at once when launched without the attribute);
+// grid_release() lets the kernel behind this one start its own preparation as SMs become free.  Called in this order, a
+// kernel's preparation never overlaps more than one kernel before it.
+__device__ __forceinline__ void grid_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void grid_release() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
 // ----------------------------------------------------------------------------------------------
 // Shared-memory helpers, mbarrier
 // ----------------------------------------------------------------------------------------------

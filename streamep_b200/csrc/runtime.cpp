@@ -1590,8 +1590,7 @@ class Runtime : public std::enable_shared_from_this<Runtime> {
     p.region_id = region; p.epoch = ++epochs_[kKindMetadata];
     p.host_overflow = cap ? host_overflow_dev_ : nullptr; p.status = status_;
     launches_ += grid.fused_count ? 1 : 2;
-    launch_local_place(p, grid, stream());
-    SEP_CUDA_CHECK(cudaGetLastError());
+    SEP_CUDA_CHECK(launch_local_place(p, grid, stream()));
     if (tiles > 0) {
       LocalGemm a(*this, *st, kEpiSwiglu, cfg.tile_n_a);
       a.operands(pool, w1, false);
@@ -1693,6 +1692,7 @@ class Runtime : public std::enable_shared_from_this<Runtime> {
       SEP_ASSERT(block_n == 128 || block_n == 256, "block_n must be 128 or 256");
       p.mode = varlen_k ? kVarlenK : kVarlenM; p.epilogue = epilogue; p.block_n = block_n;
       p.status = rt.status_; p.wait_budget_ns = rt.budget_ns_; p.num_ranks = 1;
+      p.early_start = 1;       // the kernel ahead in the stream is always one of this layer's
       p.num_experts = st.experts; p.total_rows = st.tiles * kTileM;
       p.tile_id_to_expert = st.tile_expert; p.expert_pool_block_offset = st.block_offset; p.expert_frequency = st.frequency;
     }
