@@ -211,6 +211,9 @@ struct LocalPlaceParams {
   void* pool;                    // [slots, H]
   void* x_saved;                 // optional [T, H]: a copy of x
   void* zero; size_t zero_bytes; // memory to zero on the side (the layer's output)
+  int zero_padding;              // 1: zero the pool's padding rows up to multiples of 64 (a weight-gradient GEMM will read them)
+  const void* prefetch;          // optional [E, prefetch_rows, hidden] bf16, the weights the next kernel reads: brought into the
+  int prefetch_rows;             // L2 (in part, see kPrefetchBytes) for the experts that have pairs
   int region_id, epoch;
   HostOverflow* host_overflow;
   StatusBlock* status;

@@ -51,7 +51,6 @@ LocalGrid local_grid(int num_tokens, int num_topk, int num_experts) {
   if (g.tokens_per_block < 1) g.tokens_per_block = 1;
   g.blocks = (num_tokens + g.tokens_per_block - 1) / g.tokens_per_block;
   if (g.blocks < 1) g.blocks = 1;
-  // small calls: more blocks than chunks of tokens, so that the row copies and the zero fill use the whole GPU
   g.count_ints = g.fused_count ? 0 : static_cast<size_t>(g.blocks) * num_experts;
   return g;
 }
@@ -76,6 +75,25 @@ __device__ __forceinline__ void zero_slice(void* ptr, size_t bytes, size_t part,
   const size_t vecs = bytes / 16;
   for (size_t i = part; i < vecs; i += parts) reinterpret_cast<uint4*>(ptr)[i] = make_uint4(0, 0, 0, 0);
   if (part < (bytes & 15) / 4) reinterpret_cast<int*>(ptr)[vecs * 4 + part] = 0;
+}
+
+// The pairs are sorted in 6-19 us during which HBM has little to do.  A call bound by reading the weights (fewer pairs than
+// kPrefetchRowsPerPair weight rows each) uses them to bring the first columns of every weight row of the experts it hits
+// into the L2, where the GEMM behind this kernel starts reading; as much as HBM can deliver meanwhile, well below the L2's
+// 126 MB.  Together with the padding rows that inference does not zero: 96 tokens on 32 experts, hidden 7168, 499 -> 486 us.
+constexpr size_t kPrefetchBytes = 40u << 20;
+constexpr int kPrefetchRowsPerPair = 4;
+
+__device__ __forceinline__ void prefetch_weights(const LocalPlaceParams& p, const int* s_total, int tid) {
+  int hit = 0;
+  for (int e = 0; e < p.num_experts; ++e) hit += s_total[e] > 0;
+  if (hit == 0) return;
+  const size_t row_bytes = static_cast<size_t>(p.hidden) * 2;
+  const size_t share = kPrefetchBytes / (static_cast<size_t>(hit) * p.prefetch_rows) / 128 * 128;
+  const uint32_t bytes = static_cast<uint32_t>(share < row_bytes ? share : row_bytes);
+  if (bytes == 0) return;
+  for (int i = blockIdx.x * kLocalThreads + tid; i < p.num_experts * p.prefetch_rows; i += gridDim.x * kLocalThreads)
+    if (s_total[i / p.prefetch_rows] > 0) bulk_prefetch_l2(static_cast<const char*>(p.prefetch) + static_cast<size_t>(i) * row_bytes, bytes);
 }
 
 // Zeroes the pool rows between an expert's length and the next multiple of 64 (the weight-gradient GEMM multiplies whole
@@ -133,6 +151,7 @@ __global__ void __launch_bounds__(kLocalThreads, 2) local_place_kernel(const Loc
     }
   }
   __syncthreads();
+  if (FUSED_COUNT && p.prefetch != nullptr) prefetch_weights(p, s_total, tid);
   // 2. first tile of every expert
   if (warp == 0) {
     int carry = 0, pairs = 0;
@@ -216,7 +235,7 @@ __global__ void __launch_bounds__(kLocalThreads, 2) local_place_kernel(const Loc
   for (int e = blockIdx.x; e < E; e += gridDim.x) {
     const int first = s_tiles[e] * kTileM, len = s_total[e], end = s_tiles[e + 1] * kTileM;
     for (int s = first + len + tid; s < end; s += kLocalThreads) { p.row_token[s] = -1; p.row_pair[s] = -1; p.row_weight[s] = 0.f; }
-    zero_padding_rows(static_cast<char*>(p.pool), first, len, vecs, tid, kLocalThreads);
+    if (p.zero_padding) zero_padding_rows(static_cast<char*>(p.pool), first, len, vecs, tid, kLocalThreads);
   }
   const int live = s_tiles[E];
   for (int t = blockIdx.x * kLocalThreads + tid; t < live; t += gridDim.x * kLocalThreads) {
@@ -260,7 +279,12 @@ cudaError_t launch_local_place(const LocalPlaceParams& q, const LocalGrid& g, cu
     local_count_kernel<<<g.blocks, kLocalThreads, sizeof(int) * p.num_experts, stream>>>(p.topk_idx, p.num_tokens, p.num_topk, p.num_experts,
                                                                                       g.tokens_per_block, p.counts);
   const size_t smem = sizeof(int) * (3 * static_cast<size_t>(p.num_experts) + 1 + static_cast<size_t>(g.tokens_per_block) * p.num_topk);
-  if (g.fused_count) local_place_kernel<true><<<g.blocks, kLocalThreads, smem, stream>>>(p);
+  if (g.fused_count) {
+    if (static_cast<long long>(p.num_tokens) * p.num_topk * kPrefetchRowsPerPair > static_cast<long long>(p.num_experts) * p.prefetch_rows)
+      p.prefetch = nullptr;
+    const int blocks = p.prefetch != nullptr && g.blocks < local_sms() ? local_sms() : g.blocks;    // (blocks without tokens help)
+    local_place_kernel<true><<<blocks, kLocalThreads, smem, stream>>>(p);
+  }
   else {
     cudaLaunchAttribute early;          // sets up while the counts are being made
     early.id = cudaLaunchAttributeProgrammaticStreamSerialization;

@@ -131,6 +131,10 @@ __device__ __forceinline__ void st_na_v4(void* p, uint4 v) {
 __device__ __forceinline__ void prefetch_l2(const void* p) {
   asm volatile("prefetch.global.L2 [%0];" :: "l"(p));
 }
+// `bytes` (a multiple of 16) from a 16-byte aligned address into the L2
+__device__ __forceinline__ void bulk_prefetch_l2(const void* p, uint32_t bytes) {
+  asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" :: "l"(p), "r"(bytes) : "memory");
+}
 // sigmoid through one ex2 and one approximate reciprocal (the results are rounded to bf16 anyway)
 __device__ __forceinline__ float fast_sigmoid(float x) {
   float e, r;

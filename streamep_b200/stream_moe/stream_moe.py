@@ -108,7 +108,7 @@ def moe_forward(ctx, streams, buffer, x, topk_idx, topk_weights, is_token_in_ran
     if fused and buffer.group_size == 1:
         _nvtx_push(f"fwd_fused_{_NVTX_FWD}")
         buffer._next_seq += 1
-        out, ctx.local = rt.local_forward(x, topk_idx, topk_weights, w1, w2, num_experts, level, _native_config(cfg),
+        out, ctx.local = rt.local_forward(x, topk_idx, topk_weights, w1, w2, num_experts, level, _native_config(cfg, False),
                                           comp.stream_id, comp.device_index)
         ctx.buffer, ctx.streams, ctx.fused = buffer, streams, fused
         _nvtx_pop()
@@ -416,15 +416,16 @@ def _launch_dw(buffer, handle, cfg, dl_do_pool, postact_dw2, dswiglu_in, pool, d
         dW2.zero_()
 
 
-def _native_config(cfg: TileConfig):
-    """The native form of a resolved tile configuration (kept: a program uses few)."""
-    native = _NATIVE_CONFIGS.get(cfg)
+def _native_config(cfg: TileConfig, auto_width: bool):
+    """The native form of a resolved tile configuration (kept: a program uses few).  ``auto_width``: the widths are
+    defaults, which a call with few tiles may narrow."""
+    native = _NATIVE_CONFIGS.get((cfg, auto_width))
     if native is None:
         native = _ext.load().LayerConfig(cfg.tile_n_a, cfg.tile_n_y, cfg.tile_n_y_bwd, cfg.tile_n_a_bwd, cfg.tile_n_dW1, cfg.tile_n_dW2,
-                                         cfg.num_sms_a or 0, cfg.num_sms_y or 0, cfg.num_sms_y_bwd or 0, cfg.num_sms_a_bwd or 0)
+                                         cfg.num_sms_a or 0, cfg.num_sms_y or 0, cfg.num_sms_y_bwd or 0, cfg.num_sms_a_bwd or 0, auto_width)
         if len(_NATIVE_CONFIGS) >= 256:
             _NATIVE_CONFIGS.clear()
-        _NATIVE_CONFIGS[cfg] = native
+        _NATIVE_CONFIGS[(cfg, auto_width)] = native
     return native
 
 
@@ -474,7 +475,7 @@ def stream_moe_func(buffer, x: torch.Tensor, topk_idx: torch.Tensor, topk_weight
         assert num_experts == E_local
         buffer._next_seq += 1
         comp = streams.compute
-        return buffer.runtime.local_layer(x, topk_idx, topk_weights, w1_local, w2_local, num_experts, level, _native_config(cfg),
+        return buffer.runtime.local_layer(x, topk_idx, topk_weights, w1_local, w2_local, num_experts, level, _native_config(cfg, tile_config is None),
                                           comp.stream_id, comp.device_index)
     return StreamMoEFunc.apply(streams, buffer, x, topk_idx, topk_weights, is_token_in_rank, w1_local, w2_local,
                                num_experts, cfg, activation_checkpoint_level, fused)
