@@ -2176,8 +2176,10 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
       .def("local_layer", [](const std::shared_ptr<Runtime>& r, const at::Tensor& x, const at::Tensor& idx, const at::Tensor& weights, const at::Tensor& w1,
                              const at::Tensor& w2, int num_experts, int level, const LayerConfig& cfg, int64_t stream_id, int device) {
         const auto comp = c10::cuda::CUDAStream::unpack3(stream_id, static_cast<c10::DeviceIndex>(device), c10::DeviceType::CUDA);
-        const bool differentiable = at::GradMode::is_enabled() &&
-                                    (x.requires_grad() || weights.requires_grad() || w1.requires_grad() || w2.requires_grad());
+        bool differentiable = at::GradMode::is_enabled() &&
+                              (x.requires_grad() || weights.requires_grad() || w1.requires_grad() || w2.requires_grad());
+        // forward-mode tangents: the node refuses them, the bare forward would drop them
+        for (const at::Tensor* t : {&x, &weights, &w1, &w2}) differentiable = differentiable || t->_fw_grad(0).defined();
         if (!differentiable) return r->local_forward(x, idx, weights, w1, w2, num_experts, level, cfg, false, comp).first;
         return LocalLayerFunction::apply(x, weights, w1, w2, idx, LocalLayerCall{r, num_experts, level, cfg, comp});
       })
