@@ -498,6 +498,7 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
     constexpr int kChunksPerHalf = BN / 64;
     const uint32_t stg = smem_u32(epi_stage + (warp - 2) * Cfg::kEpiStageBytes);
     int acc = 0; uint32_t acc_phase = 0;
+    uint32_t store_buf = 0;       // (store epilogue) half of the staging tile the next chunk goes through
     for (int it = 0;; ++it) {
       int lin;
       if (dyn) {
@@ -526,18 +527,14 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
         tok = t.rows_valid ? p.row_token[grow] : -1;
         if (p.row_weight != nullptr && tok >= 0) w = p.row_weight[grow];
       }
-      // scatter: where this row goes and how (0 skip, 1 bf16x2 red.add, 2 plain store)
+      // scatter to other ranks too: where this row goes and how (0 skip, 1 bf16x2 red.add, 2 plain store)
       char* dst_row = nullptr; int op = 0;
-      if (EPI == kEpiScatter && tok >= 0) {
-        if (p.remote_out.enabled) {
-          const int2 src = p.row_src[grow];
-          if (src.x == p.rank) {
-            dst_row = static_cast<char*>(p.scatter_local) + static_cast<long long>(src.y) * p.N * 2; op = 1;
-          } else {   // the source rank's per-(token, k) row: written once, reduced there in fp32
-            dst_row = s_remote_out[src.x] + (static_cast<long long>(src.y) * p.num_topk + p.row_k_slot[grow]) * p.N * 2; op = 2;
-          }
-        } else {
-          dst_row = static_cast<char*>(p.scatter_local) + static_cast<long long>(tok) * p.N * 2; op = 1;
+      if (EPI == kEpiScatter && p.remote_out.enabled && tok >= 0) {
+        const int2 src = p.row_src[grow];
+        if (src.x == p.rank) {
+          dst_row = static_cast<char*>(p.scatter_local) + static_cast<long long>(src.y) * p.N * 2; op = 1;
+        } else {   // the source rank's per-(token, k) row: written once, reduced there in fp32
+          dst_row = s_remote_out[src.x] + (static_cast<long long>(src.y) * p.num_topk + p.row_k_slot[grow]) * p.N * 2; op = 2;
         }
       }
       // dSwiGLU reads preact[row, 2n .. 2n+64) per chunk.  A thread-per-row read would touch 32 different lines
@@ -567,6 +564,27 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
         tc_fence_after_sync();
       }
       const uint32_t taddr = tmem_base + acc * BN + (static_cast<uint32_t>(quarter * 32) << 16);
+      // The accumulator goes back as soon as this warp has read its last columns (one arrival per warp, on the barrier of the
+      // CTA that issues the MMAs), not after they were stored.  With a short reduction the epilogue bounds a tile (12 k-blocks:
+      // 10,500 cycles against 6,100 of products), and the arrival as a release at cluster scope held every warp until its
+      // reductions had been performed, a sixth of its time.  Y at 32008 rows, hidden 3072, ffn 768: 172 -> 149 us; Y_bwd at
+      // 49152 rows, hidden 2048, ffn 1408: 316 -> 267 us.
+      const int c_last = min(c_begin + kChunksPerHalf, (prob_n - n0 + 31) / 32) - 1;
+      bool given_back = empty;
+      auto give_back = [&] {
+        tc_fence_before_sync();
+        __syncwarp();
+        if (lane == 0) {
+          if (CG == 2) mbar_arrive_cluster(cluster_map(&tmem_empty[acc], 0));
+          else mbar_arrive(&tmem_empty[acc]);
+        }
+        given_back = true;
+      };
+      int row_tok[EPI == kEpiScatter ? 8 : 1];     // tokens of the rows this lane stores (scatter into this GPU only)
+      if (EPI == kEpiScatter) {
+#pragma unroll
+        for (int i = 0; i < (EPI == kEpiScatter ? 8 : 1); ++i) row_tok[i] = __shfl_sync(0xffffffffu, tok, i * 4 + (lane >> 3));
+      }
       float dw_acc = 0.f;
 #pragma unroll 1
       for (int c = c_begin; c < c_begin + kChunksPerHalf; ++c) {
@@ -594,12 +612,16 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
         if (EPI != kEpiDswiglu) {
           if (!empty) {
             tmem_ld_32x32(taddr + c * 32, reinterpret_cast<uint32_t(&)[32]>(r)); tmem_ld_wait();
+            if (c == c_last) give_back();
           } else {
 #pragma unroll
             for (int i = 0; i < (EPI == kEpiDswiglu ? 1 : 32); ++i) r[i] = 0;
           }
         }
-        if (EPI == kEpiStore || EPI == kEpiSwiglu) {
+        if (EPI == kEpiStore) {          // two halves of the staging tile in turn: the store before last has read its own
+          if (lane == 0) bulk_wait_read_but_one();
+          __syncwarp();
+        } else if (EPI == kEpiSwiglu) {
           // The staging tile is reused by every chunk: the previous chunk's bulk store must have read it.
           // Waiting here, after the accumulator fetch, instead of right after the store was issued lets the
           // read overlap the TMEM load.
@@ -609,14 +631,15 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
         if (EPI == kEpiStore) {
 #pragma unroll
           for (int q = 0; q < 4; ++q)
-            st_shared_v4(stg + stage_off<64>(lane, q),
+            st_shared_v4(stg + store_buf + stage_off<64>(lane, q),
                          pack_bf16x2(__uint_as_float(r[q * 8 + 0]), __uint_as_float(r[q * 8 + 1])),
                          pack_bf16x2(__uint_as_float(r[q * 8 + 2]), __uint_as_float(r[q * 8 + 3])),
                          pack_bf16x2(__uint_as_float(r[q * 8 + 4]), __uint_as_float(r[q * 8 + 5])),
                          pack_bf16x2(__uint_as_float(r[q * 8 + 6]), __uint_as_float(r[q * 8 + 7])));
           fence_proxy_async_smem();
           __syncwarp();
-          if (lane == 0) { tma_store_3d(to0, epi_stage + (warp - 2) * Cfg::kEpiStageBytes, n, warp_row0, zc); bulk_commit(); }
+          if (lane == 0) { tma_store_3d(to0, epi_stage + (warp - 2) * Cfg::kEpiStageBytes + store_buf, n, warp_row0, zc); bulk_commit(); }
+          store_buf ^= 2048;
         } else if (EPI == kEpiSwiglu) {
           // columns (2i, 2i+1) = (gate_i, up_i); preact tile at +0 (64-byte rows), postact tile at +2048 (32-byte rows)
           if (p.out1 != nullptr) {
@@ -666,16 +689,25 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
             uint4 vs[8];      // shared-memory reads first: volatile asm keeps program order, see the dSwiGLU branch
 #pragma unroll
             for (int i = 0; i < 8; ++i) vs[i] = ld_shared_v4(stg + stage_off<128>(i * 4 + (lane >> 3), lane & 7));
+            const int piece = lane & 7, col = nbase + piece * 8;
+            const bool mine = piece < (hpos + 1) * 4 && col < p.N;
+            if (!p.remote_out.enabled) {
+              char* base = static_cast<char*>(p.scatter_local) + static_cast<long long>(col) * 2;
 #pragma unroll
-            for (int i = 0; i < 8; ++i) {
-              const int rr = i * 4 + (lane >> 3), piece = lane & 7;
-              const uint4 v = vs[i];
-              char* ptr = reinterpret_cast<char*>(__shfl_sync(0xffffffffu, reinterpret_cast<unsigned long long>(dst_row), rr));
-              const int o = __shfl_sync(0xffffffffu, op, rr);
-              const int col = nbase + piece * 8;
-              if (o != 0 && piece < (hpos + 1) * 4 && col < p.N) {
-                if (o == 1) red_add_bf16x2_v4(ptr + static_cast<long long>(col) * 2, v.x, v.y, v.z, v.w);
-                else st_na_v4(ptr + static_cast<long long>(col) * 2, v);
+              for (int i = 0; i < 8; ++i)
+                if (mine && row_tok[i] >= 0)
+                  red_add_bf16x2_v4(base + static_cast<long long>(row_tok[i]) * p.N * 2, vs[i].x, vs[i].y, vs[i].z, vs[i].w);
+            } else {
+#pragma unroll
+              for (int i = 0; i < 8; ++i) {
+                const int rr = i * 4 + (lane >> 3);
+                const uint4 v = vs[i];
+                char* ptr = reinterpret_cast<char*>(__shfl_sync(0xffffffffu, reinterpret_cast<unsigned long long>(dst_row), rr));
+                const int o = __shfl_sync(0xffffffffu, op, rr);
+                if (o != 0 && mine) {
+                  if (o == 1) red_add_bf16x2_v4(ptr + static_cast<long long>(col) * 2, v.x, v.y, v.z, v.w);
+                  else st_na_v4(ptr + static_cast<long long>(col) * 2, v);
+                }
               }
             }
             __syncwarp();
@@ -690,7 +722,10 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
               // One 16-column half at a time, fetched where it is used: fetching both halves up front, or the
               // first half before the preact hand-over, costs registers (spills at the 168-register cap of a
               // 10-warp CTA) and measured 7-12 % slower.
-              if (!empty) { tmem_ld_32x16(taddr + c * 32 + q * 8, rh); tmem_ld_wait(); }
+              if (!empty) {
+                tmem_ld_32x16(taddr + c * 32 + q * 8, rh); tmem_ld_wait();
+                if (q == 2 && c == c_last) give_back();
+              }
               else {
 #pragma unroll
                 for (int i = 0; i < 16; ++i) rh[i] = 0;
@@ -762,16 +797,8 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
           __syncwarp();
         }
       }
-      if (!empty) {
-        // one arrival per warp, on the barrier of the CTA that issues the MMAs
-        tc_fence_before_sync();
-        __syncwarp();
-        if (lane == 0) {
-          if (CG == 2) mbar_arrive_cluster(cluster_map(&tmem_empty[acc], 0));
-          else mbar_arrive(&tmem_empty[acc]);
-        }
-        acc ^= 1; if (acc == 0) acc_phase ^= 1;
-      }
+      if (!given_back) give_back();       // (no column of this tile is this warp's)
+      if (!empty) { acc ^= 1; if (acc == 0) acc_phase ^= 1; }
       if (p.timing != nullptr && epi_tid == 0) *reinterpret_cast<volatile int*>(&s_tiles_done) += 1;
       if (dyn) {                    // this queue entry may be reused once every epilogue thread is done with the tile
         epi_bar_sync();

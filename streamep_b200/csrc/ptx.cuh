@@ -247,8 +247,10 @@ __device__ __forceinline__ uint32_t cluster_map(const void* p, uint32_t rank) {
 __device__ __forceinline__ void cluster_sync() {
   asm volatile("barrier.cluster.arrive.release;\n\tbarrier.cluster.wait.acquire;" ::: "memory");
 }
+// Arrives on a barrier of another CTA of the cluster for work ordered by tcgen05 fences.  No memory of this thread has to
+// become visible with it: a release at cluster scope would wait for every global store and reduction in flight.
 __device__ __forceinline__ void mbar_arrive_cluster(uint32_t cluster_addr) {
-  asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" :: "r"(cluster_addr) : "memory");
+  asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" :: "r"(cluster_addr) : "memory");
 }
 __device__ __forceinline__ void st_cluster(uint32_t cluster_addr, int v) {
   asm volatile("st.relaxed.cluster.shared::cluster.s32 [%0], %1;" :: "r"(cluster_addr), "r"(v) : "memory");
@@ -314,6 +316,7 @@ __device__ __forceinline__ void bulk_commit() { asm volatile("cp.async.bulk.comm
 // the source shared memory of all committed groups has been read (it may be overwritten)
 __device__ __forceinline__ void bulk_wait_read() { asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory"); }
 // all committed groups are complete (their global writes are performed)
+__device__ __forceinline__ void bulk_wait_read_but_one() { asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory"); }
 __device__ __forceinline__ void bulk_wait_all() { asm volatile("cp.async.bulk.wait_group 0;" ::: "memory"); }
 
 __device__ __forceinline__ void st_shared_v4(uint32_t addr, uint32_t a, uint32_t b, uint32_t c, uint32_t d) {
