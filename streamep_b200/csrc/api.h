@@ -396,6 +396,7 @@ struct GemmParams {
   // tiles of unequal length (experts of unequal row counts) and the last wave balance out.  Two ints, zero on
   // entry, reset by the kernel: [0] next tile, [1] CTAs done.
   int* tile_counter;
+  int band;                      // height of the bands of the tile order in row tiles (even; 0 = the kernel's default)
   int early_start;               // 1: prepare (barriers, TMEM) while the kernel before this one in the stream still runs
   // Optional per-CTA time stamps, [gridDim.x][kTimingCols] int64 of %globaltimer nanoseconds (null = off):
   // 0 kernel start, 1 ns the operand pipeline stood still for tile gates, 2 first tile ready, 3 tiles this CTA had

@@ -81,15 +81,15 @@ struct TileCoord {
 // Tile order.  Consecutive linear indices (= CTAs working at the same time) walk a band of kBandM row tiles
 // column by column: a wave of 148 tiles then shares kBandM A tiles and ~148/kBandM B tiles instead of one A
 // tile and 148 B tiles, which keeps weight traffic out of HBM when one expert's weights exceed the L2.
-// Bands follow the pool order (expert-major), i.e. the order in which dispatch completes tiles.
+// Bands follow the pool order (expert-major), i.e. the order in which dispatch completes tiles.  GemmParams::band asks for
+// higher ones (see tile_band in runtime.cpp).
 constexpr int kBandM = 8;
 
-template <int BAND>
-__device__ __forceinline__ void band_decode(int lin, int num_m, int num_n, int& m_tile, int& n_tile) {
-  const int band = lin / (BAND * num_n);
-  const int rem = lin - band * (BAND * num_n);
-  const int m0 = band * BAND;
-  const int gm = min(BAND, num_m - m0);
+__device__ __forceinline__ void band_decode(int band_m, int lin, int num_m, int num_n, int& m_tile, int& n_tile) {
+  const int band = lin / (band_m * num_n);
+  const int rem = lin - band * (band_m * num_n);
+  const int m0 = band * band_m;
+  const int gm = min(band_m, num_m - m0);
   n_tile = rem / gm;
   m_tile = m0 + (rem - n_tile * gm);
 }
@@ -102,7 +102,7 @@ __device__ __forceinline__ TileCoord decode_tile(const GemmParams& p, int lin, i
   t.prob = 0;
   t.rows_valid = true;
   if (p.mode == kVarlenM) {
-    band_decode<kBandM / CG>(lin, num_m, p.num_n_tiles, t.m_tile, t.n_tile);
+    band_decode(p.band > 0 ? p.band / CG : kBandM / CG, lin, num_m, p.num_n_tiles, t.m_tile, t.n_tile);
     if (CG == 2) {
       const int pair = p.pair_tiles[t.m_tile];       // first tile * 2 + (1 if the pair has a second tile)
       t.m_tile = pair >> 1;
@@ -118,7 +118,7 @@ __device__ __forceinline__ TileCoord decode_tile(const GemmParams& p, int lin, i
     if (lin >= first) { t.prob = 1; lin -= first; nm = p.num_m_tiles2; nn = p.num_n_tiles2; m_out = p.M_out2; }
     const int per_e = nm * nn;
     t.expert = lin / per_e;
-    band_decode<kBandM / CG>(lin - t.expert * per_e, nm, nn, t.m_tile, t.n_tile);
+    band_decode(p.band > 0 ? p.band / CG : kBandM / CG, lin - t.expert * per_e, nm, nn, t.m_tile, t.n_tile);
     if (CG == 2) { t.m_tile = t.m_tile * 2 + half; t.rows_valid = t.m_tile * BM < m_out; }
     t.row0 = p.expert_pool_block_offset[t.expert] * BM;
     const int len = p.expert_frequency[t.expert];

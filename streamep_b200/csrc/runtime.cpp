@@ -1728,6 +1728,7 @@ class Runtime : public std::enable_shared_from_this<Runtime> {
       p.pair_ctas = st.pairs > 0 && p.block_n == 256; p.pair_tiles = st.pair_tiles;
       p.num_m_tiles = p.pair_ctas ? st.pairs : st.tiles; p.num_m_tiles_dev = st.sizes + (p.pair_ctas ? 3 : 0);
       p.num_n_tiles = (N + p.block_n - 1) / p.block_n;
+      p.band = tile_band(K, N);
       ta = make_tmap(a.data_ptr(), K, rows, 1, K, rows * K, 64, BM_);
       tb = b_mn ? make_tmap(w.data_ptr(), N, K, E, N, K * N, 64, 64)
                 : make_tmap(w.data_ptr(), K, N, E, K, N * K, 64, p.pair_ctas ? p.block_n / 2 : p.block_n);
@@ -1741,6 +1742,7 @@ class Runtime : public std::enable_shared_from_this<Runtime> {
       const int64_t unit_m = p.pair_ctas ? 2 * BM_ : BM_;
       p.N = N; p.M_out = M; p.out_expert_stride = M * N;
       p.num_m_tiles = units(M, unit_m); p.num_n_tiles = (N + p.block_n - 1) / p.block_n;
+      p.band = tile_band(static_cast<int64_t>(st.tokens) * st.topk / std::max<int64_t>(E, 1), std::max(N, out2 ? b2.size(1) : N));
       ta = make_tmap(a.data_ptr(), M, rows, 1, M, rows * M, 64, 64);
       tb = make_tmap(b.data_ptr(), N, rows, 1, N, rows * N, 64, 64);
       to0 = make_tmap(out.data_ptr(), N, M, E, N, M * N, 32, 32, CU_TENSOR_MAP_SWIZZLE_64B); have_o0 = true;
@@ -1753,6 +1755,17 @@ class Runtime : public std::enable_shared_from_this<Runtime> {
         have_second = true;
       }
       p.tile_counter = rt.counters_ + 10;
+    }
+    // Every band of row tiles reads the expert's whole B operand (`k` x `n`).  One that exceeds half of the L2 comes from HBM
+    // each time, which costs power more than time (the SM clock fell to 975 MHz where cuBLAS ran at 1350): bands are then as
+    // high as their own rows of A stay in half of the L2, 8 to 32 tiles.  Otherwise low bands are better, they keep fewer rows
+    // of A alive.  us for 16384 tokens, hidden 4096, ffn 14336, bands of 8 -> 16 -> 32 tiles: forward 9370 -> 9150 -> 9030, forward
+    // and backward 28500 -> 27950 -> 27990; where B fits (hidden 7168, ffn 2048): forward 3200 -> 3215 -> 3290.
+    static int tile_band(int64_t k, int64_t n) {
+      constexpr int64_t kHalfL2 = 64 << 20;
+      if (k * n * 2 <= kHalfL2) return 0;
+      const int64_t tiles = kHalfL2 / (2 * BM_ * std::max<int64_t>(k, 1));
+      return static_cast<int>(std::min<int64_t>(32, std::max<int64_t>(8, tiles / 2 * 2)));
     }
     void output0(const at::Tensor& t, uint32_t box, CUtensorMapSwizzle sw) {
       to0 = make_tmap(t.data_ptr(), t.size(1), t.size(0), 1, t.size(1), t.numel(), box, 32, sw); have_o0 = true;
