@@ -530,7 +530,12 @@ class Runtime : public std::enable_shared_from_this<Runtime> {
     if (host_overflow_ != nullptr) cudaFreeHost(host_overflow_);
     host_overflow_ = nullptr; static_.reset();
     scratch_ = nullptr; host_ = nullptr;
+    status_ = nullptr; gate_flags_ = nullptr; counters_ = nullptr;
+    available_ = false;
   }
+  // Autograd nodes and handles hold the runtime beyond Buffer.destroy(), which frees the memory that kernels report
+  // and count into: nothing may be launched or read through it any more.
+  void check_alive() const { SEP_ASSERT(!destroyed_, "this Buffer has been destroyed"); }
 
   // ---- bootstrap ---------------------------------------------------------------------------
   int get_local_device_id() const { return device_; }
@@ -645,6 +650,7 @@ class Runtime : public std::enable_shared_from_this<Runtime> {
   // kernel that still reads or writes the block is never overtaken by the block's next owner.  Work on a stream
   // the runtime has never seen is not covered: make that stream wait for the tensor's last use, or keep a reference.
   at::Tensor alloc_symmetric(const std::vector<int64_t>& sizes, at::ScalarType dtype, bool zero, size_t* offset_out = nullptr) {
+    check_alive();
     int64_t n = 1;
     for (auto s : sizes) n *= s;
     const size_t bytes = static_cast<size_t>(n) * c10::elementSize(dtype);
@@ -753,6 +759,7 @@ class Runtime : public std::enable_shared_from_this<Runtime> {
   // ---- status --------------------------------------------------------------------------------
   // Reads the device status block (synchronises the device). Returns an empty string when clean.
   std::string poll_status(bool reset) {
+    check_alive();
     SEP_CUDA_CHECK(cudaDeviceSynchronize());
     StatusBlock h;
     SEP_CUDA_CHECK(cudaMemcpy(&h, status_, sizeof(h), cudaMemcpyDeviceToHost));
@@ -772,6 +779,7 @@ class Runtime : public std::enable_shared_from_this<Runtime> {
   // ---- launch gates (reference: csrc/stream_ep.cpp:387-456) -----------------------------------
   // gate ids: 0 dispatch_main, 1 dispatch_grads, 2 kernel_y, 3 kernel_a_bwd
   void gate_wait_started(int gate, int64_t raw_stream) {
+    check_alive();
     static StreamWaitValue32Fn wait_fn = driver_fn<StreamWaitValue32Fn>("cuStreamWaitValue32");
     if (gate_issued_[gate] == 0) return;
     CUresult r = wait_fn(reinterpret_cast<CUstream>(raw_stream), reinterpret_cast<CUdeviceptr>(gate_flags_ + gate),
@@ -780,6 +788,7 @@ class Runtime : public std::enable_shared_from_this<Runtime> {
   }
   void gate_bump_issued(int gate) { ++gate_issued_[gate]; }
   at::Tensor gate_flag_tensor(int gate) {
+    check_alive();
     return at::from_blob(gate_flags_ + gate, {1}, at::TensorOptions().dtype(at::kInt).device(at::kCUDA, device_));
   }
 
@@ -788,6 +797,7 @@ class Runtime : public std::enable_shared_from_this<Runtime> {
   std::shared_ptr<DispatchState> dispatch_begin(const at::Tensor& x, const at::Tensor& topk_idx,
                                                 const at::Tensor& topk_weights, int num_experts, int tile_m,
                                                 int64_t seq, bool capacity_mode = false) {
+    check_alive();
     SEP_ASSERT(available_, "Buffer.sync has not completed");
     SEP_ASSERT(x.is_cuda() && x.dim() == 2 && x.is_contiguous() && x.scalar_type() == at::kBFloat16, "x must be a contiguous [T, H] bf16 CUDA tensor");
     SEP_ASSERT(topk_idx.dim() == 2 && topk_idx.is_contiguous() && topk_idx.scalar_type() == at::kLong, "topk_idx must be contiguous [T, K] int64");
@@ -904,6 +914,7 @@ class Runtime : public std::enable_shared_from_this<Runtime> {
   // and does not use it).  `defer_views`: create only the tensors the first GEMM launch needs; the caller
   // creates the rest with dispatch_finish_views() once that launch is queued, off the GPU's critical path.
   void dispatch_allocate(const std::shared_ptr<DispatchState>& st, bool need_o = true, bool defer_views = false) {
+    check_alive();
     if (st->region_id >= 0) { dispatch_allocate_static(st, need_o); return; }
     // The metadata kernel writes the sizes to mapped pinned memory; the epoch word goes last.
     const auto t0 = std::chrono::steady_clock::now();
@@ -1082,6 +1093,7 @@ class Runtime : public std::enable_shared_from_this<Runtime> {
   // ---- dispatch_grads --------------------------------------------------------------------------
   // `fused_buffers`: also provide the landing rows and the per-pair dL/dweight matrix of the fused backward.
   std::shared_ptr<GradsState> grads_begin(const std::shared_ptr<DispatchState>& st, bool fused_buffers = false) {
+    check_alive();
     auto g = std::make_shared<GradsState>();
     const int64_t tiles = st->total_tiles, TKp = tiles * st->tile_m, T = st->num_tokens, K = st->num_topk, H = st->hidden;
     size_t off_pool = 0, off_cnt = 0;
@@ -1553,6 +1565,7 @@ class Runtime : public std::enable_shared_from_this<Runtime> {
   std::pair<at::Tensor, c10::intrusive_ptr<LocalState>> local_forward(const at::Tensor& x_in, const at::Tensor& idx_in, const at::Tensor& weights_in,
                                                                       const at::Tensor& w1_in, const at::Tensor& w2_in, int num_experts, int level,
                                                                       const LayerConfig& cfg, bool for_backward, c10::cuda::CUDAStream comp) {
+    check_alive();
     SEP_ASSERT(available_ && num_ranks_ == 1, "Buffer.sync has not completed");
     SEP_ASSERT(x_in.is_cuda() && x_in.dim() == 2 && x_in.scalar_type() == at::kBFloat16, "x must be a [T, H] bf16 CUDA tensor");
     SEP_ASSERT(idx_in.is_cuda() && idx_in.dim() == 2 && weights_in.is_cuda() && weights_in.sizes() == idx_in.sizes() && x_in.size(0) == idx_in.size(0),
@@ -1632,6 +1645,7 @@ class Runtime : public std::enable_shared_from_this<Runtime> {
 
   // Returns {dL_dx, dL_dtopk_weights, dW1, dW2}.
   std::vector<at::Tensor> local_backward(LocalState& st, const at::Tensor& dl_dy_in, c10::cuda::CUDAStream comp) {
+    check_alive();
     const c10::cuda::CUDAStream caller = at::cuda::getCurrentCUDAStream();
     SEP_ASSERT(st.w1.defined(), "the forward of this layer kept nothing for a backward");
     at::Tensor dy = dl_dy_in.contiguous();
@@ -1886,8 +1900,9 @@ class Runtime : public std::enable_shared_from_this<Runtime> {
 
  private:
   static constexpr int BM_ = kTileM;
-  // The current torch stream; remembered so that released arena blocks wait for the work queued on it.
+  // The current torch stream, of which every launch asks; remembered so that released arena blocks wait for the work queued on it.
   at::cuda::CUDAStream stream() {
+    check_alive();
     auto s = at::cuda::getCurrentCUDAStream();
     if (s.stream() != last_stream_.load(std::memory_order_relaxed)) {
       release_ctx_->note_stream(s.stream());
