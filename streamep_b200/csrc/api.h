@@ -190,6 +190,7 @@ struct LocalGrid {
   bool fused_count;              // no count launch: every block counts all pairs
   size_t count_ints;             // scratch for the counts
 };
+constexpr int kLocalSizes = 8;
 LocalGrid local_grid(int num_tokens, int num_topk, int num_experts);
 struct LocalPlaceParams {
   const void* x;                 // [T, H] bf16
@@ -206,7 +207,8 @@ struct LocalPlaceParams {
   int* expert_pool_block_offset; // [E + 1]
   int* tile_id_to_expert;        // [tiles_cap]
   int* pair_tiles;               // [tiles_cap]
-  int* sizes;                    // [4] live tiles, tokens, overflow flag, live pairs of tiles
+  int* sizes;                    // [kLocalSizes] live tiles, tokens, overflow flag, live pairs of tiles; [4..5] zeros, the claim
+                                 // counter of the layer's weight-gradient GEMMs (GemmParams::tile_counter)
   int tiles_cap;                 // a layout with more tiles runs as an empty dispatch and is reported
   void* pool;                    // [slots, H]
   void* x_saved;                 // optional [T, H]: a copy of x

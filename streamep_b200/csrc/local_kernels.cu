@@ -257,6 +257,7 @@ __global__ void __launch_bounds__(kLocalThreads, 2) local_place_kernel(const Loc
     if (tid == 0) {
       p.expert_pool_block_offset[E] = live;
       p.sizes[0] = live; p.sizes[1] = p.num_tokens; p.sizes[2] = ok ? 0 : 1; p.sizes[3] = s_pairs;
+      p.sizes[4] = 0; p.sizes[5] = 0;
     }
   }
   // 5. the rows: a warp takes a piece of one token's row, reads it once and stores it once per pair

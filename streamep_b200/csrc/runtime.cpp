@@ -1596,7 +1596,7 @@ class Runtime : public std::enable_shared_from_this<Runtime> {
     st->pairs = pairs_pay(P, E) ? static_cast<int>(std::min<int64_t>(tiles, P / (2 * kTileM) + std::min<int64_t>(E, P))) : 0;
     const int64_t R = tiles * kTileM;
     const LocalGrid grid = local_grid(T, K, E);
-    const int64_t counts[] = {static_cast<int64_t>(grid.count_ints), P, R, R, R, E, E + 1, tiles, tiles, 4};
+    const int64_t counts[] = {static_cast<int64_t>(grid.count_ints), P, R, R, R, E, E + 1, tiles, tiles, kLocalSizes};
     int64_t off[11] = {0};
     for (int i = 0; i < 10; ++i) off[i + 1] = off[i] + (counts[i] + 3) / 4 * 4;
     auto opts = x.options();
@@ -1768,7 +1768,7 @@ class Runtime : public std::enable_shared_from_this<Runtime> {
         second[2] = make_tmap(out2->data_ptr(), N2, M2, E, N2, M2 * N2, 32, 32, CU_TENSOR_MAP_SWIZZLE_64B);
         have_second = true;
       }
-      p.tile_counter = rt.counters_ + 10;
+      p.tile_counter = st.sizes + 4;     // the layer's own: two layers of a buffer may run on different streams
     }
     // Every band of row tiles reads the expert's whole B operand (`k` x `n`).  One that exceeds half of the L2 comes from HBM
     // each time, which costs power more than time (the SM clock fell to 975 MHz where cuBLAS ran at 1350): bands are then as
