@@ -86,6 +86,11 @@ static CUtensorMap make_tmap(const void* base, uint64_t d0, uint64_t d1, uint64_
   return m;
 }
 
+// Rows are read 16 bytes at a time.  A contiguous tensor may still start anywhere (a view of a flat buffer at an odd element,
+// the gradient of an output that was concatenated behind something): such rows are copied to an aligned place first.
+static bool is_aligned(const at::Tensor& t) { return reinterpret_cast<uintptr_t>(t.data_ptr()) % 16 == 0; }
+static at::Tensor aligned_rows(const at::Tensor& t) { return !t.is_contiguous() || is_aligned(t) ? t : t.clone(); }
+
 // ---------------------------------------------------------------------------------------------
 // Peer-shareable device memory through the virtual-memory-management driver API: cuMemCreate with a POSIX file
 // descriptor as the shareable handle, cuMemAddressReserve + cuMemMap + cuMemSetAccess on the owner, and
@@ -808,7 +813,7 @@ class Runtime : public std::enable_shared_from_this<Runtime> {
     SEP_ASSERT(x.size(1) % 8 == 0, "hidden must be a multiple of 8");
     SEP_ASSERT(topk_idx.size(1) <= kMaxTopK, "num_topk too large");
     auto st = std::make_shared<DispatchState>();
-    st->x = x; st->topk_idx = topk_idx; st->topk_weights = topk_weights;
+    st->x = aligned_rows(x); st->topk_idx = topk_idx; st->topk_weights = topk_weights;
     st->num_tokens = x.size(0); st->hidden = x.size(1); st->num_topk = topk_idx.size(1);
     st->num_experts = num_experts; st->tile_m = tile_m; st->seq = seq;
     st->meta_epoch = ++epochs_[kKindMetadata];
@@ -1142,7 +1147,8 @@ class Runtime : public std::enable_shared_from_this<Runtime> {
                   int flags, int num_blocks) {
     SEP_ASSERT(dl_dy.is_cuda() && dl_dy.is_contiguous() && dl_dy.scalar_type() == at::kBFloat16 && dl_dy.dim() == 2 &&
                dl_dy.size(0) == st->num_tokens && dl_dy.size(1) == st->hidden, "dL_dy must be contiguous [T, H] bf16");
-    PushParams p = make_push_params(*st, dl_dy, true, g->record, kKindDispatchGrads, g->epoch, flags,
+    const at::Tensor rows = aligned_rows(dl_dy);
+    PushParams p = make_push_params(*st, rows, true, g->record, kKindDispatchGrads, g->epoch, flags,
                                     g->bwd_dispatch_arrival_count.data_ptr<int>(), 4);
     if (flags & 2) ++gate_issued_[1];
     ++launches_; launch_dispatch_push(p, num_blocks, stream());
@@ -1161,7 +1167,11 @@ class Runtime : public std::enable_shared_from_this<Runtime> {
     // keeps there (handle.o, handle.y_done_per_token, Buffer.alloc_symmetric results) are used in
     // place, which is what lets the gate be written while this kernel runs.
     auto to_sym = [&](const at::Tensor& t) {
-      if (t.numel() == 0 || is_symmetric(t)) return t;
+      if (t.numel() == 0) return t;
+      if (is_symmetric(t)) {       // (may still be written while the kernel runs: it cannot be moved)
+        SEP_ASSERT(t.scalar_type() != at::kBFloat16 || is_aligned(t), "combine rows in the arena must start on a 16-byte boundary");
+        return t;
+      }
       auto s = alloc_symmetric(t.sizes().vec(), t.scalar_type(), false);
       if (t.numel() > 0) SEP_CUDA_CHECK(cudaMemcpyAsync(s.data_ptr(), t.data_ptr(), t.nbytes(), cudaMemcpyDeviceToDevice, stream));
       return s;
@@ -1292,6 +1302,8 @@ class Runtime : public std::enable_shared_from_this<Runtime> {
     auto ld = [](const at::Tensor& t) { return t.dim() >= 2 ? t.stride(t.dim() - 2) : t.numel(); };
     if (a.out0.has_value()) { p.out0 = a.out0->data_ptr(); p.ld0 = ld(*a.out0); }
     if (a.out1.has_value()) { p.out1 = a.out1->data_ptr(); p.ld1 = ld(*a.out1); }
+    if (a.preact.has_value()) SEP_ASSERT(is_aligned(*a.preact) && ld(*a.preact) % 8 == 0, "preact rows must start on 16-byte boundaries");
+    if (a.scatter_local.has_value()) SEP_ASSERT(is_aligned(*a.scatter_local), "the scatter destination must start on a 16-byte boundary");
     if (a.preact.has_value()) { p.preact = a.preact->data_ptr(); p.ld_preact = ld(*a.preact); }
     if (a.row_weight.has_value()) p.row_weight = a.row_weight->data_ptr<float>();
     if (a.row_token.has_value()) p.row_token = a.row_token->data_ptr<int>();
@@ -1365,6 +1377,7 @@ class Runtime : public std::enable_shared_from_this<Runtime> {
         : static_cast<int64_t>(p.num_experts) * (static_cast<int64_t>(p.num_m_tiles) * p.num_n_tiles + static_cast<int64_t>(p.num_m_tiles2) * p.num_n_tiles2);
     PushParams pp{};
     const PushParams* ppp = nullptr;
+    at::Tensor push_rows;
     if (a.fused_push) {
       pp = make_push_params(*a.fused_push, a.fused_push->x, false, a.fused_push->record, kKindDispatch,
                             a.fused_push->push_epoch, a.push_flags, a.fused_push->pool_arrival_count.data_ptr<int>(), 2);
@@ -1372,7 +1385,8 @@ class Runtime : public std::enable_shared_from_this<Runtime> {
       ppp = &pp;
     } else if (a.fused_push_grads) {
       SEP_ASSERT(a.fused_push_routing && a.fused_push_rows.defined(), "fused dispatch_grads needs the forward routing and dL_dy");
-      pp = make_push_params(*a.fused_push_routing, a.fused_push_rows, true, a.fused_push_grads->record, kKindDispatchGrads,
+      push_rows = aligned_rows(a.fused_push_rows);
+      pp = make_push_params(*a.fused_push_routing, push_rows, true, a.fused_push_grads->record, kKindDispatchGrads,
                             a.fused_push_grads->epoch, a.push_flags, a.fused_push_grads->bwd_dispatch_arrival_count.data_ptr<int>(), 4);
       pp.started_flag = nullptr;
       ppp = &pp;
@@ -1399,7 +1413,8 @@ class Runtime : public std::enable_shared_from_this<Runtime> {
       pp.started_flag = nullptr;
       ++launches_; launch_dispatch_push(pp, num_sms(), stream);
     } else if (a.fused_push_grads) {
-      PushParams pp = make_push_params(*a.fused_push_routing, a.fused_push_rows, true, a.fused_push_grads->record, kKindDispatchGrads,
+      const at::Tensor push_rows = aligned_rows(a.fused_push_rows);
+      PushParams pp = make_push_params(*a.fused_push_routing, push_rows, true, a.fused_push_grads->record, kKindDispatchGrads,
                                        a.fused_push_grads->epoch, a.push_flags & 3, a.fused_push_grads->bwd_dispatch_arrival_count.data_ptr<int>(), 4);
       pp.started_flag = nullptr;
       ++launches_; launch_dispatch_push(pp, num_sms(), stream);
@@ -1576,7 +1591,7 @@ class Runtime : public std::enable_shared_from_this<Runtime> {
     SEP_ASSERT(w1_in.is_cuda() && w2_in.is_cuda() && w1_in.dim() == 3 && w1_in.size(0) == num_experts && w1_in.size(2) == x_in.size(1) &&
                w2_in.size(1) == x_in.size(1) && w1_in.size(1) == 2 * w2_in.size(2), "expert weights do not match x and num_experts");
     const c10::cuda::CUDAStream caller = at::cuda::getCurrentCUDAStream();
-    at::Tensor x = x_in.contiguous(), w1 = w1_in.contiguous(), w2 = w2_in.contiguous(), idx = idx_in, weights = weights_in;
+    at::Tensor x = aligned_rows(x_in.contiguous()), w1 = w1_in.contiguous(), w2 = w2_in.contiguous(), idx = idx_in, weights = weights_in;
     if (idx.scalar_type() != at::kLong) idx = idx.to(at::kLong);
     if (weights.scalar_type() != at::kFloat) weights = weights.to(at::kFloat);
     idx = idx.contiguous(); weights = weights.contiguous();
@@ -1650,6 +1665,7 @@ class Runtime : public std::enable_shared_from_this<Runtime> {
     SEP_ASSERT(st.w1.defined(), "the forward of this layer kept nothing for a backward");
     at::Tensor dy = dl_dy_in.contiguous();
     if (dy.scalar_type() != at::kBFloat16) dy = dy.to(at::kBFloat16);
+    dy = aligned_rows(dy);
     SEP_ASSERT(dy.is_cuda() && dy.dim() == 2 && dy.size(0) == st.tokens && dy.size(1) == st.hidden, "dL_dy must be [T, H]");
     stream_wait(comp, caller);
     c10::cuda::CUDAStreamGuard guard(comp);
@@ -1835,6 +1851,7 @@ class Runtime : public std::enable_shared_from_this<Runtime> {
                       const std::optional<at::Tensor>& sizes = std::nullopt) {
     SEP_ASSERT(out.is_contiguous() && out.scalar_type() == at::kBFloat16 && out.dim() == 2 && out.size(1) % 8 == 0, "out must be contiguous [T, H] bf16");
     SEP_ASSERT(topk_idx.scalar_type() == at::kLong && topk_idx.is_contiguous() && topk_idx.size(0) == out.size(0), "topk_idx must be contiguous [T, K] int64");
+    SEP_ASSERT(is_aligned(out) && (num_ranks_ == 1 || is_aligned(rows)), "out and rows must start on 16-byte boundaries");
     const bool copy_dw = dw_dst.has_value() && dw_dst->defined();
     if (out.size(0) == 0 || (num_ranks_ == 1 && !copy_dw)) return;
     if (num_ranks_ > 1) SEP_ASSERT(rows.numel() == out.size(0) * topk_idx.size(1) * out.size(1), "rows must be [T * K, H]");
@@ -1848,7 +1865,8 @@ class Runtime : public std::enable_shared_from_this<Runtime> {
                           sizes.has_value() ? sizes->data_ptr<int>() + 2 : nullptr);
     SEP_CUDA_CHECK(cudaGetLastError());
   }
-  at::Tensor pool_compress(const at::Tensor& pool, const at::Tensor& pool_recv_token, int64_t num_recv) {
+  at::Tensor pool_compress(const at::Tensor& pool_in, const at::Tensor& pool_recv_token, int64_t num_recv) {
+    const at::Tensor pool = aligned_rows(pool_in);
     SEP_ASSERT(pool.is_contiguous() && pool.scalar_type() == at::kBFloat16 && pool.size(1) % 8 == 0, "pool must be contiguous bf16 with hidden % 8 == 0");
     auto out = at::empty({num_recv, pool.size(1)}, pool.options());
     auto owner = at::empty({num_recv}, pool_recv_token.options());
@@ -1858,14 +1876,16 @@ class Runtime : public std::enable_shared_from_this<Runtime> {
     SEP_CUDA_CHECK(cudaGetLastError());
     return out;
   }
-  at::Tensor pool_expand(const at::Tensor& recv, const at::Tensor& pool_recv_token, int64_t tk_padded) {
+  at::Tensor pool_expand(const at::Tensor& recv_in, const at::Tensor& pool_recv_token, int64_t tk_padded) {
+    const at::Tensor recv = aligned_rows(recv_in);
     SEP_ASSERT(recv.is_contiguous() && recv.scalar_type() == at::kBFloat16 && recv.size(1) % 8 == 0, "recv must be contiguous bf16 with hidden % 8 == 0");
     auto out = at::empty({tk_padded, recv.size(1)}, recv.options());
     ++launches_; launch_pool_expand(recv.data_ptr(), out.data_ptr(), pool_recv_token.data_ptr<int>(), tk_padded, recv.size(1), stream());
     SEP_CUDA_CHECK(cudaGetLastError());
     return out;
   }
-  std::vector<at::Tensor> router(const at::Tensor& x, const at::Tensor& w_gate, int top_k, int num_ranks, bool renormalize, bool want_probs) {
+  std::vector<at::Tensor> router(const at::Tensor& x_in, const at::Tensor& w_gate_in, int top_k, int num_ranks, bool renormalize, bool want_probs) {
+    const at::Tensor x = aligned_rows(x_in), w_gate = aligned_rows(w_gate_in);
     SEP_ASSERT(x.is_contiguous() && w_gate.is_contiguous() && x.scalar_type() == at::kBFloat16 && w_gate.scalar_type() == at::kBFloat16, "router inputs must be contiguous bf16");
     SEP_ASSERT(x.size(1) == w_gate.size(1) && x.size(1) % 8 == 0, "router hidden mismatch");
     SEP_ASSERT(w_gate.size(0) <= 512 && top_k <= 32 && w_gate.size(0) % num_ranks == 0, "router supports up to 512 experts and top-32");
