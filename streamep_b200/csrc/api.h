@@ -93,6 +93,7 @@ struct MetadataParams {
   int* send_order_base;          // [C, E] scratch: first position in `send_list` of this rank's (channel, expert) pairs
   int* send_list;                // [T * K] pair ids (t * K + k) in push order (see push_order), then (t, k)
   int* num_send;                 // [1] number of valid pairs == used length of send_list
+  int* push_claims;              // [4] zeroed: claim and block counters of a single rank's push (dispatch, dispatch_grads)
   int* peer_total_tiles;         // [R]
   int* peer_num_recv;            // [R]
   // receiver-side outputs (local)

@@ -136,6 +136,7 @@ __global__ void __launch_bounds__(kMetaThreads, 1) dispatch_metadata_kernel(cons
   }
   if (p.phase_mask & 1) {
     const int c = blockIdx.x;
+    if (c == 0 && tid < 4) p.push_claims[tid] = 0;
     const int lo = min(per * c, T), hi = min(lo + per, T);
     for (int e = tid; e < E; e += blockDim.x) s_hist[e] = 0;
     if (tid < kMaxRanks) s_u[tid] = 0;
@@ -612,7 +613,8 @@ __global__ void __launch_bounds__(kPushThreads, 1) dispatch_push_kernel(const Pu
 // The push of a single rank: every pair of a token lands in this rank's pool, so a warp takes whole tokens, reads each row
 // once and stores it once per pair, where the general kernel reads a row per pair.  Bound by the pool's writes to HBM; the
 // caller's SM budget (80 blocks by default) asks for as many bytes in flight per SM as it can hold: 32 warps, 4 KB each.
-// 4096 tokens x 8 pairs, hidden 7168, 80 blocks: 173 -> 135 us.
+// 4096 tokens x 8 pairs, hidden 7168, 80 blocks: 173 -> 135 us.  Chunks of tokens are claimed, not dealt out by block: a
+// block needs a whole SM, and a consumer that already waits for rows may hold the SM of a block that has not started yet.
 constexpr int kLocalPushThreads = 1024;
 constexpr int kLocalPushPairs = 16;     // pairs a warp copies between two releases of their tiles
 
@@ -628,10 +630,13 @@ __global__ void __launch_bounds__(kLocalPushThreads, 1) dispatch_push_local_kern
   const int vecs = p.hidden / 8;
   const size_t row_bytes = static_cast<size_t>(p.hidden) * 2;
   const int chunk = max(1, kLocalPushPairs / K);        // tokens
-  const int warps = gridDim.x * (kLocalPushThreads / 32);
-  for (int t0 = (blockIdx.x * (kLocalPushThreads / 32) + (tid >> 5)) * chunk; t0 < p.num_tokens; t0 += warps * chunk) {
-    const int t1 = min(t0 + chunk, p.num_tokens);
-    for (int t = t0; t < t1; ++t) {
+  for (;;) {
+    int claimed = 0;
+    if (lane == 0) claimed = atomicAdd(p.work_counter, 1);
+    const long long t0 = static_cast<long long>(__shfl_sync(0xffffffffu, claimed, 0)) * chunk;
+    if (t0 >= p.num_tokens) break;
+    const int t1 = static_cast<int>(min(t0 + chunk, static_cast<long long>(p.num_tokens)));
+    for (int t = static_cast<int>(t0); t < t1; ++t) {
       const int slot = lane < K ? p.pair_slot[static_cast<size_t>(t) * K + lane] : -1;
       const char* src = static_cast<const char*>(p.x) + t * row_bytes;
       for (int v0 = 0; v0 < vecs; v0 += 256) copy_row_piece<8>(src, tg.pool[0], nullptr, v0, vecs, K, slot, lane);
@@ -653,9 +658,17 @@ __global__ void __launch_bounds__(kLocalPushThreads, 1) dispatch_push_local_kern
       }
     }
     __syncwarp();
-    for (int i = lane; i < (t1 - t0) * K; i += 32) {    // release the chunk's pairs (same GPU: device scope)
+    for (int i = lane; i < (t1 - static_cast<int>(t0)) * K; i += 32) {    // release the chunk's pairs (same GPU: device scope)
       const int slot = p.pair_slot[static_cast<size_t>(t0) * K + i];
       if (slot >= 0) red_release_gpu_add(tg.arrival_count[0] + slot / p.tile_m, 1);
+    }
+  }
+  __syncthreads();
+  if (tid == 0) {
+    __threadfence();
+    if (atomicAdd(p.blocks_done, 1) == static_cast<int>(gridDim.x) - 1) {   // last block resets the counters for another push
+      *p.work_counter = 0;
+      *p.blocks_done = 0;
     }
   }
 }

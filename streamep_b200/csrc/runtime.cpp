@@ -301,7 +301,7 @@ struct DispatchState {
   at::Tensor sender_slab;
   at::Tensor pair_rank, pair_slot, token_rank_in_channel, send_recv_token, send_head, is_token_in_rank,
       channel_prefix_matrix, send_base, send_token_base, peer_total_tiles, peer_num_recv, send_order_base, send_list,
-      num_send;
+      num_send, push_claims;
   // receiver side metadata (regular device memory)
   at::Tensor expert_frequency, expert_pool_block_offset, base_pool, seen_per_substream, rank_prefix_matrix,
       recv_channel_prefix_matrix, tile_id_to_expert, pool_arrival_target, pair_tiles;
@@ -822,7 +822,7 @@ class Runtime : public std::enable_shared_from_this<Runtime> {
     const int64_t tiles_cap = capacity_mode ? static_->tiles_cap : 0;
     if (capacity_mode) SEP_ASSERT(static_fits(T, st->hidden, st->num_topk), "this dispatch does not fit the capacity-mode regions (tokens, hidden or top-k differ)");
     const int64_t n_i32 = T * K * 3 + T * R * 3 + (T * R + 3) / 4 + R * C + 2 * C * E + C * R + 2 * R + EL + (EL + 1) +
-                          2 * C * R * EL + R * R + R * C + 3 * tiles_cap + 108;
+                          2 * C * R * EL + R * R + R * C + 3 * tiles_cap + 112;
     st->sender_slab = at::empty({n_i32}, x.options().dtype(at::kInt));
     int64_t off = 0;
     auto take = [&](std::vector<int64_t> shape) {
@@ -836,7 +836,7 @@ class Runtime : public std::enable_shared_from_this<Runtime> {
     st->is_token_in_rank = take({(T * R + 3) / 4}).view(at::kBool).narrow(0, 0, T * R).view({T, R});
     st->channel_prefix_matrix = take({R, C}); st->send_base = take({C, E}); st->send_token_base = take({C, R});
     st->peer_total_tiles = take({R}); st->peer_num_recv = take({R});
-    st->send_order_base = take({C, E}); st->send_list = take({T * K}); st->num_send = take({1});
+    st->send_order_base = take({C, E}); st->send_list = take({T * K}); st->num_send = take({1}); st->push_claims = take({4});
     st->expert_frequency = take({EL}); st->expert_pool_block_offset = take({EL + 1});
     st->base_pool = take({C, R, EL}); st->seen_per_substream = take({C, R, EL});
     st->rank_prefix_matrix = take({R, R}); st->recv_channel_prefix_matrix = take({R, C});
@@ -878,7 +878,7 @@ class Runtime : public std::enable_shared_from_this<Runtime> {
     p.channel_prefix_matrix = st->channel_prefix_matrix.data_ptr<int>();
     p.send_base = st->send_base.data_ptr<int>(); p.send_token_base = st->send_token_base.data_ptr<int>();
     p.send_order_base = st->send_order_base.data_ptr<int>(); p.send_list = st->send_list.data_ptr<int>();
-    p.num_send = st->num_send.data_ptr<int>();
+    p.num_send = st->num_send.data_ptr<int>(); p.push_claims = st->push_claims.data_ptr<int>();
     p.peer_total_tiles = st->peer_total_tiles.data_ptr<int>(); p.peer_num_recv = st->peer_num_recv.data_ptr<int>();
     p.expert_frequency = st->expert_frequency.data_ptr<int>();
     p.expert_pool_block_offset = st->expert_pool_block_offset.data_ptr<int>();
@@ -1081,7 +1081,9 @@ class Runtime : public std::enable_shared_from_this<Runtime> {
     p.own_arrival_count = own_count; p.own_arrival_target = st.pool_arrival_target.data_ptr<int>();
     p.own_total_tiles = st.total_tiles;
     p.started_flag = gate_flags_ + (is_grads ? 1 : 0);
-    p.work_counter = counters_ + counter_base; p.blocks_done = counters_ + counter_base + 1;
+    // (one rank alone: counters of this dispatch, so that pushes on different streams do not share them)
+    int* counters = num_ranks_ == 1 ? st.push_claims.data_ptr<int>() + (is_grads ? 2 : 0) : counters_ + counter_base;
+    p.work_counter = counters; p.blocks_done = counters + 1;
     p.status = status_; p.wait_budget_ns = budget_ns_;
     return p;
   }
