@@ -135,6 +135,8 @@ def main():
     x = torch.randn(T, H, device=dev).to(torch.bfloat16)
     dy = (torch.randn(T, H, device=dev) * 0.1).to(torch.bfloat16)
     routes = [layer.route(x) for layer in layers]
+    if args.sweep and world == 1:
+        ap.error("--sweep compares push settings, and one rank alone pushes nothing: run it on several ranks")
     if args.sweep:
         return sweep(args, buf, layers, routes, x, dy, rank, world, local)
     stamps = None

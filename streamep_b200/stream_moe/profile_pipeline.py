@@ -15,41 +15,53 @@ from __future__ import annotations
 
 import argparse
 import os
+import re
 import statistics
 import sys
 
 import torch
 import torch.distributed as dist
 
-LOGICAL = [  # substring of the kernel name -> logical name (template args: BN, A_MN, B_MN, EPI, PUSH)
-    ("dispatch_metadata_kernel", "metadata"),
-    ("fill_tile_metadata_kernel", "tile fill"),
-    ("dispatch_push_kernel", "dispatch / dispatch_grads (stand-alone push)"),
-    ("combine_pull_kernel", "combine / combine_grads (stand-alone pull)"),
-    ("false, false, 1, true>", "dispatch (+) GEMM-A SwiGLU (fused)"),
-    ("false, false, 1, false>", "GEMM-A SwiGLU"),
-    ("false, false, 2, false>", "GEMM-Y (+ combine when remote)"),
-    ("false, true, 3, true>", "dispatch_grads (+) GEMM-Y_bwd dSwiGLU (fused)"),
-    ("false, true, 3, false>", "GEMM-Y_bwd dSwiGLU"),
-    ("false, true, 2, false>", "GEMM-A_bwd (+ combine_grads when remote)"),
-    ("true, true, 0, false>", "dW grouped GEMM"),
-    ("false, false, 0, false>", "preact recompute GEMM"),
-    ("false, false, 4, false>", "router logits GEMM (fp32 store)"),
-    ("router_finish_kernel", "router softmax / top-k"),
-    ("pool_rows_kernel", "pool compress / expand"),
-    ("router_kernel", "router (SIMT path)"),
-    ("device_barrier_kernel", "barrier / tail handshake"),
-]
+KERNELS = {  # kernel function -> logical name
+    "dispatch_metadata_kernel": "metadata",
+    "fill_tile_metadata_kernel": "tile fill",
+    "dispatch_push_kernel": "dispatch / dispatch_grads (stand-alone push)",
+    "dispatch_push_local_kernel": "dispatch / dispatch_grads (stand-alone push)",
+    "combine_pull_kernel": "combine / combine_grads (stand-alone pull)",
+    "combine_reduce_kernel": "combine of landed rows",
+    "local_count_kernel": "single-rank dispatch (sort, rows into the pool)",
+    "local_place_kernel": "single-rank dispatch (sort, rows into the pool)",
+    "local_rows_kernel": "single-rank dispatch_grads (rows into the pool)",
+    "zero_pool_padding_kernel": "pool padding rows",
+    "pool_owner_kernel": "pool compress / expand",
+    "pool_rows_kernel": "pool compress / expand",
+    "router_mma_kernel": "router",
+    "router_kernel": "router (SIMT path)",
+    "device_barrier_kernel": "barrier / tail handshake",
+    "tile_producer_kernel": "tile producer (test stand-in for a dispatch)",
+}
+GEMMS = {  # (A is MN-major, B is MN-major, epilogue, fused push) of grouped_gemm_kernel -> logical name
+    (0, 0, 1, 1): "dispatch (+) GEMM-A SwiGLU (fused)",
+    (0, 0, 1, 0): "GEMM-A SwiGLU",
+    (0, 0, 2, 0): "GEMM-Y (+ combine when remote)",
+    (0, 1, 3, 1): "dispatch_grads (+) GEMM-Y_bwd dSwiGLU (fused)",
+    (0, 1, 3, 0): "GEMM-Y_bwd dSwiGLU",
+    (0, 1, 2, 0): "GEMM-A_bwd (+ combine_grads when remote)",
+    (1, 1, 0, 0): "dW grouped GEMM",
+    (0, 0, 0, 0): "preact recompute GEMM",
+}
 
 
 def classify(name: str) -> str:
-    name = name.replace(", 0, 0,", ", false, false,").replace(", 0, 1,", ", false, true,").replace(", 1, 1,", ", true, true,")
-    for key, label in LOGICAL:
-        if key in name:
-            return label
-    for epi, push, label in ((1, 1, 4), (1, 0, 5), (2, 0, 6), (3, 1, 7), (3, 0, 8)):
-        if name.endswith(f"{epi}, {push}>") or f", {epi}, {push}>(" in name:
-            return LOGICAL[label][1]
+    m = re.search(r"(\w+_kernel)(?:<([^<>]*)>)?", name)
+    if m and m.group(1) == "grouped_gemm_kernel" and m.group(2):
+        # template arguments: BN, A_MN, B_MN, EPI, PUSH, CG ("true" or "1" or "(bool)1", as the tool prints them)
+        args = [re.sub(r"^\(\w+\)", "", a.strip()) for a in m.group(2).split(",")]
+        args = [{"true": 1, "false": 0}.get(a, int(a) if a.isdigit() else -1) for a in args]
+        if len(args) == 6 and tuple(args[1:5]) in GEMMS:
+            return GEMMS[tuple(args[1:5])]
+    elif m and m.group(1) in KERNELS:
+        return KERNELS[m.group(1)]
     if "Memset" in name or "memset" in name or "FillFunctor" in name:
         return "memset / fill (torch)"
     return "other: " + name[:60]
@@ -166,10 +178,12 @@ def main():
         lines.append(f"config: tokens/rank={T} hidden={H} ffn={I} experts={E} ({args.experts_per_rank}/rank) top{K} "
                      f"layers={args.layers} world={world} fused={args.fused} ckpt_level={args.ckpt_level} "
                      f"capacity_factor={args.capacity_factor}")
-        from ..utils.roofline import layer_rooflines, load_peaks
+        from ..utils.roofline import layer_rooflines, load_peaks, single_rank_rooflines
         peaks = load_peaks()
         roof = layer_rooflines(T, H, I, K, world, peaks, experts_per_rank=args.experts_per_rank,
                                store_preact=args.ckpt_level == 0)
+        if world == 1:
+            roof.update(single_rank_rooflines(T, H, I, K, peaks, experts=args.experts_per_rank, store_preact=args.ckpt_level == 0))
         lines.append(f"{'kernel':58s} {'calls/step':>10s} {'us/step':>10s} {'roofline us':>12s} {'fraction':>9s}  bound")
         for label, (n, us) in sorted(agg.items(), key=lambda kv: -kv[1][1]):
             row = f"{label:58s} {n / args.steps:10.1f} {us / args.steps:10.1f}"

@@ -88,6 +88,20 @@ def layer_rooflines(tokens: int, hidden: int, ffn: int, topk: int, world: int, p
     return out
 
 
+def single_rank_rooflines(tokens: int, hidden: int, ffn: int, topk: int, peaks: Optional[Peaks] = None,
+                          experts: int = 8, store_preact: bool = True) -> Dict[str, KernelRoofline]:
+    """The kernels that one rank alone runs instead of the fused pushes of :func:`layer_rooflines`: rows are copied into the pool by
+    kernels of their own (a token's row read once and written once per pair, an output zeroed), and the GEMMs only read it."""
+    pk = peaks or load_peaks()
+    T, P, H, I = float(tokens), float(tokens) * topk, float(hidden), float(ffn)
+    row_h, row_i, w = H * 2, I * 2, experts * H * I * 2
+    rows = _k(0.0, T * row_h + P * row_h + T * row_h, 0.0, pk)
+    return {"GEMM-A SwiGLU": _k(2 * P * H * 2 * I, P * row_h + P * row_i + (P * 2 * row_i if store_preact else 0) + 2 * w, 0.0, pk),
+            "GEMM-Y_bwd dSwiGLU": _k(2 * P * H * I, P * row_h + P * 2 * row_i + P * 2 * row_i + P * row_i + w, 0.0, pk),
+            "single-rank dispatch (sort, rows into the pool)": rows,
+            "single-rank dispatch_grads (rows into the pool)": rows}
+
+
 def step_flops(tokens: int, hidden: int, ffn: int, topk: int, layers: int = 1, recompute: bool = False) -> float:
     """Forward 6 + backward 12 (+ 4 when the first GEMM is recomputed) FLOPs per (pair, hidden, ffn) element."""
     return (22.0 if recompute else 18.0) * tokens * topk * hidden * ffn * layers
