@@ -90,8 +90,9 @@ def _fused_default() -> bool:
 # forward
 # ---------------------------------------------------------------------------------------------
 def moe_forward(ctx, streams, buffer, x, topk_idx, topk_weights, is_token_in_rank, w1, w2, num_experts,
-                cfg: TileConfig, level: int, fused: bool):
-    """Forward of one layer; fills ``ctx`` (any attribute bag) for :func:`moe_backward`."""
+                cfg: TileConfig, level: int, fused: bool, auto_width: bool = False):
+    """Forward of one layer; fills ``ctx`` (any attribute bag) for :func:`moe_backward`.  ``auto_width``: see
+    :func:`_native_config`."""
     global _NVTX_FWD
     _NVTX_FWD += 1
     _nvtx_push(f"moe_fwd_{_NVTX_FWD}")
@@ -108,7 +109,7 @@ def moe_forward(ctx, streams, buffer, x, topk_idx, topk_weights, is_token_in_ran
     if fused and buffer.group_size == 1:
         _nvtx_push(f"fwd_fused_{_NVTX_FWD}")
         buffer._next_seq += 1
-        out, ctx.local = rt.local_forward(x, topk_idx, topk_weights, w1, w2, num_experts, level, _native_config(cfg, False),
+        out, ctx.local = rt.local_forward(x, topk_idx, topk_weights, w1, w2, num_experts, level, _native_config(cfg, auto_width),
                                           comp.stream_id, comp.device_index)
         ctx.buffer, ctx.streams, ctx.fused = buffer, streams, fused
         _nvtx_pop()
@@ -437,17 +438,17 @@ class StreamMoEFunc(torch.autograd.Function):
 
     @staticmethod
     def forward(ctx, streams, buffer, x, topk_idx, topk_weights, is_token_in_rank, w1_local, w2_local,
-                num_experts, cfg, activation_checkpoint_level, fused):
+                num_experts, cfg, activation_checkpoint_level, fused, auto_width=False):
         ctx.state = SimpleNamespace()
         out = moe_forward(ctx.state, streams, buffer, x, topk_idx, topk_weights, is_token_in_rank, w1_local,
-                          w2_local, num_experts, cfg, activation_checkpoint_level, fused)
+                          w2_local, num_experts, cfg, activation_checkpoint_level, fused, auto_width)
         return out
 
     @staticmethod
     def backward(ctx, dL_dy):
         dL_dx, dL_dw, dW1, dW2 = moe_backward(ctx.state, dL_dy)
         ctx.state = None
-        return None, None, dL_dx, None, dL_dw, None, dW1, dW2, None, None, None, None
+        return None, None, dL_dx, None, dL_dw, None, dW1, dW2, None, None, None, None, None
 
 
 def stream_moe_func(buffer, x: torch.Tensor, topk_idx: torch.Tensor, topk_weights: torch.Tensor,
@@ -467,15 +468,21 @@ def stream_moe_func(buffer, x: torch.Tensor, topk_idx: torch.Tensor, topk_weight
     cfg = _resolve_tile_config(tile_config, I, H)
     if fused is None:
         fused = _fused_default()
-    if fused and buffer.group_size == 1 and not _NVTX_ENABLED:
+    if fused and buffer.group_size == 1:
         level = activation_checkpoint_level
         assert level in (0, 1, 2), "activation_checkpoint_level must be 0, 1 or 2"
         assert x.dtype == torch.bfloat16 and w1_local.dtype == torch.bfloat16 and w2_local.dtype == torch.bfloat16, "bf16 only"
         assert w2_local.shape == (E_local, H, I), f"w2_local must be [E_local, H, I], got {tuple(w2_local.shape)}"
         assert num_experts == E_local
-        buffer._next_seq += 1
-        comp = streams.compute
-        return buffer.runtime.local_layer(x, topk_idx, topk_weights, w1_local, w2_local, num_experts, level, _native_config(cfg, tile_config is None),
-                                          comp.stream_id, comp.device_index)
+        # With NVTX ranges on, a call that is differentiated goes through the Python node, whose backward can mark them; the
+        # kernels are the same.
+        if not _NVTX_ENABLED or not (torch.is_grad_enabled() and any(t.requires_grad for t in (x, topk_weights, w1_local, w2_local))):
+            _nvtx_push("moe_fwd")
+            buffer._next_seq += 1
+            comp = streams.compute
+            out = buffer.runtime.local_layer(x, topk_idx, topk_weights, w1_local, w2_local, num_experts, level,
+                                             _native_config(cfg, tile_config is None), comp.stream_id, comp.device_index)
+            _nvtx_pop()
+            return out
     return StreamMoEFunc.apply(streams, buffer, x, topk_idx, topk_weights, is_token_in_rank, w1_local, w2_local,
-                               num_experts, cfg, activation_checkpoint_level, fused)
+                               num_experts, cfg, activation_checkpoint_level, fused, tile_config is None)
