@@ -1554,8 +1554,7 @@ class Runtime : public std::enable_shared_from_this<Runtime> {
       d.mode = kVarlenK; d.epilogue = kEpiStore; d.a_mn_major = d.b_mn_major = true; d.dynamic_tiles = true;
       d.expert_pool_block_offset = st->expert_pool_block_offset; d.expert_frequency = st->expert_frequency;
       // Y_bwd wrote zeros into the padding rows of its two outputs; the pools get theirs here
-      ++launches_; launch_zero_pool_padding(pool.data_ptr(), g->dl_do_pool.data_ptr(), st->expert_frequency.data_ptr<int>(),
-                                            st->expert_pool_block_offset.data_ptr<int>(), st->num_experts / num_ranks_, H, stream());
+      zero_pool_padding(st, pool, g->dl_do_pool);
       d.padding_is_zero = true;
       if (tile_n_dw1 == tile_n_dw2) {
         d.block_n = tile_n_dw1;
@@ -1839,6 +1838,13 @@ class Runtime : public std::enable_shared_from_this<Runtime> {
     return tiles + 1.0 <= kPairWaste * (tiles + 0.5);
   }
 
+  // What the weight-gradient GEMM on CTA pairs asks of both pools (see launch_zero_pool_padding).
+  void zero_pool_padding(const std::shared_ptr<DispatchState>& st, const at::Tensor& pool, const at::Tensor& dl_pool) {
+    ++launches_; launch_zero_pool_padding(pool.data_ptr(), dl_pool.data_ptr(), st->expert_frequency.data_ptr<int>(),
+                                          st->expert_pool_block_offset.data_ptr<int>(), st->num_experts / num_ranks_, st->hidden, stream());
+    SEP_CUDA_CHECK(cudaGetLastError());
+  }
+
   // ---- small ops ---------------------------------------------------------------------------------------
   void tile_producer(const at::Tensor& count, const at::Tensor& target, double delay_us) {
     ++launches_; launch_tile_producer(count.data_ptr<int>(), target.data_ptr<int>(), count.numel(), static_cast<long long>(delay_us * 1000.0),
@@ -2108,7 +2114,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
       RO(x) RO(topk_idx) RO(topk_weights) RO(num_tokens) RO(hidden) RO(num_topk) RO(num_experts) RO(tile_m) RO(seq)
       RO(pair_rank) RO(pair_slot) RO(token_rank_in_channel) RO(send_recv_token) RO(send_head) RO(is_token_in_rank)
       RO(channel_prefix_matrix) RO(send_base) RO(send_token_base) RO(peer_total_tiles) RO(peer_num_recv)
-      RO(send_order_base) RO(send_list) RO(num_send)
+      RO(send_order_base) RO(send_list) RO(num_send) RO(pair_tiles) RO(num_pairs)
       RO(expert_frequency) RO(expert_pool_block_offset) RO(base_pool) RO(seen_per_substream) RO(rank_prefix_matrix)
       RO(recv_channel_prefix_matrix) RO(tile_id_to_expert) RO(pool_arrival_target)
       RO(pool) RO(pool_topk_weight) RO(pool_recv_token) RO(pool_k_slot) RO(pool_src) RO(recv_token_to_slots)
@@ -2220,6 +2226,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
       .def("get_epochs", &Runtime::get_epochs)
       .def("set_epochs", &Runtime::set_epochs)
       .def("grouped_gemm", &Runtime::grouped_gemm)
+      .def("zero_pool_padding", &Runtime::zero_pool_padding)
       .def("mark_local_phase", &Runtime::mark_local_phase)
       .def("local_phase_event", &Runtime::local_phase_event)
       // x, topk_idx, topk_weights, w1, w2, num_experts, level, config, stream id and device of the compute stream

@@ -64,6 +64,12 @@ def _args():
     return _ext.load().GemmArgs()
 
 
+def _use_pairs(a, pairs):
+    """Work on pairs of row tiles with CTA pairs where the dispatch (its native state) has a list of pairs worth using."""
+    if pairs is not None and pairs.num_pairs > 0:
+        a.pair_tiles, a.num_pairs = pairs.pair_tiles, pairs.num_pairs
+
+
 def streaming_moe_a(pool: torch.Tensor, w1: torch.Tensor, tile_id_to_expert: torch.Tensor, *,
                     postact_a: Optional[torch.Tensor] = None, preact_a: Optional[torch.Tensor] = None,
                     store_preact: bool = False,
@@ -71,7 +77,7 @@ def streaming_moe_a(pool: torch.Tensor, w1: torch.Tensor, tile_id_to_expert: tor
                     pool_arrival_target: Optional[torch.Tensor] = None,
                     tile_n: Optional[int] = None, num_sms: Optional[int] = None, buffer=None,
                     fused_dispatch=None, push_flags: int = 3, num_tiles: Optional[int] = None,
-                    live_tiles: Optional[torch.Tensor] = None):
+                    live_tiles: Optional[torch.Tensor] = None, pairs=None):
     """``postact[TKp, I] = swiglu(pool[TKp, H] @ w1[e]^T)`` tile by tile.
 
     ``w1`` is ``[E_local, 2I, H]`` with gate/up rows interleaved.  With
@@ -79,6 +85,7 @@ def streaming_moe_a(pool: torch.Tensor, w1: torch.Tensor, tile_id_to_expert: tor
     reached its target.  ``fused_dispatch`` (the native state of a dispatch whose
     push was not launched) makes the same kernel ship this rank's token rows to
     the peers' pools while its tensor-core warps consume tiles as they land.
+    ``pairs`` (a dispatch's native state): tiles are taken two by two where its list of pairs is worth using.
     Returns ``(postact_a, preact_a or None)``.
     """
     rows, H = pool.shape
@@ -106,13 +113,14 @@ def streaming_moe_a(pool: torch.Tensor, w1: torch.Tensor, tile_id_to_expert: tor
         a.push_flags = push_flags
     if live_tiles is not None and num_tiles is None:
         a.num_m_tiles_dev = live_tiles
+    _use_pairs(a, pairs)
     _rt(buffer).grouped_gemm(a)
     return postact_a, preact_a
 
 
 def grouped_gemm_preact(pool: torch.Tensor, w1: torch.Tensor, tile_id_to_expert: torch.Tensor, *,
                         out: Optional[torch.Tensor] = None, tile_n: Optional[int] = None,
-                        num_sms: Optional[int] = None, live_tiles: Optional[torch.Tensor] = None, buffer=None):
+                        num_sms: Optional[int] = None, live_tiles: Optional[torch.Tensor] = None, buffer=None, pairs=None):
     """``preact[TKp, 2I] = pool @ w1[e]^T`` (activation-checkpoint recompute)."""
     rows = pool.shape[0]
     two_i = w1.shape[1]
@@ -125,6 +133,7 @@ def grouped_gemm_preact(pool: torch.Tensor, w1: torch.Tensor, tile_id_to_expert:
         a.num_m_tiles_dev = live_tiles
     if num_sms:
         a.num_ctas = num_sms
+    _use_pairs(a, pairs)
     _rt(buffer).grouped_gemm(a)
     return out
 
@@ -160,7 +169,7 @@ def streaming_moe_y(postact_a: torch.Tensor, w2: torch.Tensor, tile_id_to_expert
                     pool_k_slot: Optional[torch.Tensor] = None, num_topk: int = 0,
                     tail_wait: bool = True, started_flag: bool = False,
                     tile_n: Optional[int] = None, num_sms: Optional[int] = None, buffer=None,
-                    remote_static_offset: int = -1, live_tiles: Optional[torch.Tensor] = None):
+                    remote_static_offset: int = -1, live_tiles: Optional[torch.Tensor] = None, pairs=None):
     """``y = postact @ w2[e]^T`` scaled by the slot's top-k weight and reduced
     with 16-byte bf16x2 ``red.add`` into
 
@@ -189,6 +198,7 @@ def streaming_moe_y(postact_a: torch.Tensor, w2: torch.Tensor, tile_id_to_expert
                     live_tiles=live_tiles)
     if num_sms:
         a.num_ctas = num_sms
+    _use_pairs(a, pairs)
     _rt(buffer).grouped_gemm(a)
     return o
 
@@ -202,7 +212,7 @@ def streaming_moe_a_bwd(dL_dswiglu_in: torch.Tensor, w1: torch.Tensor, tile_id_t
                         pool_k_slot: Optional[torch.Tensor] = None, num_topk: int = 0,
                         tail_wait: bool = True, started_flag: bool = False,
                         tile_n: Optional[int] = None, num_sms: Optional[int] = None, buffer=None,
-                        remote_static_offset: int = -1, live_tiles: Optional[torch.Tensor] = None):
+                        remote_static_offset: int = -1, live_tiles: Optional[torch.Tensor] = None, pairs=None):
     """``dpool = dL_dswiglu_in[TKp, 2I] @ w1[e]`` (NN GEMM, K = 2I) reduced into
     ``dL_dx_per_r[r]`` locally or into the source rank's ``dL_dx`` remotely
     (fused combine_grads).  No per-slot weight: it is already folded into
@@ -221,6 +231,7 @@ def streaming_moe_a_bwd(dL_dswiglu_in: torch.Tensor, w1: torch.Tensor, tile_id_t
                     remote_static_offset=remote_static_offset, live_tiles=live_tiles)
     if num_sms:
         a.num_ctas = num_sms
+    _use_pairs(a, pairs)
     _rt(buffer).grouped_gemm(a)
     return dL_dx_per_r
 
@@ -238,7 +249,7 @@ def streaming_moe_y_bwd(dL_do_pool: torch.Tensor, w2: torch.Tensor, preact_a: to
                         fused_dispatch_grads=None, fused_routing=None, fused_rows: Optional[torch.Tensor] = None,
                         push_flags: int = 3, num_tiles: Optional[int] = None,
                         tile_n: Optional[int] = None, num_sms: Optional[int] = None, buffer=None,
-                        remote_static_offset: int = -1, live_tiles: Optional[torch.Tensor] = None):
+                        remote_static_offset: int = -1, live_tiles: Optional[torch.Tensor] = None, pairs=None):
     """``g = dL_do_pool[TKp, H] @ w2[e]`` (NN GEMM, K = H) followed by the SwiGLU
     backward on the saved ``preact_a``:
 
@@ -284,6 +295,7 @@ def streaming_moe_y_bwd(dL_do_pool: torch.Tensor, w2: torch.Tensor, preact_a: to
         a.push_flags = push_flags
     if num_sms:
         a.num_ctas = num_sms
+    _use_pairs(a, pairs)
     _rt(buffer).grouped_gemm(a)
     return dL_dswiglu_in, postact_a_for_dW2, dL_dweight
 
@@ -292,7 +304,7 @@ def grouped_gemm_dw(lhs: torch.Tensor, rhs: torch.Tensor, expert_pool_block_offs
                     expert_frequency: torch.Tensor, *, out: Optional[torch.Tensor] = None,
                     tile_n: Optional[int] = None, num_sms: Optional[int] = None, buffer=None,
                     lhs2: Optional[torch.Tensor] = None, rhs2: Optional[torch.Tensor] = None,
-                    out2: Optional[torch.Tensor] = None, dynamic_tiles: bool = False):
+                    out2: Optional[torch.Tensor] = None, dynamic_tiles: bool = False, padding_is_zero: bool = False):
     """Per-expert weight gradient ``out[e] = lhs[rows_e]^T @ rhs[rows_e]`` with
     ``rows_e`` the expert's TRUE row range (padding rows never contribute, whatever
     they hold).  ``lhs [TKp, M]``, ``rhs [TKp, N]`` -> ``out [E, M, N]`` bf16, fp32
@@ -302,7 +314,8 @@ def grouped_gemm_dw(lhs: torch.Tensor, rhs: torch.Tensor, expert_pool_block_offs
     together: one tail wave instead of two); then ``(out, out2)`` is returned.  ``dynamic_tiles``: CTAs claim
     tiles from a device counter instead of striding by the grid size, so tiles of unequal length (experts with
     unequal row counts) balance out (reference: the ``atomicAdd`` claim of
-    stream_ep/stream_moe/tile_scheduler.py:336-342)."""
+    stream_ep/stream_moe/tile_scheduler.py:336-342).  ``padding_is_zero``: the caller warrants that in all operands the
+    rows past an expert's length, up to the next multiple of 64, hold zeros, which the form on CTA pairs needs."""
     E = expert_frequency.numel()
     M, N = lhs.shape[1], rhs.shape[1]
     if out is None:
@@ -312,7 +325,7 @@ def grouped_gemm_dw(lhs: torch.Tensor, rhs: torch.Tensor, expert_pool_block_offs
     a.a_mn_major = a.b_mn_major = True
     a.a, a.b, a.out0 = lhs, rhs, out
     a.expert_pool_block_offset, a.expert_frequency = expert_pool_block_offset, expert_frequency
-    a.dynamic_tiles = bool(dynamic_tiles)
+    a.dynamic_tiles, a.padding_is_zero = bool(dynamic_tiles), bool(padding_is_zero)
     if lhs2 is not None:
         if out2 is None:
             out2 = torch.empty(E, lhs2.shape[1], rhs2.shape[1], dtype=lhs.dtype, device=lhs.device)

@@ -171,7 +171,7 @@ def moe_forward(ctx, streams, buffer, x, topk_idx, topk_weights, is_token_in_ran
             _nvtx_push(f"fwd_combine_{_NVTX_FWD}")
             gg.streaming_moe_y(postact, w2c, handle.tile_id_to_expert, handle.pool_topk_weight,
                                handle.pool_recv_token, o=out, remote_out_offsets=(KIND_DISPATCH, st.push_epoch, AUX0),
-                               remote_static_offset=landing_off, live_tiles=st.dev_sizes if cap else None,
+                               remote_static_offset=landing_off, live_tiles=st.dev_sizes if cap else None, pairs=st,
                                pool_src=handle.pool_src, pool_k_slot=handle.pool_k_slot, num_topk=K,
                                tail_wait=not buffer._emulated, tile_n=cfg.tile_n_y, num_sms=cfg.num_sms_y, buffer=buffer)
             buffer._phase()
@@ -236,7 +236,7 @@ def _launch_fused_a(buffer, handle, w1, postact, preact, cfg):
     st = handle._dispatch_out
     common = dict(postact_a=postact, preact_a=preact, pool_arrival_count=handle.pool_arrival_count,
                   pool_arrival_target=handle.pool_arrival_target, tile_n=cfg.tile_n_a, num_sms=cfg.num_sms_a,
-                  buffer=buffer, fused_dispatch=st, live_tiles=st.dev_sizes if st.region_id >= 0 else None)
+                  buffer=buffer, fused_dispatch=st, live_tiles=st.dev_sizes if st.region_id >= 0 else None, pairs=st)
     if not buffer._emulated:
         gg.streaming_moe_a(handle.pool, w1, handle.tile_id_to_expert, push_flags=3, **common)
         return
@@ -315,7 +315,7 @@ def moe_backward(ctx, dL_dy):
         if preact is None:
             preact = gg.grouped_gemm_preact(pool, sv.w1, handle.tile_id_to_expert, tile_n=cfg.tile_n_a,
                                             live_tiles=st.dev_sizes if st.region_id >= 0 else None,
-                                            buffer=buffer) if tiles > 0 else pool.new_empty(0, 2 * I)
+                                            pairs=st if fused else None, buffer=buffer) if tiles > 0 else pool.new_empty(0, 2 * I)
         return pool, preact
 
     if fused:
@@ -330,7 +330,7 @@ def moe_backward(ctx, dL_dy):
             ykw = dict(dL_dswiglu_in=dswiglu_in, postact_a_for_dW2=postact_dw2, dL_dweight=dl_dweight,
                        arrival_count=bwd_count, arrival_target=handle.pool_arrival_target,
                        remote_dw_offsets=(KIND_DISPATCH_GRADS, g.epoch, AUX1), remote_static_offset=g.dwt_off,
-                       live_tiles=live, pool_src=handle.pool_src,
+                       live_tiles=live, pairs=st, pool_src=handle.pool_src,
                        pool_k_slot=handle.pool_k_slot, num_topk=K, tile_n_stripes_done=stripes_y,
                        fused_dispatch_grads=g, fused_routing=st, fused_rows=dL_dy, tile_n=cfg.tile_n_y_bwd,
                        num_sms=cfg.num_sms_y_bwd, buffer=buffer)
@@ -345,7 +345,7 @@ def moe_backward(ctx, dL_dy):
                 gg.streaming_moe_y_bwd(*yargs, push_flags=0, **ykw)
             gg.streaming_moe_a_bwd(dswiglu_in, sv.w1, handle.tile_id_to_expert, handle.pool_recv_token,
                                    dL_dx_per_r=dx, remote_out_offsets=(KIND_DISPATCH_GRADS, g.epoch, AUX0),
-                                   remote_static_offset=g.landing_off, live_tiles=live,
+                                   remote_static_offset=g.landing_off, live_tiles=live, pairs=st,
                                    pool_src=handle.pool_src, pool_k_slot=handle.pool_k_slot, num_topk=K,
                                    tail_wait=not buffer._emulated, tile_n=cfg.tile_n_a_bwd,
                                    num_sms=cfg.num_sms_a_bwd, buffer=buffer)
@@ -359,7 +359,9 @@ def moe_backward(ctx, dL_dy):
                 gg.combine_reduce(dx, landing, st.topk_idx, st.num_experts, buffer=buffer)
             buffer._phase()
             del landing
-            _launch_dw(buffer, handle, cfg, dl_do_pool, postact_dw2, dswiglu_in, pool, dW1, dW2)
+            if tiles > 0:     # (Y_bwd wrote zeros into the padding rows of its outputs)
+                rt.zero_pool_padding(st, pool, dl_do_pool)
+            _launch_dw(buffer, handle, cfg, dl_do_pool, postact_dw2, dswiglu_in, pool, dW1, dW2, padding_is_zero=True)
         dL_dx, dL_dw = dx, dwt
     else:
         with torch.cuda.stream(comm):
@@ -398,20 +400,20 @@ def moe_backward(ctx, dL_dy):
     return dL_dx, dL_dw, dW1, dW2
 
 
-def _launch_dw(buffer, handle, cfg, dl_do_pool, postact_dw2, dswiglu_in, pool, dW1, dW2):
+def _launch_dw(buffer, handle, cfg, dl_do_pool, postact_dw2, dswiglu_in, pool, dW1, dW2, padding_is_zero=False):
     """dW2[e] = dL_do_pool[rows_e]^T @ (w * postact)[rows_e];  dW1[e] = dL_dswiglu_in[rows_e]^T @ pool[rows_e]
     (stream_ep/stream_moe/stream_moe.py:1107-1146, including the empty-rank guard)."""
     buffer.runtime.mark_local_phase()
     if handle.total_tiles > 0:
         if cfg.tile_n_dW1 == cfg.tile_n_dW2:      # one launch for both, tiles claimed dynamically
             gg.grouped_gemm_dw(dswiglu_in, pool, handle.expert_pool_block_offset, handle.expert_frequency, out=dW1,
-                               lhs2=dl_do_pool, rhs2=postact_dw2, out2=dW2, tile_n=cfg.tile_n_dW1, dynamic_tiles=True,
+                               lhs2=dl_do_pool, rhs2=postact_dw2, out2=dW2, tile_n=cfg.tile_n_dW1, dynamic_tiles=True, padding_is_zero=padding_is_zero,
                                buffer=buffer)
         else:
             gg.grouped_gemm_dw(dl_do_pool, postact_dw2, handle.expert_pool_block_offset, handle.expert_frequency,
-                               out=dW2, tile_n=cfg.tile_n_dW2, dynamic_tiles=True, buffer=buffer)
+                               out=dW2, tile_n=cfg.tile_n_dW2, dynamic_tiles=True, padding_is_zero=padding_is_zero, buffer=buffer)
             gg.grouped_gemm_dw(dswiglu_in, pool, handle.expert_pool_block_offset, handle.expert_frequency,
-                               out=dW1, tile_n=cfg.tile_n_dW1, dynamic_tiles=True, buffer=buffer)
+                               out=dW1, tile_n=cfg.tile_n_dW1, dynamic_tiles=True, padding_is_zero=padding_is_zero, buffer=buffer)
     else:
         dW1.zero_()
         dW2.zero_()
