@@ -1588,7 +1588,7 @@ class Runtime : public std::enable_shared_from_this<Runtime> {
                "topk_idx and topk_weights must be [T, K] CUDA tensors over the tokens of x");
     SEP_ASSERT(num_experts <= ctl_.num_experts_cap, "num_experts must fit the Buffer's expert capacity");
     SEP_ASSERT(x_in.size(1) % 8 == 0 && w2_in.size(2) % 8 == 0, "hidden and ffn must be multiples of 8");
-    SEP_ASSERT(idx_in.size(1) >= 1 && idx_in.size(1) <= kMaxTopK, "num_topk out of range");
+    SEP_ASSERT(idx_in.size(1) <= kMaxTopK, "num_topk too large");
     SEP_ASSERT(w1_in.is_cuda() && w2_in.is_cuda() && w1_in.dim() == 3 && w1_in.size(0) == num_experts && w1_in.size(2) == x_in.size(1) &&
                w2_in.size(1) == x_in.size(1) && w1_in.size(1) == 2 * w2_in.size(2), "expert weights do not match x and num_experts");
     const c10::cuda::CUDAStream caller = at::cuda::getCurrentCUDAStream();
