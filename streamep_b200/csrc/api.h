@@ -310,8 +310,9 @@ struct RouterParams {
 };
 void launch_router(const RouterParams& p, cudaStream_t stream);
 // The tensor-core router in one launch: `map_w` [E, H] with boxes of 128 x 64 and `map_x` [T, H] with boxes of
-// router_tile_tokens() x 64 elements, both bf16 with 128-byte swizzle (p.x / p.w_gate are not read).
-int router_tile_tokens(const RouterParams& p, int sms);
+// RouterTile::tile_tokens x 64 elements, both bf16 with 128-byte swizzle (p.x / p.w_gate are not read).
+struct RouterTile { int tile_tokens, splits, blocks, stages, smem_bytes, tmem_cols; };
+RouterTile router_tile(const RouterParams& p, int sms);
 cudaError_t launch_router_mma(const RouterParams& p, const void* map_w, const void* map_x, int sms, StatusBlock* status,
                               unsigned long long wait_budget_ns, cudaStream_t stream);
 

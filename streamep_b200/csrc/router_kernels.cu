@@ -92,8 +92,6 @@ constexpr int kRouterThreads = 512;
 constexpr int kRouterMaxStages = 8;
 constexpr int kRouterMaxSmem = 224 * 1024;
 
-struct RouterTile { int tile_tokens, splits, blocks, stages, smem_bytes, tmem_cols; };
-
 // logits of a tile: rows of e_pad floats (odd, so that the 32 experts a warp writes for one token and the rows of
 // consecutive tokens fall into different banks)
 __host__ __device__ constexpr int router_e_pad(int experts) { return (experts + 127) / 128 * 128 + 1; }
@@ -237,8 +235,6 @@ RouterTile router_tile(const RouterParams& p, int sms) {
   while (g.tmem_cols < g.blocks * g.tile_tokens) g.tmem_cols *= 2;
   return g;
 }
-
-int router_tile_tokens(const RouterParams& p, int sms) { return router_tile(p, sms).tile_tokens; }
 
 template <int EPL>
 static cudaError_t launch_router_width(const RouterParams& p, const RouterTile& g, const CUtensorMap& map_w, const CUtensorMap& map_x,

@@ -1914,7 +1914,7 @@ class Runtime : public std::enable_shared_from_this<Runtime> {
       if (router_on_tensor_cores_) {
         const int64_t T = x.size(0), H = x.size(1), E = w_gate.size(0);
         const CUtensorMap mw = make_tmap(w_gate.data_ptr(), H, E, 1, H, E * H, 64, 128);
-        const CUtensorMap mx = make_tmap(x.data_ptr(), H, T, 1, H, T * H, 64, router_tile_tokens(p, num_sms()));
+        const CUtensorMap mx = make_tmap(x.data_ptr(), H, T, 1, H, T * H, 64, router_tile(p, num_sms()).tile_tokens);
         SEP_CUDA_CHECK(launch_router_mma(p, &mw, &mx, num_sms(), status_, budget_ns_, stream()));
       } else {
         launch_router(p, stream());
@@ -1922,6 +1922,13 @@ class Runtime : public std::enable_shared_from_this<Runtime> {
     }
     SEP_CUDA_CHECK(cudaGetLastError());
     return {idx, w, in_rank, probs};
+  }
+  // {tokens per tile, CTAs that share the hidden dimension, pipeline stages} of the tensor-core router for a shape
+  std::vector<int> router_plan(int tokens, int hidden, int experts) {
+    RouterParams p{};
+    p.num_tokens = tokens; p.hidden = hidden; p.num_experts = experts;
+    const RouterTile g = router_tile(p, num_sms());
+    return {g.tile_tokens, g.splits, g.stages};
   }
   // false: the SIMT router kernel
   void set_router_on_tensor_cores(bool on) { router_on_tensor_cores_ = on; }
@@ -2187,6 +2194,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
       .def("set_split_local", &Runtime::set_split_local)
       .def("set_active_push_warps", &Runtime::set_active_push_warps)
       .def("set_push_order", &Runtime::set_push_order)
+      .def("router_plan", &Runtime::router_plan)
       .def("set_router_on_tensor_cores", &Runtime::set_router_on_tensor_cores)
       .def("arena_bytes_in_use", &Runtime::arena_bytes_in_use)
       .def("arena_high_water", &Runtime::arena_high_water)

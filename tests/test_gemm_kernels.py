@@ -281,9 +281,10 @@ def test_pool_compress_roundtrip(native):
                                        (257, 1032, 256, 8, 8), (64, 512, 136, 3, 1)])
 @pytest.mark.parametrize("tensor_cores", [True, False])
 def test_router(native, T, H, E, K, R, tensor_cores):
-    """Both router paths - logits from the tcgen05 grouped GEMM with the fp32 store epilogue plus the finishing
-    kernel, and the SIMT kernel in every expert-width instance (16 / 32 / 64 experts per pass, several passes,
-    widths that are not a multiple of the chunk) - against softmax -> top-k -> renormalise in fp32."""
+    """Both router paths - the tcgen05 kernel with the hidden dimension split over a cluster (short calls; the long ones
+    and its other tiles: tests/test_router_tiles.py) and the SIMT kernel in every expert-width instance (16 / 32 / 64
+    experts per pass, several passes, widths that are not a multiple of the chunk) - against softmax -> top-k ->
+    renormalise in fp32."""
     from streamep_b200.models.reference import router_reference
     gg = _ops()
     g = torch.Generator(device="cpu").manual_seed(20)
