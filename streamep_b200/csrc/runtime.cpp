@@ -407,6 +407,20 @@ struct LayerConfig {
   bool auto_width;                     // the widths are defaults, not the caller's choice
 };
 
+static int64_t up(int64_t a, int64_t b) { return (a + b - 1) / b; }
+// Work on pairs of row tiles leaves half of a pair idle where a count is odd.  Pairs pay as long as they have at most this many
+// times as many tile slots as there are tiles.
+static constexpr double kPairWaste = 1.15;
+// Row tiles of experts, from the mean load (for a dispatch whose counts the host does not read): half a tile lost per expert.
+static bool pairs_pay(int64_t pairs, int64_t experts) {
+  const double tiles = static_cast<double>(pairs) / static_cast<double>(experts) / kTileM;      // per expert
+  return tiles + 1.0 <= kPairWaste * (tiles + 0.5);
+}
+// Row tiles of weight gradients with `m` and (0: none) `m2` rows.
+static bool dw_pairs_pay(int64_t m, int64_t m2) {
+  return 2.0 * (up(m, 2 * kTileM) + up(m2, 2 * kTileM)) <= kPairWaste * (up(m, kTileM) + up(m2, kTileM));
+}
+
 // What the forward of a single-rank layer keeps for its backward.
 struct LocalState : torch::CustomClassHolder {
   std::shared_ptr<Runtime> runtime;
@@ -422,26 +436,30 @@ struct LocalState : torch::CustomClassHolder {
   at::Tensor preact, w1, w2;
   std::shared_ptr<void> region_guard;  // capacity mode
 
-  // Tile width of a GEMM over row tiles with `n` output columns.  128 instead of 256 when that ends at least a quarter
-  // earlier by the count of rounds x width (experts equally loaded): a call with few tiles, whose 256-wide ones leave SMs idle
-  // or a last round nearly empty.  Wide tiles feed the tensor cores better (half the operand bytes per product), which
-  // is why a tie goes to them.  1777 tokens, hidden 1000, ffn 520, 12 experts: 198 -> 187 us a training pass; 16 tokens,
-  // hidden 2048, 8 experts: 52.7 -> 50.5 us a forward (with the prefetch of local_kernels.cu).
+  // Tile width of a GEMM over row tiles with `n` output columns, from the count of rounds (experts equally loaded).  A round of
+  // 128-wide tiles reads 32 KB of operands per SM and k-block, as much as a round of CTA pairs and two thirds of a round of
+  // 256-wide tiles of single CTAs, and operands are what these kernels wait for.  Against pairs, narrow tiles therefore pay
+  // only where they need a single round (a call that leaves SMs idle: half the epilogue, twice the SMs), and against single
+  // CTAs where they need at most 3 rounds for 2.  us, 128 / 256 wide, top-6 of 8 experts, hidden 2048, ffn 1408 where nothing
+  // else is said: pairs, 512 tokens: 2 rounds each 50 / 46 (Y_bwd), 3 for 2 49 / 37 (Y), 4 for 3 68 / 52 (A); 683 tokens: 6 for 4
+  // 79 / 53 (A); 1200 tokens, top-2 of 4, hidden 256, ffn 128: 1 round each 0.62 to 0.78 of the time.  Single CTAs: 1 round each
+  // 27 / 45 (16 tokens, Y), 3 for 2 63 / 70 (384 tokens, A_bwd), 2 for 1 0.82 to 1.44 of the time over ten shapes.
   int width(int preferred, int64_t n, int sms) const {
     if (!cfg.auto_width || preferred != 256 || n <= 128) return preferred;
     const int64_t P = static_cast<int64_t>(tokens) * topk, hit = std::max<int64_t>(1, std::min<int64_t>(experts, P));
     const int64_t per = up(up(P, hit), kTileM);          // row tiles of an expert
-    const int64_t wide = pairs > 0 ? up(hit * up(per, 2) * up(n, 256), sms / 2) : up(hit * per * up(n, 256), sms);
     const int64_t narrow = up(hit * per * up(n, 128), sms);
-    return narrow * 128 * 4 <= wide * 256 * 3 ? 128 : 256;
+    if (pairs > 0) return narrow == 1 ? 128 : 256;
+    return narrow * 2 <= up(hit * per * up(n, 256), sms) * 3 ? 128 : 256;
   }
-  // One width for dW1 [2 ffn, hidden] and dW2 [hidden, ffn] in one launch, by the same count (0: two launches, the caller's widths).
+  // One width for dW1 [2 ffn, hidden] and dW2 [hidden, ffn] in one launch (0: two launches, the caller's widths).  Pairs are
+  // never slower here, not even where both need one round (9.8 us against 10.6: 4 experts, hidden 256, ffn 128).
   int dw_width(int sms) const {
     if (!cfg.auto_width) return cfg.tile_n_dw1 == cfg.tile_n_dw2 ? cfg.tile_n_dw1 : 0;
-    auto units = [&](int64_t m) { return experts * (up(2 * ffn, m) * up(hidden, m) + up(hidden, m) * up(ffn, m)); };
-    return up(units(128), sms) * 128 * 4 <= up(units(256), sms / 2) * 256 * 3 ? 128 : 256;
+    if (dw_pairs_pay(2 * static_cast<int64_t>(ffn), hidden)) return 256;
+    auto units = [&](int64_t n) { return experts * (up(2 * ffn, kTileM) * up(hidden, n) + up(hidden, kTileM) * up(ffn, n)); };
+    return up(units(128), sms) * 2 <= up(units(256), sms) * 3 ? 128 : 256;
   }
-  static int64_t up(int64_t a, int64_t b) { return (a + b - 1) / b; }
 };
 
 class Runtime : public std::enable_shared_from_this<Runtime> {
@@ -1270,8 +1288,7 @@ class Runtime : public std::enable_shared_from_this<Runtime> {
       const int64_t M2_ = a.a2.has_value() ? a.a2->size(1) : 0;
       // Pairs of 128-row tiles of the output, unless too many of them would have no second tile.
       auto units = [](int64_t m, int64_t rows_per_unit) { return (m + rows_per_unit - 1) / rows_per_unit; };
-      p.pair_ctas = a.padding_is_zero && BN == 256 &&
-                    2.0 * (units(M, 2 * BM_) + units(M2_, 2 * BM_)) <= kPairWaste * (units(M, BM_) + units(M2_, BM_));
+      p.pair_ctas = a.padding_is_zero && BN == 256 && dw_pairs_pay(M, M2_);
       const int64_t unit_m = p.pair_ctas ? 2 * BM_ : BM_;
       p.num_m_tiles = units(M, unit_m); p.num_n_tiles = (N + BN - 1) / BN;
       p.expert_pool_block_offset = a.expert_pool_block_offset->data_ptr<int>();
@@ -1769,7 +1786,7 @@ class Runtime : public std::enable_shared_from_this<Runtime> {
       const int64_t rows = a.size(0), M = a.size(1), N = b.size(1), M2 = out2 ? a2.size(1) : 0, E = st.experts;
       auto units = [](int64_t m, int64_t rows_per_unit) { return (m + rows_per_unit - 1) / rows_per_unit; };
       p.a_mn_major = p.b_mn_major = 1;
-      p.pair_ctas = p.block_n == 256 && 2.0 * (units(M, 2 * BM_) + units(M2, 2 * BM_)) <= kPairWaste * (units(M, BM_) + units(M2, BM_));
+      p.pair_ctas = p.block_n == 256 && dw_pairs_pay(M, M2);
       const int64_t unit_m = p.pair_ctas ? 2 * BM_ : BM_;
       p.N = N; p.M_out = M; p.out_expert_stride = M * N;
       p.num_m_tiles = units(M, unit_m); p.num_n_tiles = (N + p.block_n - 1) / p.block_n;
@@ -1829,13 +1846,17 @@ class Runtime : public std::enable_shared_from_this<Runtime> {
   static void use_pairs(GemmArgs& a, const DispatchState& st) {
     if (st.num_pairs > 0) { a.pair_tiles = st.pair_tiles; a.num_pairs = st.num_pairs; }
   }
-  // An expert with an odd number of row tiles leaves half of its last pair idle, half a tile per expert on average.
-  // Pairs pay as long as they have at most this many times as many tile slots as there are tiles.
-  static constexpr double kPairWaste = 1.15;
-  // The same decision from the mean load, for a dispatch whose counts the host does not read.
-  static bool pairs_pay(int64_t pairs, int64_t experts) {
-    const double tiles = static_cast<double>(pairs) / static_cast<double>(experts) / kTileM;      // per expert
-    return tiles + 1.0 <= kPairWaste * (tiles + 0.5);
+  // {A, Y, Y_bwd, A_bwd, dW} tile widths of a single-rank layer on `sms` SMs, negative where the GEMM runs on CTA pairs.
+  static std::vector<int> layer_widths(int tokens, int hidden, int ffn, int experts, int topk, int sms, const LayerConfig& cfg) {
+    LocalState st;
+    st.cfg = cfg; st.tokens = tokens; st.hidden = hidden; st.ffn = ffn; st.experts = experts; st.topk = topk;
+    st.pairs = pairs_pay(static_cast<int64_t>(tokens) * topk, experts) ? 1 : 0;
+    std::vector<int> w = {st.width(cfg.tile_n_a, 2 * ffn, sms), st.width(cfg.tile_n_y, hidden, sms), st.width(cfg.tile_n_y_bwd, ffn, sms),
+                          st.width(cfg.tile_n_a_bwd, hidden, sms)};
+    for (int& v : w) if (v == 256 && st.pairs > 0) v = -v;
+    const int d = st.dw_width(sms);
+    w.push_back(d == 256 && dw_pairs_pay(2 * static_cast<int64_t>(ffn), hidden) ? -d : d);
+    return w;
   }
 
   // What the weight-gradient GEMM on CTA pairs asks of both pools (see launch_zero_pool_padding).
@@ -2085,6 +2106,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.attr("MAX_CHANNELS") = kMaxChannels;
   m.attr("MAX_EXPERTS") = kMaxExperts;
   m.def("is_sm100_compiled", [] { return true; });
+  m.def("layer_widths", &Runtime::layer_widths);
   m.def("layer_bytes_hint", &ArenaSizeHint::layer_bytes);
 
   py::class_<ArenaProbe>(m, "ArenaProbe")
