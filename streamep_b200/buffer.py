@@ -307,7 +307,10 @@ class Buffer:
         and in ``overflow_info()``, and reported by ``check_status()`` as :class:`StreamEPOverflow` - i.e. one
         step late, without a device sync in the step itself.  Dispatches whose shape differs from the
         configured one (more tokens, another hidden size or top-k) keep using exactly sized buffers.
-        The stand-alone ``dispatch`` keeps exact sizing unless called with ``capacity_mode=True``."""
+        The stand-alone ``dispatch`` keeps exact sizing unless called with ``capacity_mode=True``.
+
+        The regions are handed out in the order of the host calls and reused in the order of one stream: issue the layers of a
+        buffer in this mode through one ``StreamHolder`` (in exact mode, layers of a single rank may run on several)."""
         import torch.distributed as dist
 
         R = self.group_size

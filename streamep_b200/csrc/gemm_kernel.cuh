@@ -565,9 +565,8 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
       }
       const uint32_t taddr = tmem_base + acc * BN + (static_cast<uint32_t>(quarter * 32) << 16);
       // The accumulator goes back as soon as this warp has read its last columns (one arrival per warp, on the barrier of the
-      // CTA that issues the MMAs), not after they were stored.  With a short reduction the epilogue bounds a tile (12 k-blocks:
-      // 10,500 cycles against 6,100 of products), and the arrival as a release at cluster scope held every warp until its
-      // reductions had been performed, a sixth of its time.  Y at 32008 rows, hidden 3072, ffn 768: 172 -> 149 us; Y_bwd at
+      // CTA that issues the MMAs), not after they were stored.  With a short reduction the epilogue bounds a tile, and an
+      // arrival that releases at cluster scope held every warp until its reductions had been performed.  Y at 32008 rows, hidden 3072, ffn 768: 172 -> 149 us; Y_bwd at
       // 49152 rows, hidden 2048, ffn 1408: 316 -> 267 us.
       const int c_last = min(c_begin + kChunksPerHalf, (prob_n - n0 + 31) / 32) - 1;
       bool given_back = empty;

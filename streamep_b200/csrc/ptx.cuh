@@ -248,7 +248,8 @@ __device__ __forceinline__ void cluster_sync() {
   asm volatile("barrier.cluster.arrive.release;\n\tbarrier.cluster.wait.acquire;" ::: "memory");
 }
 // Arrives on a barrier of another CTA of the cluster for work ordered by tcgen05 fences.  No memory of this thread has to
-// become visible with it: a release at cluster scope would wait for every global store and reduction in flight.
+// become visible to that CTA with it, so the instruction keeps its default, a release at CTA scope: one at cluster scope
+// would wait for every global store and reduction in flight.
 __device__ __forceinline__ void mbar_arrive_cluster(uint32_t cluster_addr) {
   asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" :: "r"(cluster_addr) : "memory");
 }
@@ -315,8 +316,9 @@ __device__ __forceinline__ void tma_store_3d(const void* tmap, const void* smem_
 __device__ __forceinline__ void bulk_commit() { asm volatile("cp.async.bulk.commit_group;" ::: "memory"); }
 // the source shared memory of all committed groups has been read (it may be overwritten)
 __device__ __forceinline__ void bulk_wait_read() { asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory"); }
-// all committed groups are complete (their global writes are performed)
+// ... of all but the last committed group
 __device__ __forceinline__ void bulk_wait_read_but_one() { asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory"); }
+// all committed groups are complete (their global writes are performed)
 __device__ __forceinline__ void bulk_wait_all() { asm volatile("cp.async.bulk.wait_group 0;" ::: "memory"); }
 
 __device__ __forceinline__ void st_shared_v4(uint32_t addr, uint32_t a, uint32_t b, uint32_t c, uint32_t d) {

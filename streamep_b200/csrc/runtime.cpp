@@ -638,8 +638,8 @@ class Runtime : public std::enable_shared_from_this<Runtime> {
     return local_phase_ ? std::optional<EventHandle>(*local_phase_) : std::nullopt;
   }
   // Per-CTA time stamps of the GEMM kernels (see GemmParams::timing).  Returns the tensor the launches that follow
-  // fill: int64 [10, num_sms, 8], first index = epilogue kind (0 store, 1 SwiGLU, 2 scatter, 3 dSwiGLU, 4 fp32 store),
-  // + 5 for the launches with a fused push.  Each launch overwrites the rows of its kind.  `on = false` stops it.
+  // fill: int64 [10, num_sms, kTimingCols], first index = kind of launch: 0 weight gradients, 1 A, 2 Y, 3 Y_bwd, 5 recomputed
+  // pre-activation, 6 A and 8 Y_bwd with a fused push, 7 A_bwd.  Each launch overwrites the rows of its kind.  `on = false` stops it.
   at::Tensor set_kernel_timing(bool on) {
     if (!on) { timing_ = at::Tensor(); return timing_; }
     timing_ = at::zeros({10, num_sms(), kTimingCols}, at::TensorOptions().dtype(at::kLong).device(at::kCUDA, device_));
@@ -1808,7 +1808,9 @@ class Runtime : public std::enable_shared_from_this<Runtime> {
     // each time, which costs power more than time (the SM clock fell to 975 MHz where cuBLAS ran at 1350): bands are then as
     // high as their own rows of A stay in half of the L2, 8 to 32 tiles.  Otherwise low bands are better, they keep fewer rows
     // of A alive.  us for 16384 tokens, hidden 4096, ffn 14336, bands of 8 -> 16 -> 32 tiles: forward 9370 -> 9150 -> 9030, forward
-    // and backward 28500 -> 27950 -> 27990; where B fits (hidden 7168, ffn 2048): forward 3200 -> 3215 -> 3290.
+    // and backward 28500 -> 27950 -> 27990; where B fits (hidden 7168, ffn 2048): forward 3200 -> 3215 -> 3290.  The line lies where B
+    // stops fitting; for a B of 80 to 160 MB (six shapes of 2048 to 16384 tokens) neither order is ahead by more than the
+    // runs of one order differ (0.96 to 1.03 of its time, at a clock that the power cap moves).
     static int tile_band(int64_t k, int64_t n) {
       constexpr int64_t kHalfL2 = 64 << 20;
       if (k * n * 2 <= kHalfL2) return 0;

@@ -1,6 +1,6 @@
 """Python entry points of the tcgen05 grouped-GEMM kernels.
 
-One native kernel template (``csrc/gemm_kernels.cu``) serves all of these; the
+One native kernel template (``csrc/gemm_kernel.cuh``) serves all of these; the
 wrappers only assemble its argument bag.  Names and argument order follow the
 reference wrappers so call sites read the same:
 

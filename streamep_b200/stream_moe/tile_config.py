@@ -3,8 +3,8 @@
 Same public surface as the reference (stream_ep/stream_moe/stream_moe.py:126-367):
 a frozen, all-optional ``TileConfig`` of overrides, ``default_tile_config(I, H)``
 and ``_resolve_tile_config``.  The values differ because the kernels do: on
-sm_100a one CTA drives a 128 x tile_n UMMA with the accumulator in tensor
-memory, so
+sm_100a one CTA drives a 128 x tile_n UMMA, or a pair of CTAs a 256 x 256 one,
+with the accumulator in tensor memory, so
 
 * ``tile_m`` is structurally 128 (one UMMA M tile == the pool padding grain);
 * every ``tile_n`` is 128 or 256 (two accumulator buffers of ``tile_n`` fp32
