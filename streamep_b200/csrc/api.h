@@ -414,7 +414,7 @@ constexpr int kTimingCols = 12;
 
 // tmap_a / tmap_b: 128-byte CUtensorMap blobs (3-D, bf16, 128-byte swizzle) built by the host.
 // tmap_o0 / tmap_o1: output maps for the TMA-store epilogues (store, swiglu, dswiglu); box 32 rows x one
-// staging row (32, 64 or 128 bytes) with the matching swizzle.  Null for the scatter epilogue.
+// staging row (32, 64 or 128 bytes; store: 128) with the matching swizzle.  Null for the scatter epilogue.
 // Returns false, launching nothing, when no kernel instance exists for the mode / layout / epilogue combination.
 // `setup_error` (optional) receives the error of the per-device kernel set-up (shared-memory attribute); when it is
 // not cudaSuccess nothing was launched either.

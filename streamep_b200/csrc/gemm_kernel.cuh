@@ -42,12 +42,22 @@ constexpr int kGemmWarps = 10;   // 0: TMA producer, 1: MMA issuer + TMEM owner,
 // the tile gates AHEAD of the TMA producer.  A gate poll is an acquire load at system scope, microseconds long
 // while NVLink traffic is landing; done by the producer itself it stalls the operand pipeline once per tile.
 constexpr bool has_gate_warp(int epi) { return epi == kEpiSwiglu || epi == kEpiDswiglu; }
-constexpr int base_warps(int epi) { return kGemmWarps + (has_gate_warp(epi) ? 1 : 0); }
+// The weight-gradient kernels (VarlenK, both operands MN-major) carry one whose lane 0 schedules: it claims the next unit, reads
+// its expert's rows and queues the result for the other roles of both CTAs.  Operands arrive at the rate at which L2 delivers
+// them, so time that the producer spends on anything else is never made up for: a claim (an atomic, a copy to the other CTA, two
+// loads), and each store with release semantics, which waits for the copies in flight.  The other roles therefore report to
+// the scheduler with plain stores.  SM cycles of the MMA loop before and after: 32 experts of 512 rows, hidden 3072, ffn 768
+// 412 -> 323 thousand; of 1250 rows, hidden 7168, ffn 2048 4130 -> 3775; 12 of 440, hidden 1000, ffn 520 48 -> 39; 8 of 6144 (few long
+// units) 785 -> 795.  The kernels over row tiles, whose order is static, lose by such a queue (Y of 32008 rows 171 -> 187).
+constexpr int base_warps(int epi, bool schedules) { return kGemmWarps + (schedules || has_gate_warp(epi) ? 1 : 0); }
 // extra warps of the fused variants; the dSwiGLU epilogue keeps two preact segments in registers, so it gets fewer
 // (Y_bwd: 16 warps x 128 registers, A: 20 warps x 96 registers fill the register file)
 constexpr int push_warps(int epi) { return epi == kEpiDswiglu ? 5 : 9; }
 constexpr int kMaxDevices = 64;  // per-device host-side tables (kernel attributes, no-alloc scratch address)
-constexpr int kTileQueue = 8;    // dynamic tile claim: tiles the TMA thread may be ahead of the epilogue
+constexpr int kTileQueue = 8;    // tiles the scheduler may be ahead of the epilogue
+// A claimed tile is work that no idle CTA can take any more, so the scheduler claims late: when the producer has this many
+// k-blocks of the tile before left to issue, about the time that a claim takes until its first operands can be requested.
+constexpr int kClaimAhead = 10;
 constexpr int kEpiWarps = 8;     // two threads per accumulator row: each takes half of the tile's columns
 
 template <int BN, int CG> struct GemmCfg {
@@ -68,6 +78,9 @@ template <int BN>
 __device__ __forceinline__ int tile_cols(int n, int n0) { return min(BN, (n - n0 + 31) / 32 * 32); }
 
 struct SecondMaps { CUtensorMap a, b, o; };   // operands and output of the second VarlenK problem
+
+// What the scheduler queues: a linear tile index (past the last tile: the end) and what decode_unit found for it.
+struct __align__(16) TileEntry { int lin, m, n_tile, expert, row0, k_blocks, k_tail, prob; };
 
 struct TileCoord {
   int prob;        // VarlenK: 0 / 1 = first / second problem of the launch
@@ -94,38 +107,54 @@ __device__ __forceinline__ void band_decode(int band_m, int lin, int num_m, int 
   m_tile = m0 + (rem - n_tile * gm);
 }
 
-// `num_m`: live number of M units, i.e. row tiles (CG = 1) or pairs of row tiles (CG = 2); may come from device memory.
-// Ignored for VarlenK.  `half` = rank of this CTA in its pair (0 with CG = 1).
+// The unit with linear index `lin`, as it looks to both CTAs of a pair.  `num_m`: live number of M units, i.e. row tiles (CG = 1)
+// or pairs of row tiles (CG = 2); may come from device memory.  Ignored for VarlenK.  TileEntry::m: VarlenM with CG = 2 the
+// pair's first tile * 2 + (1 if it has a second one), VarlenK the unit, otherwise the row tile.
 template <int CG>
-__device__ __forceinline__ TileCoord decode_tile(const GemmParams& p, int lin, int num_m, int half) {
+__device__ __forceinline__ TileEntry decode_unit(const GemmParams& p, int lin, int num_m) {
+  TileEntry e;
+  e.lin = lin; e.prob = 0;
+  if (p.mode == kVarlenM) {
+    band_decode(p.band > 0 ? p.band / CG : kBandM / CG, lin, num_m, p.num_n_tiles, e.m, e.n_tile);
+    if (CG == 2) e.m = p.pair_tiles[e.m];
+    e.expert = p.tile_id_to_expert[CG == 2 ? e.m >> 1 : e.m];
+    e.row0 = 0;
+    e.k_blocks = (p.K + BK - 1) / BK;
+    e.k_tail = 0;
+  } else {
+    int nm = p.num_m_tiles, nn = p.num_n_tiles;
+    const int first = p.num_experts * nm * nn;
+    if (lin >= first) { e.prob = 1; lin -= first; nm = p.num_m_tiles2; nn = p.num_n_tiles2; }
+    const int per_e = nm * nn;
+    e.expert = lin / per_e;
+    band_decode(p.band > 0 ? p.band / CG : kBandM / CG, lin - e.expert * per_e, nm, nn, e.m, e.n_tile);
+    e.row0 = p.expert_pool_block_offset[e.expert] * BM;
+    const int len = p.expert_frequency[e.expert];
+    e.k_blocks = (len + BK - 1) / BK;
+    e.k_tail = len % BK;
+  }
+  return e;
+}
+// ... and to CTA `half` of the pair (0 with CG = 1).
+template <int CG>
+__device__ __forceinline__ TileCoord unit_coord(const GemmParams& p, const TileEntry& e, int half) {
   TileCoord t;
-  t.prob = 0;
+  t.prob = e.prob; t.n_tile = e.n_tile; t.expert = e.expert; t.k_blocks = e.k_blocks; t.k_tail = e.k_tail;
   t.rows_valid = true;
   if (p.mode == kVarlenM) {
-    band_decode(p.band > 0 ? p.band / CG : kBandM / CG, lin, num_m, p.num_n_tiles, t.m_tile, t.n_tile);
-    if (CG == 2) {
-      const int pair = p.pair_tiles[t.m_tile];       // first tile * 2 + (1 if the pair has a second tile)
-      t.m_tile = pair >> 1;
-      if (half != 0) { if (pair & 1) ++t.m_tile; else t.rows_valid = false; }   // no second tile: its loads repeat the first
-    }
-    t.expert = p.tile_id_to_expert[t.m_tile];
+    t.m_tile = CG == 2 ? e.m >> 1 : e.m;
+    if (CG == 2 && half != 0) { if (e.m & 1) ++t.m_tile; else t.rows_valid = false; }   // no second tile: its loads repeat the first
     t.row0 = t.m_tile * BM;
-    t.k_blocks = (p.K + BK - 1) / BK;
-    t.k_tail = 0;
   } else {
-    int nm = p.num_m_tiles, nn = p.num_n_tiles, m_out = p.M_out;
-    const int first = p.num_experts * nm * nn;
-    if (lin >= first) { t.prob = 1; lin -= first; nm = p.num_m_tiles2; nn = p.num_n_tiles2; m_out = p.M_out2; }
-    const int per_e = nm * nn;
-    t.expert = lin / per_e;
-    band_decode(p.band > 0 ? p.band / CG : kBandM / CG, lin - t.expert * per_e, nm, nn, t.m_tile, t.n_tile);
-    if (CG == 2) { t.m_tile = t.m_tile * 2 + half; t.rows_valid = t.m_tile * BM < m_out; }
-    t.row0 = p.expert_pool_block_offset[t.expert] * BM;
-    const int len = p.expert_frequency[t.expert];
-    t.k_blocks = (len + BK - 1) / BK;
-    t.k_tail = len % BK;
+    t.m_tile = e.m * CG + half;
+    if (CG == 2) t.rows_valid = t.m_tile * BM < (e.prob ? p.M_out2 : p.M_out);
+    t.row0 = e.row0;
   }
   return t;
+}
+template <int CG>
+__device__ __forceinline__ TileCoord decode_tile(const GemmParams& p, int lin, int num_m, int half) {
+  return unit_coord<CG>(p, decode_unit<CG>(p, lin, num_m), half);
 }
 
 __device__ __forceinline__ void st_global_v4(void* p, uint32_t a, uint32_t b, uint32_t c, uint32_t d) {
@@ -150,7 +179,7 @@ __device__ __forceinline__ bool epi_vote_any(bool pred) {
 }
 
 template <int BN, bool A_MN, bool B_MN, int EPI, bool PUSH, int CG>
-__global__ void __launch_bounds__((base_warps(EPI) + (PUSH ? push_warps(EPI) : 0)) * 32, 1)
+__global__ void __launch_bounds__((base_warps(EPI, A_MN) + (PUSH ? push_warps(EPI) : 0)) * 32, 1)
 grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b,
                     const __grid_constant__ CUtensorMap tmap_o0, const __grid_constant__ CUtensorMap tmap_o1,
                     const GemmParams p, const PushParams pp, const __grid_constant__ SecondMaps maps2) {
@@ -172,9 +201,9 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
   __shared__ int s_gates_open;   // how many of this CTA's tiles have an open gate (-1: the gate warp gave up)
   __shared__ int s_tiles_done;   // tiles whose epilogue finished (read by the time stamps only)
   __shared__ uint64_t s_push_bar[32][2];   // push-only CTAs: two bulk-load barriers per warp
-  __shared__ int s_q[kTileQueue];          // dynamic tile claim: claimed tile ids ...
-  __shared__ int s_q_head, s_q_tail;       // ... how many were claimed, how many the epilogue has finished
-  __shared__ int s_q_read;                 // ... how many entries the MMA warp has read
+  __shared__ TileEntry s_q[kTileQueue];    // the scheduler's queue ...
+  __shared__ int s_q_head, s_q_tail;       // ... how many tiles were queued, how many the epilogue has finished
+  __shared__ int s_q_read, s_q_prod;       // ... how many entries the MMA warp has read, how many the producer is (nearly) done with
   __shared__ int s_q_tail_peer, s_q_read_peer;   // (CG = 2, first CTA of a pair) the peer's epilogue / producer
   __shared__ char* s_remote_out[kMaxRanks];
   __shared__ float* s_remote_dw[kMaxRanks];
@@ -183,9 +212,10 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
   const int half_of_pair = CG == 2 ? static_cast<int>(cluster_ctarank()) : 0;   // the pair's first CTA issues its MMAs
   const bool leader = half_of_pair == 0;
   const int unit = static_cast<int>(blockIdx.x) / CG, num_units = static_cast<int>(gridDim.x) / CG;
-  // Tile feed.  Static: CTA b takes tiles b, b + stride, ...  Dynamic (VarlenK with a counter): the TMA thread claims
-  // the next tile and hands it to the MMA and epilogue warps through a small queue in shared memory.
-  const bool dyn = p.mode == kVarlenK && p.tile_counter != nullptr;
+  // Tile feed.  Static: CTA b takes tiles b, b + stride, ...  Dynamic (VarlenK with a counter): tiles are claimed.  VarlenK units are
+  // queued by the scheduler warp of the first CTA, in shared memory of both CTAs; otherwise every role decodes on its own.
+  constexpr bool queued = A_MN;
+  const bool dyn = queued && p.tile_counter != nullptr;
   const unsigned long long budget = p.wait_budget_ns;
   // Fused push, two ways of sharing the GPU.  Mixed (push_ctas == 0): every CTA multiplies and its extra warps push.
   // Dedicated (push_ctas > 0): the last push_ctas CTAs only push, with all their warps, and the others only multiply.
@@ -206,7 +236,7 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
     if (PUSH) s_push_ok = 1;
     s_gates_open = 0;
     s_tiles_done = 0;
-    s_q_head = 0; s_q_tail = 0; s_q_read = 0; s_q_tail_peer = 0; s_q_read_peer = 0;
+    s_q_head = 0; s_q_tail = 0; s_q_read = 0; s_q_prod = 0; s_q_tail_peer = 0; s_q_read_peer = 0;
     if (p.timing != nullptr) {
       long long* tm = p.timing + static_cast<size_t>(blockIdx.x) * kTimingCols;
       tm[0] = static_cast<long long>(globaltimer_ns());
@@ -227,7 +257,7 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
   const int total_tiles = p.mode == kVarlenM ? num_m * p.num_n_tiles
                                              : p.num_experts * (p.num_m_tiles * p.num_n_tiles + p.num_m_tiles2 * p.num_n_tiles2);
   if (PUSH) {
-    if ((pp.flags & 1) && !pp.static_targets && blockIdx.x == 0 && warp == base_warps(EPI) && lane < pp.num_ranks)
+    if ((pp.flags & 1) && !pp.static_targets && blockIdx.x == 0 && warp == base_warps(EPI, A_MN) && lane < pp.num_ranks)
       publish_record(pp.own, pp.peer_base, pp.ctl, pp.kind, pp.epoch, pp.rank, lane);
   }
   if ((EPI == kEpiScatter || EPI == kEpiDswiglu) && warp == 2 && lane < p.num_ranks) {
@@ -301,33 +331,21 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
     if (lane == 0) {
       int stage = 0; uint32_t phase = 0; int issued = 0; bool ok = true; int my_tile = 0;
       for (int it = 0; ok; ++it) {
+        TileCoord t;
         int lin;
-        if (dyn && leader) {
-          // claim the next tile; wait for a free queue entry first (every reader is at most kTileQueue tiles behind)
-          if (!spin_until([&] { return it - ld_acquire_cta_shared(&s_q_tail) < kTileQueue && it - ld_acquire_cta_shared(&s_q_read) < kTileQueue &&
-                                       (CG == 1 || (it - ld_acquire_cluster_shared(&s_q_tail_peer) < kTileQueue &&
-                                                    it - ld_acquire_cluster_shared(&s_q_read_peer) < kTileQueue)); }, budget, p.status)) {
-            report_failure(p.status, kStatusTimeoutPipeline, kKernelGemm, 4, p.rank, it, 0, 0);
-            ok = false;
-            lin = total_tiles;
-          } else {
-            lin = atomicAdd(p.tile_counter, 1);
-          }
-          s_q[it % kTileQueue] = lin;
-          st_release_cta_shared(&s_q_head, it + 1);
-          if (CG == 2) {       // the pair's second CTA works on the same unit: it gets a copy of the queue
-            st_cluster(cluster_map(&s_q[it % kTileQueue], 1), lin);
-            st_release_cluster(cluster_map(&s_q_head, 1), it + 1);
-          }
-        } else if (dyn) {
-          if (!spin_until([&] { return ld_acquire_cluster_shared(&s_q_head) > it; }, budget, p.status)) { ok = false; break; }
-          lin = s_q[it % kTileQueue];
-          st_release_cluster(cluster_map(&s_q_read_peer, 0), it + 1);
+        if constexpr (queued) {
+          if (!spin_until([&] { return (leader ? ld_acquire_cta_shared(&s_q_head) : ld_acquire_cluster_shared(&s_q_head)) > it; }, budget, p.status)) { ok = false; break; }
+          const TileEntry e = s_q[it % kTileQueue];
+          lin = e.lin;
+          t = unit_coord<CG>(p, e, half_of_pair);
+          if (lin >= total_tiles) break;
+          if (CG == 2 && !leader) st_cluster(cluster_map(&s_q_read_peer, 0), it + 1);
+          if (leader && t.k_blocks == 0) st_volatile_shared(&s_q_prod, it + 1);
         } else {
           lin = first_lin + it * lin_stride;
+          if (lin >= total_tiles || lin < 0) break;
+          t = decode_tile<CG>(p, lin, num_m, half_of_pair);
         }
-        if (lin >= total_tiles || lin < 0) break;
-        const TileCoord t = decode_tile<CG>(p, lin, num_m, half_of_pair);
         const int n0 = t.n_tile * BN;
         const int b0 = n0 + half_of_pair * (tile_cols<BN>(t.prob ? p.N2 : p.N, n0) / CG);   // first column of B this CTA loads
         const CUtensorMap* ta = t.prob ? &maps2.a : &tmap_a;
@@ -356,6 +374,7 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
           ++my_tile;
         }
         for (int kb = 0; kb < t.k_blocks; ++kb) {
+          if (queued && leader && kb == max(t.k_blocks - kClaimAhead, 0)) st_volatile_shared(&s_q_prod, it + 1);
           if (!mbar_wait(&empty_bar[stage], phase ^ 1, budget, p.status)) {
             report_failure(p.status, kStatusTimeoutPipeline, kKernelGemm, 0, p.rank, lin, kb, stage);
             ok = false; break;
@@ -418,17 +437,19 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
     auto tile_loop = [&](auto timed) {
     constexpr bool stamp = decltype(timed)::value;
     for (int it = 0; ok; ++it) {
-      int lin;
-      if (dyn) {
+      TileCoord t;
+      if constexpr (queued) {
         if (!__all_sync(0xffffffffu, spin_until([&] { return ld_acquire_cta_shared(&s_q_head) > it; }, budget, p.status))) { ok = false; break; }
-        lin = s_q[it % kTileQueue];
+        const TileEntry e = s_q[it % kTileQueue];
+        if (e.lin >= total_tiles) break;
         __syncwarp();
-        if (lane == 0) st_release_cta_shared(&s_q_read, it + 1);
+        if (lane == 0) st_volatile_shared(&s_q_read, it + 1);
+        t = unit_coord<CG>(p, e, 0);
       } else {
-        lin = first_lin + it * lin_stride;
+        const int lin = first_lin + it * lin_stride;
+        if (lin >= total_tiles || lin < 0) break;
+        t = decode_tile<CG>(p, lin, num_m, 0);
       }
-      if (lin >= total_tiles || lin < 0) break;
-      const TileCoord t = decode_tile<CG>(p, lin, num_m, 0);
       const uint32_t idesc = idesc0 | (static_cast<uint32_t>(tile_cols<BN>(t.prob ? p.N2 : p.N, t.n_tile * BN) >> 3) << 17);
       if (t.k_blocks == 0) continue;   // empty expert: the epilogue writes zeros on its own
       // all 32 lanes wait; the outcome is made warp-uniform so that no lane leaves ahead of elect_one / __syncwarp
@@ -498,20 +519,23 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
     constexpr int kChunksPerHalf = BN / 64;
     const uint32_t stg = smem_u32(epi_stage + (warp - 2) * Cfg::kEpiStageBytes);
     int acc = 0; uint32_t acc_phase = 0;
-    uint32_t store_buf = 0;       // (store epilogue) half of the staging tile the next chunk goes through
     for (int it = 0;; ++it) {
       int lin;
-      if (dyn) {
+      TileCoord t;
+      if constexpr (queued) {
         // every epilogue thread reads the queue itself; the give-up decision is taken together (see below)
-        const bool got = spin_until([&] { return (CG == 2 ? ld_acquire_cluster_shared(&s_q_head) : ld_acquire_cta_shared(&s_q_head)) > it; },
+        const bool got = spin_until([&] { return (leader ? ld_acquire_cta_shared(&s_q_head) : ld_acquire_cluster_shared(&s_q_head)) > it; },
                                     budget, p.status);
         if (epi_vote_any(!got)) break;
-        lin = s_q[it % kTileQueue];
+        const TileEntry e = s_q[it % kTileQueue];
+        lin = e.lin;
+        if (lin >= total_tiles) break;
+        t = unit_coord<CG>(p, e, half_of_pair);
       } else {
         lin = first_lin + it * lin_stride;
+        if (lin >= total_tiles || lin < 0) break;
+        t = decode_tile<CG>(p, lin, num_m, half_of_pair);
       }
-      if (lin >= total_tiles || lin < 0) break;
-      const TileCoord t = decode_tile<CG>(p, lin, num_m, half_of_pair);
       const CUtensorMap* to0 = t.prob ? &maps2.o : &tmap_o0;
       // output width of this tile's problem (0: this CTA's half of the pair has no rows)
       const int prob_n = !t.rows_valid ? 0 : t.prob ? p.N2 : p.N;
@@ -617,9 +641,13 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
             for (int i = 0; i < (EPI == kEpiDswiglu ? 1 : 32); ++i) r[i] = 0;
           }
         }
-        if (EPI == kEpiStore) {          // two halves of the staging tile in turn: the store before last has read its own
-          if (lane == 0) bulk_wait_read_but_one();
-          __syncwarp();
+        // Two chunks side by side leave as one store of 128-byte rows: half the rows for the TMA unit of stores of 32 columns each,
+        // two of which fitted the staging tile (weight gradients as above 323 -> 311 and 3775 -> 3705 thousand cycles).
+        if (EPI == kEpiStore) {
+          if (((c - c_begin) & 1) == 0) {
+            if (lane == 0) bulk_wait_read();
+            __syncwarp();
+          }
         } else if (EPI == kEpiSwiglu) {
           // The staging tile is reused by every chunk: the previous chunk's bulk store must have read it.
           // Waiting here, after the accumulator fetch, instead of right after the store was issued lets the
@@ -628,17 +656,19 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
           __syncwarp();
         }
         if (EPI == kEpiStore) {
+          const int hpos = (c - c_begin) & 1;
 #pragma unroll
           for (int q = 0; q < 4; ++q)
-            st_shared_v4(stg + store_buf + stage_off<64>(lane, q),
+            st_shared_v4(stg + stage_off<128>(lane, hpos * 4 + q),
                          pack_bf16x2(__uint_as_float(r[q * 8 + 0]), __uint_as_float(r[q * 8 + 1])),
                          pack_bf16x2(__uint_as_float(r[q * 8 + 2]), __uint_as_float(r[q * 8 + 3])),
                          pack_bf16x2(__uint_as_float(r[q * 8 + 4]), __uint_as_float(r[q * 8 + 5])),
                          pack_bf16x2(__uint_as_float(r[q * 8 + 6]), __uint_as_float(r[q * 8 + 7])));
-          fence_proxy_async_smem();
-          __syncwarp();
-          if (lane == 0) { tma_store_3d(to0, epi_stage + (warp - 2) * Cfg::kEpiStageBytes + store_buf, n, warp_row0, zc); bulk_commit(); }
-          store_buf ^= 2048;
+          if (hpos == 1 || n + 32 >= prob_n || c + 1 == c_begin + kChunksPerHalf) {    // (columns past the last are clipped)
+            fence_proxy_async_smem();
+            __syncwarp();
+            if (lane == 0) { tma_store_3d(to0, epi_stage + (warp - 2) * Cfg::kEpiStageBytes, n - hpos * 32, warp_row0, zc); bulk_commit(); }
+          }
         } else if (EPI == kEpiSwiglu) {
           // columns (2i, 2i+1) = (gate_i, up_i); preact tile at +0 (64-byte rows), postact tile at +2048 (32-byte rows)
           if (p.out1 != nullptr) {
@@ -799,7 +829,7 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
       if (!given_back) give_back();       // (no column of this tile is this warp's)
       if (!empty) { acc ^= 1; if (acc == 0) acc_phase ^= 1; }
       if (p.timing != nullptr && epi_tid == 0) *reinterpret_cast<volatile int*>(&s_tiles_done) += 1;
-      if (dyn) {                    // this queue entry may be reused once every epilogue thread is done with the tile
+      if constexpr (queued) {      // this queue entry may be reused once every epilogue thread is done with the tile
         epi_bar_sync();
         if (epi_tid == 0) {
           if (CG == 2 && !leader) st_release_cluster(cluster_map(&s_q_tail_peer, 0), it + 1);
@@ -838,9 +868,38 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
     }
     if (lane == 0) bulk_wait_all();     // every bulk store this warp issued has been performed
     if (p.tail.enabled) __threadfence_system();
-  } else if (has_gate_warp(EPI) && warp == kGemmWarps) {
-    // ------------------------------------------------------------------ gate warp: polls tile gates ahead of the producer
-    if (lane == 0 && p.mode == kVarlenM && p.arrival_count != nullptr) {
+  } else if (warp == kGemmWarps) {
+    if constexpr (queued) {
+      // ------------------------------------------------------------------ scheduler: tiles into the queue of both CTAs
+      if (leader && lane == 0) {
+        for (int it = 0;; ++it) {
+          // A free entry: every role of both CTAs is done with what it held.  And not too early (kClaimAhead).
+          const bool ok = spin_until([&] {
+            if (it > ld_acquire_cta_shared(&s_q_prod)) { __nanosleep(128); return false; }      // (seldom: polls take issue slots)
+            return it - ld_acquire_cta_shared(&s_q_read) < kTileQueue && it - ld_acquire_cta_shared(&s_q_tail) < kTileQueue &&
+                   (CG == 1 || (it - ld_acquire_cluster_shared(&s_q_read_peer) < kTileQueue && it - ld_acquire_cluster_shared(&s_q_tail_peer) < kTileQueue));
+          }, budget, p.status);
+          int lin = total_tiles;
+          if (!ok) report_failure(p.status, kStatusTimeoutPipeline, kKernelGemm, 4, p.rank, it, 0, 0);
+          else lin = dyn ? atomicAdd(p.tile_counter, 1) : first_lin + it * lin_stride;
+          const bool end = lin >= total_tiles || lin < 0;
+          TileEntry e{};
+          if (end) e.lin = total_tiles;
+          else e = decode_unit<CG>(p, lin, num_m);
+          TileEntry* q = &s_q[it % kTileQueue];
+          *q = e;
+          st_release_cta_shared(&s_q_head, it + 1);
+          if (CG == 2) {
+            const uint32_t peer = cluster_map(q, 1);
+            st_cluster_v4(peer, e.lin, e.m, e.n_tile, e.expert);
+            st_cluster_v4(peer + 16, e.row0, e.k_blocks, e.k_tail, e.prob);
+            st_release_cluster(cluster_map(&s_q_head, 1), it + 1);
+          }
+          if (end) break;
+        }
+      }
+    } else if (has_gate_warp(EPI) && lane == 0 && p.mode == kVarlenM && p.arrival_count != nullptr) {
+      // ------------------------------------------------------------------ gate warp: polls tile gates ahead of the producer
       const bool local_only = p.num_ranks == 1;   // every writer of the counters is on this GPU: device scope is enough
       int n = 0;
       for (int lin = first_lin; lin < total_tiles; lin += lin_stride) {
@@ -866,7 +925,7 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
     // this rank: local copies drain fast and do not back up the load/store path)
     const bool local_walker = num_push_ctas > 0 && pp.split_local && pp.work_counter_local != nullptr;
     if ((pp.flags & 2) && (num_push_ctas == 0 || local_walker)) {
-      const int pw = warp - base_warps(EPI);
+      const int pw = warp - base_warps(EPI, A_MN);
       if (pw == 0 && lane < pp.num_ranks) {
         const unsigned long long* rec = pp.static_targets
             ? reinterpret_cast<const unsigned long long*>(&pp.own)
@@ -958,7 +1017,7 @@ cudaError_t launch_instance(const GemmParams& p, const LaunchMaps& m, const Push
   }
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = dim3(static_cast<unsigned>((num_ctas + CG - 1) / CG * CG));
-  cfg.blockDim = dim3((base_warps(EPI) + (PUSH ? push_warps(EPI) : 0)) * 32);
+  cfg.blockDim = dim3((base_warps(EPI, A_MN) + (PUSH ? push_warps(EPI) : 0)) * 32);
   cfg.dynamicSmemBytes = smem;
   cfg.stream = stream;
   cudaLaunchAttribute attr[2];

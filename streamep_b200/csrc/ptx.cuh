@@ -216,6 +216,10 @@ __device__ __forceinline__ bool mbar_try_wait_cluster(uint64_t* bar, uint32_t pa
       : "=r"(ok) : "r"(smem_u32(bar)), "r"(parity) : "memory");
   return ok != 0;
 }
+// A progress counter that other warps poll; orders nothing (a release would make this thread wait for all it has in flight).
+__device__ __forceinline__ void st_volatile_shared(int* p, int v) {
+  asm volatile("st.volatile.shared::cta.s32 [%0], %1;" :: "r"(smem_u32(p)), "r"(v) : "memory");
+}
 // Bounded mbarrier wait: returns false when the budget ran out or another wait already failed.
 template <bool kCluster = false>
 __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, unsigned long long budget_ns,
@@ -255,6 +259,9 @@ __device__ __forceinline__ void mbar_arrive_cluster(uint32_t cluster_addr) {
 }
 __device__ __forceinline__ void st_cluster(uint32_t cluster_addr, int v) {
   asm volatile("st.relaxed.cluster.shared::cluster.s32 [%0], %1;" :: "r"(cluster_addr), "r"(v) : "memory");
+}
+__device__ __forceinline__ void st_cluster_v4(uint32_t cluster_addr, int a, int b, int c, int d) {
+  asm volatile("st.shared::cluster.v4.b32 [%0], {%1, %2, %3, %4};" :: "r"(cluster_addr), "r"(a), "r"(b), "r"(c), "r"(d) : "memory");
 }
 __device__ __forceinline__ void st_release_cluster(uint32_t cluster_addr, int v) {
   asm volatile("st.release.cluster.shared::cluster.s32 [%0], %1;" :: "r"(cluster_addr), "r"(v) : "memory");
@@ -316,8 +323,6 @@ __device__ __forceinline__ void tma_store_3d(const void* tmap, const void* smem_
 __device__ __forceinline__ void bulk_commit() { asm volatile("cp.async.bulk.commit_group;" ::: "memory"); }
 // the source shared memory of all committed groups has been read (it may be overwritten)
 __device__ __forceinline__ void bulk_wait_read() { asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory"); }
-// ... of all but the last committed group
-__device__ __forceinline__ void bulk_wait_read_but_one() { asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory"); }
 // all committed groups are complete (their global writes are performed)
 __device__ __forceinline__ void bulk_wait_all() { asm volatile("cp.async.bulk.wait_group 0;" ::: "memory"); }
 

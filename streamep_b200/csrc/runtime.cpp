@@ -1378,10 +1378,10 @@ class Runtime : public std::enable_shared_from_this<Runtime> {
       return make_tmap(t.data_ptr(), cols, rows, experts, ld, experts > 1 ? t.stride(0) : rows * ld, box_cols, 32, sw);
     };
     if (a.epilogue == kEpiStore) {
-      if (a.mode == kVarlenM) to0 = out_map(*a.out0, p.N, p.total_rows, 1, 32, CU_TENSOR_MAP_SWIZZLE_64B);
-      else to0 = out_map(*a.out0, p.N, p.M_out, p.num_experts, 32, CU_TENSOR_MAP_SWIZZLE_64B);
+      if (a.mode == kVarlenM) to0 = out_map(*a.out0, p.N, p.total_rows, 1, 64, CU_TENSOR_MAP_SWIZZLE_128B);
+      else to0 = out_map(*a.out0, p.N, p.M_out, p.num_experts, 64, CU_TENSOR_MAP_SWIZZLE_128B);
       have_o0 = true;
-      if (have_maps2) maps2[2] = out_map(*a.out2, p.N2, p.M_out2, p.num_experts, 32, CU_TENSOR_MAP_SWIZZLE_64B);
+      if (have_maps2) maps2[2] = out_map(*a.out2, p.N2, p.M_out2, p.num_experts, 64, CU_TENSOR_MAP_SWIZZLE_128B);
     } else if (a.epilogue == kEpiSwiglu) {
       SEP_ASSERT(p.N % 16 == 0, "SwiGLU epilogue needs an output width that is a multiple of 16");
       to0 = out_map(*a.out0, p.N / 2, p.total_rows, 1, 16, CU_TENSOR_MAP_SWIZZLE_32B); have_o0 = true;
@@ -1714,7 +1714,7 @@ class Runtime : public std::enable_shared_from_this<Runtime> {
         preact = at::empty({R, 2 * I}, opts);
         LocalGemm r(*this, st, kEpiStore, st.width(cfg.tile_n_a, 2 * I, num_sms()));
         r.operands(pool, st.w1, false);
-        r.output0(preact, 32, CU_TENSOR_MAP_SWIZZLE_64B);
+        r.output0(preact, 64, CU_TENSOR_MAP_SWIZZLE_128B);
         r.launch(0, 5);
       }
       at::Tensor dswiglu_in = at::empty({R, 2 * I}, opts), postact_dw2 = at::empty({R, I}, opts);
@@ -1793,13 +1793,13 @@ class Runtime : public std::enable_shared_from_this<Runtime> {
       p.band = tile_band(static_cast<int64_t>(st.tokens) * st.topk / std::max<int64_t>(E, 1), std::max(N, out2 ? b2.size(1) : N));
       ta = make_tmap(a.data_ptr(), M, rows, 1, M, rows * M, 64, 64);
       tb = make_tmap(b.data_ptr(), N, rows, 1, N, rows * N, 64, 64);
-      to0 = make_tmap(out.data_ptr(), N, M, E, N, M * N, 32, 32, CU_TENSOR_MAP_SWIZZLE_64B); have_o0 = true;
+      to0 = make_tmap(out.data_ptr(), N, M, E, N, M * N, 64, 32, CU_TENSOR_MAP_SWIZZLE_128B); have_o0 = true;
       if (out2) {
         const int64_t N2 = b2.size(1);
         p.N2 = N2; p.M_out2 = M2; p.num_m_tiles2 = units(M2, unit_m); p.num_n_tiles2 = (N2 + p.block_n - 1) / p.block_n;
         second[0] = make_tmap(a2.data_ptr(), M2, rows, 1, M2, rows * M2, 64, 64);
         second[1] = make_tmap(b2.data_ptr(), N2, rows, 1, N2, rows * N2, 64, 64);
-        second[2] = make_tmap(out2->data_ptr(), N2, M2, E, N2, M2 * N2, 32, 32, CU_TENSOR_MAP_SWIZZLE_64B);
+        second[2] = make_tmap(out2->data_ptr(), N2, M2, E, N2, M2 * N2, 64, 32, CU_TENSOR_MAP_SWIZZLE_128B);
         have_second = true;
       }
       p.tile_counter = st.sizes + 4;     // the layer's own: two layers of a buffer may run on different streams
