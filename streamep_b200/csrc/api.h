@@ -181,7 +181,7 @@ struct PushParams {
   StatusBlock* status;
   unsigned long long wait_budget_ns;
 };
-void launch_dispatch_push(const PushParams& p, int num_blocks, cudaStream_t stream);
+cudaError_t launch_dispatch_push(const PushParams& p, int num_blocks, cudaStream_t stream);
 
 // ---------------------------------------------------------------------------------------------
 // Dispatch of a single rank (local_kernels.cu): slots by a counting sort, rows copied into the pool, no exchange

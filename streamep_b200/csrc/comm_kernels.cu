@@ -9,6 +9,7 @@
 // counter.  Reference counterparts: csrc/kernels/intranode.cu:124-440 (metadata), :551-599 (tile
 // fill), :601-1106 (dispatch), :1161-1439 (dispatch_grads), :1505-1880 (combine),
 // csrc/kernels/runtime.cu:18-31 (barrier).
+#include <atomic>
 #include <cstdio>
 
 #include "comm_common.cuh"
@@ -613,7 +614,7 @@ __global__ void __launch_bounds__(kPushThreads, 1) dispatch_push_kernel(const Pu
 // The push of a single rank: every pair of a token lands in this rank's pool, so a warp takes whole tokens, reads each row
 // once and stores it once per pair, where the general kernel reads a row per pair.  Bound by the pool's writes to HBM; the
 // caller's SM budget (80 blocks by default) asks for as many bytes in flight per SM as it can hold: 32 warps, 4 KB each.
-// 4096 tokens x 8 pairs, hidden 7168, 80 blocks: 173 -> 135 us.  Chunks of tokens are claimed, not dealt out by block: a
+// 4096 tokens x 8 pairs, hidden 512, 80 blocks: 23 us.  Chunks of tokens are claimed, not dealt out by block: a
 // block needs a whole SM, and a consumer that already waits for rows may hold the SM of a block that has not started yet.
 constexpr int kLocalPushThreads = 1024;
 constexpr int kLocalPushPairs = 16;     // pairs a warp copies between two releases of their tiles
@@ -673,9 +674,143 @@ __global__ void __launch_bounds__(kLocalPushThreads, 1) dispatch_push_local_kern
   }
 }
 
-void launch_dispatch_push(const PushParams& p, int num_blocks, cudaStream_t stream) {
+// The same push for rows of kBulkPushRow bytes and more, through the bulk-copy engine: a warp brings a chunk (whole tokens, or a
+// piece of a token whose row is longer) to shared memory and every pair leaves from there as one bulk store.  No register
+// holds a row, so the six warps of a block keep up to 2 x 16 KB each in flight where the loads and stores of 32 warps kept 4 KB.
+// Bound by the pool's writes to HBM once there are enough tokens, and by latency below.  us on 80 blocks, before -> now: hidden 7168,
+// top-8, 4096 tokens 138 -> 121 (4.4 TB/s), 16384 tokens 468 -> 437, 1000 tokens 82 -> 39; top-2, 1000 tokens 72 -> 19; hidden 2048,
+// top-8, 4096 tokens 49 -> 46; hidden 1024, top-8 32 -> 31.  Shorter rows mean too many bulk stores: hidden 512, top-8, 16384 tokens 49
+// -> 55, 4096 tokens 23 -> 25; 256 35 -> 39, so those keep the kernel above.
+constexpr int kBulkPushRow = 2048;      // bytes
+constexpr int kBulkPushWarps = 6;
+constexpr int kBulkPushSlot = 16384;
+
+__global__ void __launch_bounds__(kBulkPushWarps * 32, 1) dispatch_push_local_bulk_kernel(const PushParams p) {
+  extern __shared__ __align__(128) unsigned char s_slots[];       // [warps][2][kBulkPushSlot]
+  __shared__ PushTargets tg;
+  __shared__ uint64_t s_bar[kBulkPushWarps][2];
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, K = p.num_topk;
+  if (blockIdx.x == 0 && tid == 0 && p.started_flag != nullptr) atomicAdd(p.started_flag, 1);
+  if ((p.flags & 1) && !p.static_targets && blockIdx.x == 0 && tid == 0)
+    publish_record(p.own, p.peer_base, p.ctl, p.kind, p.epoch, p.rank, 0);
+  if (tid == 0) resolve_push_targets(tg, 0, p.peer_base[0], reinterpret_cast<const unsigned long long*>(&p.own));
+  if (lane == 0) { mbar_init(&s_bar[warp][0], 1); mbar_init(&s_bar[warp][1], 1); mbar_fence_init(); }
+  __syncthreads();
+  if (!(p.flags & 2) || *p.num_send <= 0) return;       // (no pair, or the metadata kernel gave up)
+  const uint32_t row_bytes = static_cast<uint32_t>(p.hidden) * 2;
+  const int chunk = max(1, min(static_cast<int>(kBulkPushSlot / row_bytes), 32 / K));      // tokens: a lane for every pair
+  const int pieces = static_cast<int>((row_bytes + kBulkPushSlot - 1) / kBulkPushSlot);    // (more than 1: chunk is 1)
+  const uint32_t slot_smem = smem_u32(s_slots) + warp * 2 * kBulkPushSlot;
+  const char* x = static_cast<const char*>(p.x);
+  const int num_chunks = (p.num_tokens + chunk - 1) / chunk;
+  auto claim = [&] {
+    int c = 0;
+    if (lane == 0) c = atomicAdd(p.work_counter, 1);
+    return __shfl_sync(0xffffffffu, c, 0);
+  };
+  // item = (chunk, piece); bytes of it and where they start in x
+  auto load = [&](int c, int piece, int s) {
+    if (lane != 0) return;
+    const int t0 = c * chunk, n = min(chunk, p.num_tokens - t0);
+    const uint32_t off = static_cast<uint32_t>(piece) * kBulkPushSlot;
+    const uint32_t bytes = pieces > 1 ? min(static_cast<uint32_t>(kBulkPushSlot), row_bytes - off) : n * row_bytes;
+    mbar_arrive_expect_tx(&s_bar[warp][s], bytes);
+    bulk_load_1d(slot_smem + s * kBulkPushSlot, x + static_cast<size_t>(t0) * row_bytes + off, bytes, &s_bar[warp][s]);
+  };
+  // one add per pair, by the lane that stored it (same GPU: device scope)
+  auto release = [&](int slot) {
+    fence_proxy_async();            // the stores of this thread's pairs have been performed: order them before the release
+    __syncwarp();
+    if (slot >= 0) red_release_gpu_add(tg.arrival_count[0] + slot / p.tile_m, 1);
+  };
+  __nanosleep(warp * 256);          // the first chunks of a short call go to different blocks
+  int c = claim(), piece = 0, s = 0;
+  uint32_t phase[2] = {0, 0};
+  int done_slot = -1;               // this lane's pair of the chunk before, stored but not released yet
+  bool ok = true;
+  if (c < num_chunks) load(c, 0, 0);
+  while (c < num_chunks) {
+    const int t0 = c * chunk, n = min(chunk, p.num_tokens - t0) * K;
+    const int slot = lane < n ? p.pair_slot[static_cast<size_t>(t0) * K + lane] : -1;
+    const int t = t0 + lane / K, k = lane - (lane / K) * K;
+    if (!__all_sync(0xffffffffu, mbar_wait(&s_bar[warp][s], phase[s], p.wait_budget_ns, p.status))) { ok = false; break; }
+    phase[s] ^= 1;
+    const uint32_t off = static_cast<uint32_t>(piece) * kBulkPushSlot;
+    const uint32_t bytes = pieces > 1 ? min(static_cast<uint32_t>(kBulkPushSlot), row_bytes - off) : row_bytes;
+    if (slot >= 0) bulk_store_1d(tg.pool[0] + static_cast<size_t>(slot) * row_bytes + off, slot_smem + s * kBulkPushSlot + (lane / K) * row_bytes, bytes);
+    bulk_commit();
+    if (piece == 0 && !p.is_grads) {
+      const unsigned pairs = __ballot_sync(0xffffffffu, slot >= 0);
+      const unsigned mine = lane < n ? (pairs >> (lane - k)) & (K == 32 ? 0xffffffffu : (1u << K) - 1u) : 0;      // pairs of this lane's token
+      if (mine != 0) {
+        const int r = p.send_recv_token[t];
+        if (slot >= 0) {
+          tg.pool_topk_weight[0][slot] = p.topk_weights[static_cast<size_t>(t) * K + k];
+          tg.pool_recv_token[0][slot] = r;
+          tg.pool_k_slot[0][slot] = k;
+          tg.pool_src[0][slot] = make_int2(p.rank, t);
+          tg.recv_token_to_slots[0][static_cast<size_t>(r) * K + k] = slot;     // skipped k stay -1
+        }
+        if (k == 0) {
+          tg.k_local_total[0][r] = __popc(mine);
+          tg.k_local_remaining[0][r] = __popc(mine);
+          tg.recv_src[0][r] = make_int2(p.rank, t);
+        }
+      }
+    }
+    // the next item goes into the other half once the stores from there have read it
+    const bool last_piece = piece + 1 == pieces;
+    const int next_c = last_piece ? claim() : c, next_piece = last_piece ? 0 : piece + 1;
+    bulk_wait_read_but_one();
+    __syncwarp();
+    if (next_c < num_chunks) load(next_c, next_piece, s ^ 1);
+    if (piece == 0) {               // all stores but those of this item have been performed: the chunk before is complete
+      bulk_wait_all_but_one();
+      release(done_slot);
+    }
+    if (last_piece) done_slot = slot; else done_slot = -1;
+    c = next_c; piece = next_piece; s ^= 1;
+  }
+  if (ok) {
+    bulk_wait_all();
+    release(done_slot);
+  } else if (lane == 0) {           // give up: report, let a load in flight land (bounded); the chunk's tiles are not released
+    report_failure(p.status, kStatusTimeoutPipeline, p.is_grads ? kKernelDispatchGrads : kKernelDispatch, 3, p.rank, c, 0, 0);
+    const unsigned long long t0 = globaltimer_ns();
+    while (!mbar_try_wait(&s_bar[warp][s], phase[s]) && globaltimer_ns() - t0 < 2000000ull) {}
+  }
+  bulk_wait_all();
+  __syncthreads();
+  if (tid == 0) {
+    __threadfence();
+    if (atomicAdd(p.blocks_done, 1) == static_cast<int>(gridDim.x) - 1) {   // last block resets the counters for another push
+      *p.work_counter = 0;
+      *p.blocks_done = 0;
+    }
+  }
+}
+
+static cudaError_t launch_push_local_bulk(const PushParams& p, int num_blocks, cudaStream_t stream) {
+  constexpr int smem = kBulkPushWarps * 2 * kBulkPushSlot;
+  static std::atomic<bool> configured[64];      // the shared-memory limit is an attribute of the function on a device
+  int dev = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e != cudaSuccess) return e;
+  if (dev < 0 || dev >= 64) return cudaErrorInvalidDevice;
+  if (!configured[dev].load(std::memory_order_acquire)) {
+    e = cudaFuncSetAttribute(dispatch_push_local_bulk_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    if (e != cudaSuccess) return e;
+    configured[dev].store(true, std::memory_order_release);
+  }
+  dispatch_push_local_bulk_kernel<<<num_blocks, kBulkPushWarps * 32, smem, stream>>>(p);
+  return cudaGetLastError();
+}
+
+cudaError_t launch_dispatch_push(const PushParams& p, int num_blocks, cudaStream_t stream) {
+  if (p.num_ranks == 1 && p.hidden * 2 >= kBulkPushRow) return launch_push_local_bulk(p, num_blocks, stream);
   if (p.num_ranks == 1) dispatch_push_local_kernel<<<num_blocks, kLocalPushThreads, 0, stream>>>(p);
   else dispatch_push_kernel<<<num_blocks, kPushThreads, 0, stream>>>(p);
+  return cudaGetLastError();
 }
 
 // =============================================================================================
@@ -683,8 +818,8 @@ void launch_dispatch_push(const PushParams& p, int num_blocks, cudaStream_t stre
 // =============================================================================================
 // 16-byte loads in flight per lane and contributing rank, and threads of a block: one rank alone has no round trip over
 // NVLink to hide behind the other ranks' loads, so it takes a row in larger pieces and twice the warps (the caller's SM
-// budget sets the blocks).  4096 tokens, hidden 7168, 80 blocks, one rank: 84 -> 39 us.
-constexpr int pull_unroll(int ranks) { return ranks == 1 ? 4 : 2; }
+// budget sets the blocks).  4096 tokens, hidden 7168, 80 blocks, one rank: 84 -> 34 us.
+constexpr int pull_unroll(int ranks) { return ranks == 1 ? 8 : 2; }
 constexpr int combine_threads(int ranks) { return ranks == 1 ? 1024 : 512; }
 
 template <int NR>      // 1, or kMaxRanks for any number

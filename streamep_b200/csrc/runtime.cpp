@@ -1111,7 +1111,7 @@ class Runtime : public std::enable_shared_from_this<Runtime> {
     PushParams p = make_push_params(*st, st->x, false, st->record, kKindDispatch, st->push_epoch, flags,
                                     st->pool_arrival_count.data_ptr<int>(), 2);
     if (flags & 2) ++gate_issued_[0];
-    ++launches_; launch_dispatch_push(p, num_blocks, stream());
+    ++launches_; SEP_CUDA_CHECK(launch_dispatch_push(p, num_blocks, stream()));
     SEP_CUDA_CHECK(cudaGetLastError());
   }
 
@@ -1171,7 +1171,7 @@ class Runtime : public std::enable_shared_from_this<Runtime> {
     PushParams p = make_push_params(*st, rows, true, g->record, kKindDispatchGrads, g->epoch, flags,
                                     g->bwd_dispatch_arrival_count.data_ptr<int>(), 4);
     if (flags & 2) ++gate_issued_[1];
-    ++launches_; launch_dispatch_push(p, num_blocks, stream());
+    ++launches_; SEP_CUDA_CHECK(launch_dispatch_push(p, num_blocks, stream()));
     SEP_CUDA_CHECK(cudaGetLastError());
   }
 
@@ -1430,13 +1430,13 @@ class Runtime : public std::enable_shared_from_this<Runtime> {
       PushParams pp = make_push_params(*a.fused_push, a.fused_push->x, false, a.fused_push->record, kKindDispatch,
                                        a.fused_push->push_epoch, a.push_flags & 3, a.fused_push->pool_arrival_count.data_ptr<int>(), 2);
       pp.started_flag = nullptr;
-      ++launches_; launch_dispatch_push(pp, num_sms(), stream);
+      ++launches_; SEP_CUDA_CHECK(launch_dispatch_push(pp, num_sms(), stream));
     } else if (a.fused_push_grads) {
       const at::Tensor push_rows = aligned_rows(a.fused_push_rows);
       PushParams pp = make_push_params(*a.fused_push_routing, push_rows, true, a.fused_push_grads->record, kKindDispatchGrads,
                                        a.fused_push_grads->epoch, a.push_flags & 3, a.fused_push_grads->bwd_dispatch_arrival_count.data_ptr<int>(), 4);
       pp.started_flag = nullptr;
-      ++launches_; launch_dispatch_push(pp, num_sms(), stream);
+      ++launches_; SEP_CUDA_CHECK(launch_dispatch_push(pp, num_sms(), stream));
     }
     if (a.tail) {
       BarrierParams b{};

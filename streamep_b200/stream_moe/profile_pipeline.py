@@ -27,6 +27,7 @@ KERNELS = {  # kernel function -> logical name
     "fill_tile_metadata_kernel": "tile fill",
     "dispatch_push_kernel": "dispatch / dispatch_grads (stand-alone push)",
     "dispatch_push_local_kernel": "dispatch / dispatch_grads (stand-alone push)",
+    "dispatch_push_local_bulk_kernel": "dispatch / dispatch_grads (stand-alone push)",
     "combine_pull_kernel": "combine / combine_grads (stand-alone pull)",
     "combine_reduce_kernel": "combine of landed rows",
     "local_count_kernel": "single-rank dispatch (sort, rows into the pool)",
