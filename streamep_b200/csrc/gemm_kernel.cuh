@@ -79,8 +79,8 @@ __device__ __forceinline__ int tile_cols(int n, int n0) { return min(BN, (n - n0
 
 struct SecondMaps { CUtensorMap a, b, o; };   // operands and output of the second VarlenK problem
 
-// What the scheduler queues: a linear tile index (past the last tile: the end) and what decode_unit found for it.
-struct __align__(16) TileEntry { int lin, m, n_tile, expert, row0, k_blocks, k_tail, prob; };
+// What the scheduler queues: a linear tile index (past the last tile: the end) and what decode_tile found for it.
+struct __align__(16) TileEntry { int lin, m_tile, n_tile, expert, row0, k_blocks, k_tail, prob; };
 
 struct TileCoord {
   int prob;        // VarlenK: 0 / 1 = first / second problem of the launch
@@ -107,54 +107,50 @@ __device__ __forceinline__ void band_decode(int band_m, int lin, int num_m, int 
   m_tile = m0 + (rem - n_tile * gm);
 }
 
-// The unit with linear index `lin`, as it looks to both CTAs of a pair.  `num_m`: live number of M units, i.e. row tiles (CG = 1)
-// or pairs of row tiles (CG = 2); may come from device memory.  Ignored for VarlenK.  TileEntry::m: VarlenM with CG = 2 the
-// pair's first tile * 2 + (1 if it has a second one), VarlenK the unit, otherwise the row tile.
+// `num_m`: live number of M units, i.e. row tiles (CG = 1) or pairs of row tiles (CG = 2); may come from device memory.
+// Ignored for VarlenK.  `half` = rank of this CTA in its pair (0 with CG = 1).  The kernels over row tiles decode in every role,
+// straight into the coordinates: by way of a TileEntry the six instances with a fused push spilled 8 to 20 bytes a thread
+// instead of 0 to 12.
 template <int CG>
-__device__ __forceinline__ TileEntry decode_unit(const GemmParams& p, int lin, int num_m) {
-  TileEntry e;
-  e.lin = lin; e.prob = 0;
-  if (p.mode == kVarlenM) {
-    band_decode(p.band > 0 ? p.band / CG : kBandM / CG, lin, num_m, p.num_n_tiles, e.m, e.n_tile);
-    if (CG == 2) e.m = p.pair_tiles[e.m];
-    e.expert = p.tile_id_to_expert[CG == 2 ? e.m >> 1 : e.m];
-    e.row0 = 0;
-    e.k_blocks = (p.K + BK - 1) / BK;
-    e.k_tail = 0;
-  } else {
-    int nm = p.num_m_tiles, nn = p.num_n_tiles;
-    const int first = p.num_experts * nm * nn;
-    if (lin >= first) { e.prob = 1; lin -= first; nm = p.num_m_tiles2; nn = p.num_n_tiles2; }
-    const int per_e = nm * nn;
-    e.expert = lin / per_e;
-    band_decode(p.band > 0 ? p.band / CG : kBandM / CG, lin - e.expert * per_e, nm, nn, e.m, e.n_tile);
-    e.row0 = p.expert_pool_block_offset[e.expert] * BM;
-    const int len = p.expert_frequency[e.expert];
-    e.k_blocks = (len + BK - 1) / BK;
-    e.k_tail = len % BK;
-  }
-  return e;
-}
-// ... and to CTA `half` of the pair (0 with CG = 1).
-template <int CG>
-__device__ __forceinline__ TileCoord unit_coord(const GemmParams& p, const TileEntry& e, int half) {
+__device__ __forceinline__ TileCoord decode_tile(const GemmParams& p, int lin, int num_m, int half) {
   TileCoord t;
-  t.prob = e.prob; t.n_tile = e.n_tile; t.expert = e.expert; t.k_blocks = e.k_blocks; t.k_tail = e.k_tail;
+  t.prob = 0;
   t.rows_valid = true;
   if (p.mode == kVarlenM) {
-    t.m_tile = CG == 2 ? e.m >> 1 : e.m;
-    if (CG == 2 && half != 0) { if (e.m & 1) ++t.m_tile; else t.rows_valid = false; }   // no second tile: its loads repeat the first
+    band_decode(p.band > 0 ? p.band / CG : kBandM / CG, lin, num_m, p.num_n_tiles, t.m_tile, t.n_tile);
+    if (CG == 2) {
+      const int pair = p.pair_tiles[t.m_tile];       // first tile * 2 + (1 if the pair has a second tile)
+      t.m_tile = pair >> 1;
+      if (half != 0) { if (pair & 1) ++t.m_tile; else t.rows_valid = false; }   // no second tile: its loads repeat the first
+    }
+    t.expert = p.tile_id_to_expert[t.m_tile];
     t.row0 = t.m_tile * BM;
+    t.k_blocks = (p.K + BK - 1) / BK;
+    t.k_tail = 0;
   } else {
-    t.m_tile = e.m * CG + half;
-    if (CG == 2) t.rows_valid = t.m_tile * BM < (e.prob ? p.M_out2 : p.M_out);
-    t.row0 = e.row0;
+    int nm = p.num_m_tiles, nn = p.num_n_tiles, m_out = p.M_out;
+    const int first = p.num_experts * nm * nn;
+    if (lin >= first) { t.prob = 1; lin -= first; nm = p.num_m_tiles2; nn = p.num_n_tiles2; m_out = p.M_out2; }
+    const int per_e = nm * nn;
+    t.expert = lin / per_e;
+    band_decode(p.band > 0 ? p.band / CG : kBandM / CG, lin - t.expert * per_e, nm, nn, t.m_tile, t.n_tile);
+    if (CG == 2) { t.m_tile = t.m_tile * 2 + half; t.rows_valid = t.m_tile * BM < m_out; }
+    t.row0 = p.expert_pool_block_offset[t.expert] * BM;
+    const int len = p.expert_frequency[t.expert];
+    t.k_blocks = (len + BK - 1) / BK;
+    t.k_tail = len % BK;
   }
   return t;
 }
+
+// A queued VarlenK unit (decoded for the pair's first CTA) as it looks to CTA `half` of the pair.
 template <int CG>
-__device__ __forceinline__ TileCoord decode_tile(const GemmParams& p, int lin, int num_m, int half) {
-  return unit_coord<CG>(p, decode_unit<CG>(p, lin, num_m), half);
+__device__ __forceinline__ TileCoord unit_coord(const GemmParams& p, const TileEntry& e, int half) {
+  TileCoord t;
+  t.prob = e.prob; t.n_tile = e.n_tile; t.expert = e.expert; t.row0 = e.row0; t.k_blocks = e.k_blocks; t.k_tail = e.k_tail;
+  t.m_tile = e.m_tile + half;
+  t.rows_valid = CG == 1 || t.m_tile * BM < (e.prob ? p.M_out2 : p.M_out);
+  return t;
 }
 
 __device__ __forceinline__ void st_global_v4(void* p, uint32_t a, uint32_t b, uint32_t c, uint32_t d) {
@@ -215,7 +211,7 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
   // Tile feed.  Static: CTA b takes tiles b, b + stride, ...  Dynamic (VarlenK with a counter): tiles are claimed.  VarlenK units are
   // queued by the scheduler warp of the first CTA, in shared memory of both CTAs; otherwise every role decodes on its own.
   constexpr bool queued = A_MN;
-  const bool dyn = queued && p.tile_counter != nullptr;
+  const bool dyn = p.mode == kVarlenK && p.tile_counter != nullptr;
   const unsigned long long budget = p.wait_budget_ns;
   // Fused push, two ways of sharing the GPU.  Mixed (push_ctas == 0): every CTA multiplies and its extra warps push.
   // Dedicated (push_ctas > 0): the last push_ctas CTAs only push, with all their warps, and the others only multiply.
@@ -884,14 +880,17 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
           else lin = dyn ? atomicAdd(p.tile_counter, 1) : first_lin + it * lin_stride;
           const bool end = lin >= total_tiles || lin < 0;
           TileEntry e{};
-          if (end) e.lin = total_tiles;
-          else e = decode_unit<CG>(p, lin, num_m);
+          e.lin = end ? total_tiles : lin;
+          if (!end) {
+            const TileCoord t = decode_tile<CG>(p, lin, num_m, 0);
+            e = TileEntry{lin, t.m_tile, t.n_tile, t.expert, t.row0, t.k_blocks, t.k_tail, t.prob};
+          }
           TileEntry* q = &s_q[it % kTileQueue];
           *q = e;
           st_release_cta_shared(&s_q_head, it + 1);
           if (CG == 2) {
             const uint32_t peer = cluster_map(q, 1);
-            st_cluster_v4(peer, e.lin, e.m, e.n_tile, e.expert);
+            st_cluster_v4(peer, e.lin, e.m_tile, e.n_tile, e.expert);
             st_cluster_v4(peer + 16, e.row0, e.k_blocks, e.k_tail, e.prob);
             st_release_cluster(cluster_map(&s_q_head, 1), it + 1);
           }
