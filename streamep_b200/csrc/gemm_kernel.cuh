@@ -46,7 +46,7 @@ constexpr bool has_gate_warp(int epi) { return epi == kEpiSwiglu || epi == kEpiD
 // its expert's rows and queues the result for the other roles of both CTAs.  Operands arrive at the rate at which L2 delivers
 // them, so time that the producer spends on anything else is never made up for: a claim (an atomic, a copy to the other CTA, two
 // loads), and each store with release semantics, which waits for the copies in flight.  The other roles therefore report to
-// the scheduler with plain stores.  SM cycles of the MMA loop before and after: 32 experts of 512 rows, hidden 3072, ffn 768
+// the scheduler with plain stores (of units with products, see s_q).  SM cycles of the MMA loop before and after: 32 experts of 512 rows, hidden 3072, ffn 768
 // 412 -> 323 thousand; of 1250 rows, hidden 7168, ffn 2048 4130 -> 3775; 12 of 440, hidden 1000, ffn 520 48 -> 39; 8 of 6144 (few long
 // units) 785 -> 795.  The kernels over row tiles, whose order is static, lose by such a queue (Y of 32008 rows 171 -> 187).
 constexpr int base_warps(int epi, bool schedules) { return kGemmWarps + (schedules || has_gate_warp(epi) ? 1 : 0); }
@@ -197,7 +197,11 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
   __shared__ int s_gates_open;   // how many of this CTA's tiles have an open gate (-1: the gate warp gave up)
   __shared__ int s_tiles_done;   // tiles whose epilogue finished (read by the time stamps only)
   __shared__ uint64_t s_push_bar[32][2];   // push-only CTAs: two bulk-load barriers per warp
-  __shared__ TileEntry s_q[kTileQueue];    // the scheduler's queue ...
+  // The scheduler's queue.  It overwrites an entry once every role that reads it has reported so.  A unit with products: producers
+  // and MMA warp report with plain stores, since the epilogue, whose report is a release, comes after the copies and products
+  // that were issued from what they read.  A unit without any (an expert without rows) makes no role wait for another, so each
+  // reports with a release; a later plain store by the same thread to the same counter still carries it.
+  __shared__ TileEntry s_q[kTileQueue];
   __shared__ int s_q_head, s_q_tail;       // ... how many tiles were queued, how many the epilogue has finished
   __shared__ int s_q_read, s_q_prod;       // ... how many entries the MMA warp has read, how many the producer is (nearly) done with
   __shared__ int s_q_tail_peer, s_q_read_peer;   // (CG = 2, first CTA of a pair) the peer's epilogue / producer
@@ -335,8 +339,12 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
           lin = e.lin;
           t = unit_coord<CG>(p, e, half_of_pair);
           if (lin >= total_tiles) break;
-          if (CG == 2 && !leader) st_cluster(cluster_map(&s_q_read_peer, 0), it + 1);
-          if (leader && t.k_blocks == 0) st_volatile_shared(&s_q_prod, it + 1);
+          // (see s_q: only the report of a unit without products has to order the read of its entry)
+          if (CG == 2 && !leader) {
+            if (t.k_blocks == 0) st_release_cluster(cluster_map(&s_q_read_peer, 0), it + 1);
+            else st_cluster(cluster_map(&s_q_read_peer, 0), it + 1);
+          }
+          if (leader && t.k_blocks == 0) st_release_cta_shared(&s_q_prod, it + 1);
         } else {
           lin = first_lin + it * lin_stride;
           if (lin >= total_tiles || lin < 0) break;
@@ -439,7 +447,10 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
         const TileEntry e = s_q[it % kTileQueue];
         if (e.lin >= total_tiles) break;
         __syncwarp();
-        if (lane == 0) st_volatile_shared(&s_q_read, it + 1);
+        if (lane == 0) {
+          if (e.k_blocks == 0) st_release_cta_shared(&s_q_read, it + 1);
+          else st_volatile_shared(&s_q_read, it + 1);
+        }
         t = unit_coord<CG>(p, e, 0);
       } else {
         const int lin = first_lin + it * lin_stride;

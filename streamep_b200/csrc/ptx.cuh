@@ -216,7 +216,8 @@ __device__ __forceinline__ bool mbar_try_wait_cluster(uint64_t* bar, uint32_t pa
       : "=r"(ok) : "r"(smem_u32(bar)), "r"(parity) : "memory");
   return ok != 0;
 }
-// A progress counter that other warps poll; orders nothing (a release would make this thread wait for all it has in flight).
+// A progress counter that other warps poll.  By itself it orders nothing (a release would make this thread wait for all it has in
+// flight); after a release by this thread to the same counter, whoever acquires this value has what was released then.
 __device__ __forceinline__ void st_volatile_shared(int* p, int v) {
   asm volatile("st.volatile.shared::cta.s32 [%0], %1;" :: "r"(smem_u32(p)), "r"(v) : "memory");
 }
