@@ -818,13 +818,15 @@ cudaError_t launch_dispatch_push(const PushParams& p, int num_blocks, cudaStream
 // =============================================================================================
 // 16-byte loads in flight per lane and contributing rank, and threads of a block: one rank alone has no round trip over
 // NVLink to hide behind the other ranks' loads, so it takes a row in larger pieces and twice the warps (the caller's SM
-// budget sets the blocks).  4096 tokens, hidden 7168, 80 blocks, one rank: 84 -> 34 us.
-constexpr int pull_unroll(int ranks) { return ranks == 1 ? 8 : 2; }
+// budget sets the blocks).  4096 tokens, hidden 7168, 80 blocks, one rank: 84 -> 34 us.  With 8 loads a lane's first reduction
+// waits for all of them, so that width pays only where warps take several pieces; where every piece of 4 loads finds a warp
+// of its own, 4 are faster.  us at 4 / 8 loads, hidden 2048: 256 tokens 12.4 / 13.9, 1000 tokens (2000 pieces for 2560 warps)
+// 13.1 / 14.4, 4096 tokens 20.8 / 19.3; hidden 7168: 256 tokens (1792 pieces) 13.3 / 14.4, 1000 tokens 18.2 / 17.8.
+constexpr int kPullUnroll = 2, kPullUnrollLocal = 8, kPullUnrollLocalFew = 4;
 constexpr int combine_threads(int ranks) { return ranks == 1 ? 1024 : 512; }
 
-template <int NR>      // 1, or kMaxRanks for any number
+template <int NR, int U>      // NR: 1, or kMaxRanks for any number; U: see above
 __global__ void __launch_bounds__(combine_threads(NR), 1) combine_pull_kernel(const CombineParams p) {
-  constexpr int U = pull_unroll(NR);
   __shared__ const char* s_x[NR];
   __shared__ const long long* s_done[NR];
   __shared__ const float* s_w[NR];
@@ -945,8 +947,15 @@ __global__ void __launch_bounds__(combine_threads(NR), 1) combine_pull_kernel(co
 }
 
 void launch_combine_pull(const CombineParams& p, int num_blocks, cudaStream_t stream) {
-  if (p.num_ranks == 1) combine_pull_kernel<1><<<num_blocks, combine_threads(1), 0, stream>>>(p);
-  else combine_pull_kernel<kMaxRanks><<<num_blocks, combine_threads(kMaxRanks), 0, stream>>>(p);
+  if (p.num_ranks > 1) {
+    combine_pull_kernel<kMaxRanks, kPullUnroll><<<num_blocks, combine_threads(kMaxRanks), 0, stream>>>(p);
+    return;
+  }
+  const long long pieces = (p.hidden / 8 + 32 * kPullUnrollLocalFew - 1) / (32 * kPullUnrollLocalFew);
+  if (p.num_tokens * pieces <= static_cast<long long>(num_blocks) * (combine_threads(1) / 32))
+    combine_pull_kernel<1, kPullUnrollLocalFew><<<num_blocks, combine_threads(1), 0, stream>>>(p);
+  else
+    combine_pull_kernel<1, kPullUnrollLocal><<<num_blocks, combine_threads(1), 0, stream>>>(p);
 }
 
 // =============================================================================================
