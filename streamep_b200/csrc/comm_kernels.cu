@@ -612,12 +612,16 @@ __global__ void __launch_bounds__(kPushThreads, 1) dispatch_push_kernel(const Pu
 }
 
 // The push of a single rank: every pair of a token lands in this rank's pool, so a warp takes whole tokens, reads each row
-// once and stores it once per pair, where the general kernel reads a row per pair.  Bound by the pool's writes to HBM; the
-// caller's SM budget (80 blocks by default) asks for as many bytes in flight per SM as it can hold: 32 warps, 4 KB each.
-// 4096 tokens x 8 pairs, hidden 512, 80 blocks: 23 us.  Chunks of tokens are claimed, not dealt out by block: a
+// once and stores it once per pair, where the general kernel reads a row per pair.  Rows shorter than kBulkPushRow: a lane has at
+// most 4 vectors of one, so a warp keeps less than 2 KB in flight and 32 warps of each of the num_blocks SMs (80 unless the
+// caller sets another number) less than 64 KB.  Bound by that latency, not by HBM: 4096 tokens x 8 pairs, hidden 512, 80
+// blocks: 18.6 us (1.8 TB/s), 1000 tokens 9.4.  Chunks of tokens are claimed, not dealt out by block: a
 // block needs a whole SM, and a consumer that already waits for rows may hold the SM of a block that has not started yet.
 constexpr int kLocalPushThreads = 1024;
 constexpr int kLocalPushPairs = 16;     // pairs a warp copies between two releases of their tiles
+constexpr int kBulkPushRow = 2048;      // bytes; rows of this length and more go through dispatch_push_local_bulk_kernel
+constexpr int kLocalPushVecs = 4;       // 16-byte vectors a lane has of a row
+static_assert(kBulkPushRow <= 32 * kLocalPushVecs * 16, "a warp takes a row in one piece");
 
 __global__ void __launch_bounds__(kLocalPushThreads, 1) dispatch_push_local_kernel(const PushParams p) {
   __shared__ PushTargets tg;
@@ -640,7 +644,7 @@ __global__ void __launch_bounds__(kLocalPushThreads, 1) dispatch_push_local_kern
     for (int t = static_cast<int>(t0); t < t1; ++t) {
       const int slot = lane < K ? p.pair_slot[static_cast<size_t>(t) * K + lane] : -1;
       const char* src = static_cast<const char*>(p.x) + t * row_bytes;
-      for (int v0 = 0; v0 < vecs; v0 += 256) copy_row_piece<8>(src, tg.pool[0], nullptr, v0, vecs, K, slot, lane);
+      copy_row_piece<kLocalPushVecs>(src, tg.pool[0], nullptr, 0, vecs, K, slot, lane);
       const unsigned valid = __ballot_sync(0xffffffffu, slot >= 0);
       if (!p.is_grads && valid != 0) {
         const int r = p.send_recv_token[t];
@@ -681,7 +685,6 @@ __global__ void __launch_bounds__(kLocalPushThreads, 1) dispatch_push_local_kern
 // top-8, 4096 tokens 138 -> 121 (4.4 TB/s), 16384 tokens 468 -> 437, 1000 tokens 82 -> 39; top-2, 1000 tokens 72 -> 19; hidden 2048,
 // top-8, 4096 tokens 49 -> 46; hidden 1024, top-8 32 -> 31.  Shorter rows mean too many bulk stores: hidden 512, top-8, 16384 tokens 49
 // -> 55, 4096 tokens 23 -> 25; 256 35 -> 39, so those keep the kernel above.
-constexpr int kBulkPushRow = 2048;      // bytes
 constexpr int kBulkPushWarps = 6;
 constexpr int kBulkPushSlot = 16384;
 
