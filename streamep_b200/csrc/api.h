@@ -255,6 +255,7 @@ struct CombineParams {
   StatusBlock* status;
   unsigned long long wait_budget_ns;
 };
+int combine_piece_vectors(long long num_tokens, long long hidden, int num_blocks);    // one rank: 16-byte loads in flight per lane
 void launch_combine_pull(const CombineParams& p, int num_blocks, cudaStream_t stream);
 
 // ---------------------------------------------------------------------------------------------

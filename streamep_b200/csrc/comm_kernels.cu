@@ -951,13 +951,17 @@ __global__ void __launch_bounds__(combine_threads(NR), 1) combine_pull_kernel(co
   }
 }
 
+int combine_piece_vectors(long long num_tokens, long long hidden, int num_blocks) {
+  const long long pieces = (hidden / 8 + 32 * kPullUnrollLocalFew - 1) / (32 * kPullUnrollLocalFew);
+  return num_tokens * pieces <= static_cast<long long>(num_blocks) * (combine_threads(1) / 32) ? kPullUnrollLocalFew : kPullUnrollLocal;
+}
+
 void launch_combine_pull(const CombineParams& p, int num_blocks, cudaStream_t stream) {
   if (p.num_ranks > 1) {
     combine_pull_kernel<kMaxRanks, kPullUnroll><<<num_blocks, combine_threads(kMaxRanks), 0, stream>>>(p);
     return;
   }
-  const long long pieces = (p.hidden / 8 + 32 * kPullUnrollLocalFew - 1) / (32 * kPullUnrollLocalFew);
-  if (p.num_tokens * pieces <= static_cast<long long>(num_blocks) * (combine_threads(1) / 32))
+  if (combine_piece_vectors(p.num_tokens, p.hidden, num_blocks) == kPullUnrollLocalFew)
     combine_pull_kernel<1, kPullUnrollLocalFew><<<num_blocks, combine_threads(1), 0, stream>>>(p);
   else
     combine_pull_kernel<1, kPullUnrollLocal><<<num_blocks, combine_threads(1), 0, stream>>>(p);

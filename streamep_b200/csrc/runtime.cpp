@@ -2109,6 +2109,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.attr("MAX_EXPERTS") = kMaxExperts;
   m.def("is_sm100_compiled", [] { return true; });
   m.def("layer_widths", &Runtime::layer_widths);
+  m.def("combine_piece_vectors", &combine_piece_vectors);
   m.def("layer_bytes_hint", &ArenaSizeHint::layer_bytes);
 
   py::class_<ArenaProbe>(m, "ArenaProbe")

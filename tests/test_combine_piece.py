@@ -1,15 +1,11 @@
-"""The combine of one rank takes a row in pieces of 32 lanes x 4 vectors while every piece finds a warp of its own, and x 8 beyond: which
-kernel ran on both sides of that line, at row ends inside and on the edge of a piece, and its values (rows are moved: exact)."""
-import re
-
+"""The combine of one rank takes a row in pieces of 32 lanes x 4 vectors while every piece finds a warp of its own, and x 8 beyond: the rule
+(CPU), and the values on both sides of its line, at row ends inside and on the edge of a piece (rows are moved: exact)."""
 import pytest
 import torch
 
-pytestmark = pytest.mark.gpu
-DEV = "cuda"
+from streamep_b200 import _ext
 
-
-@pytest.mark.parametrize("T,H,blocks,vectors", [
+CASES = [
     (1, 8, 2, 4),
     (64, 1024, 2, 4),        # one piece a row, exactly as many as warps (2 blocks x 32)
     (65, 1024, 2, 8),        # one more: half of a wide piece
@@ -17,30 +13,32 @@ DEV = "cuda"
     (33, 2048, 2, 8),        # exactly one wide piece
     (40, 2056, 2, 8),        # ... and one vector more
     (21, 2056, 2, 4),        # three pieces, the last of one vector
-    (1000, 7168, None, 8),   # the default number of blocks
-    (300, 7168, None, 4),
-])
-def test_combine_piece(native, T, H, blocks, vectors):
-    from torch.profiler import ProfilerActivity, profile
+    (1000, 7168, 80, 8),     # the default number of blocks
+    (300, 7168, 80, 4),
+]
 
+
+@pytest.mark.parametrize("T,H,blocks,vectors", CASES)
+def test_combine_piece_rule(T, H, blocks, vectors):
+    assert _ext.load().combine_piece_vectors(T, H, blocks) == vectors
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("T,H,blocks,vectors", CASES)
+def test_combine_piece_values(native, T, H, blocks, vectors):
     from streamep_b200.models.moe_layer import make_buffer
     g = torch.Generator(device="cpu").manual_seed(T + H)
     E, K = 8, 2
-    x, rows = (torch.randn(T, H, generator=g).to(torch.bfloat16).to(DEV) for _ in range(2))
-    idx = torch.rand(T, E, generator=g).topk(K, dim=1).indices.to(DEV)
-    w = torch.rand(T, K, generator=g).to(DEV)
-    config = None if blocks is None else native.Config(blocks, 24, 256, 6, 128)
+    x, rows = (torch.randn(T, H, generator=g).to(torch.bfloat16).cuda() for _ in range(2))
+    idx = torch.rand(T, E, generator=g).topk(K, dim=1).indices.cuda()
+    w = torch.rand(T, K, generator=g).cuda()
     buf = make_buffer(None, T, H, K, E)
     _, h, _ = buf.dispatch(x, idx, w, None, E)
     sym = buf.alloc_symmetric([T, H], torch.bfloat16)
     sym.copy_(rows)
     h.y_done_per_token.fill_(1)
-    torch.cuda.synchronize()
     for _ in range(2):
-        with profile(activities=[ProfilerActivity.CUDA]) as prof:
-            out, _ = buf.combine(sym, h, combine_seq=1, config=config)
-            torch.cuda.synchronize()
+        out, _ = buf.combine(sym, h, combine_seq=1, config=native.Config(blocks, 24, 256, 6, 128))
+        torch.cuda.synchronize()
         buf.check_status()
         assert torch.equal(out, rows)
-    ran = [re.search(r"combine_pull_kernel<([^>]*)>", ev.name).group(1) for ev in prof.events() if "combine_pull_kernel" in ev.name]
-    assert [[int(n) for n in re.findall(r"\d+", r)] for r in ran] == [[1, vectors]], ran
