@@ -681,10 +681,11 @@ __global__ void __launch_bounds__(kLocalPushThreads, 1) dispatch_push_local_kern
 // The same push for rows of kBulkPushRow bytes and more, through the bulk-copy engine: a warp brings a chunk (whole tokens, or a
 // piece of a token whose row is longer) to shared memory and every pair leaves from there as one bulk store.  No register
 // holds a row, so the six warps of a block keep up to 2 x 16 KB each in flight where the loads and stores of 32 warps kept 4 KB.
-// Bound by the pool's writes to HBM once there are enough tokens, and by latency below.  us on 80 blocks, before -> now: hidden 7168,
-// top-8, 4096 tokens 138 -> 121 (4.4 TB/s), 16384 tokens 468 -> 437, 1000 tokens 82 -> 39; top-2, 1000 tokens 72 -> 19; hidden 2048,
-// top-8, 4096 tokens 49 -> 46; hidden 1024, top-8 32 -> 31.  Shorter rows mean too many bulk stores: hidden 512, top-8, 16384 tokens 49
-// -> 55, 4096 tokens 23 -> 25; 256 35 -> 39, so those keep the kernel above.
+// Bound by the pool's writes to HBM once there are enough tokens, and by latency below.  us of the kernel on 80 blocks, registers -> now:
+// hidden 7168, top-8, 4096 tokens 136 -> 112 (4.7 TB/s), 1000 tokens 72 -> 34; top-2, 1000 tokens 42 -> 14, 64 tokens 31 -> 6.3; hidden
+// 2048, top-8, 4096 tokens 44 -> 40; hidden 1024, top-8, 4096 tokens 26.8 -> 26.4, 64 tokens 8.2 -> 6.6, top-1, 64 tokens 16 -> 6.8,
+// one token 5.6 -> 5.4.  Many pairs of shorter rows mean too many bulk stores (us of the call, hidden 512, top-8, 16384 tokens 49 -> 55,
+// 4096 tokens 23 -> 25; 256 35 -> 39), so shorter rows keep the kernel above; few tokens of them were not compared.
 constexpr int kBulkPushWarps = 6;
 constexpr int kBulkPushSlot = 16384;
 

@@ -46,9 +46,12 @@ constexpr bool has_gate_warp(int epi) { return epi == kEpiSwiglu || epi == kEpiD
 // its expert's rows and queues the result for the other roles of both CTAs.  Operands arrive at the rate at which L2 delivers
 // them, so time that the producer spends on anything else is never made up for: a claim (an atomic, a copy to the other CTA, two
 // loads), and each store with release semantics, which waits for the copies in flight.  The other roles therefore report to
-// the scheduler with plain stores (of units with products, see s_q).  SM cycles of the MMA loop before and after: 32 experts of 512 rows, hidden 3072, ffn 768
-// 412 -> 323 thousand; of 1250 rows, hidden 7168, ffn 2048 4130 -> 3775; 12 of 440, hidden 1000, ffn 520 48 -> 39; 8 of 6144 (few long
-// units) 785 -> 795.  The kernels over row tiles, whose order is static, lose by such a queue (Y of 32008 rows 171 -> 187).
+// the scheduler with plain stores (of units with products, see s_q).  Before and after, with the wider stores below, thousand SM cycles of
+// the MMA loop and us of a launch on its own: 32 experts of 512 rows, hidden 3072, ffn 768 425 -> 319, 268 -> 221 us; of 1250 rows, hidden
+// 7168, ffn 2048 4170 -> 3745, 2850 -> 2716; 12 of 440, hidden 1000, ffn 520 48 -> 40, 42 -> 38; 4 of 4096, hidden and ffn 4096 1532 -> 1523,
+// 1156 -> 1160.  Long units beside narrow outputs lose: 8 of 6144, hidden 2048, ffn 1408 783 -> 792, 603 -> 613 us, hidden 4096 1564 -> 1580;
+// all pairs then wait alike for operands (322 -> 364 thousand cycles), where claims had set them apart.  The kernels over row tiles,
+// whose order is static, lose by such a queue (Y of 32008 rows 171 -> 187).
 constexpr int base_warps(int epi, bool schedules) { return kGemmWarps + (schedules || has_gate_warp(epi) ? 1 : 0); }
 // extra warps of the fused variants; the dSwiGLU epilogue keeps two preact segments in registers, so it gets fewer
 // (Y_bwd: 16 warps x 128 registers, A: 20 warps x 96 registers fill the register file)
@@ -56,7 +59,9 @@ constexpr int push_warps(int epi) { return epi == kEpiDswiglu ? 5 : 9; }
 constexpr int kMaxDevices = 64;  // per-device host-side tables (kernel attributes, no-alloc scratch address)
 constexpr int kTileQueue = 8;    // tiles the scheduler may be ahead of the epilogue
 // A claimed tile is work that no idle CTA can take any more, so the scheduler claims late: when the producer has this many
-// k-blocks of the tile before left to issue, about the time that a claim takes until its first operands can be requested.
+// k-blocks of the tile before left to issue, about the time that a claim takes until its first operands can be requested.  Thousand
+// cycles at 2, 5, 10, 20, 40: 32 experts of 512 rows 358, 323, 319, 319, 319; of 1250 rows 4010, 3780, 3745, 3746, 3747; 8 of 6144
+// 810, 796, 792, 792, 793.
 constexpr int kClaimAhead = 10;
 constexpr int kEpiWarps = 8;     // two threads per accumulator row: each takes half of the tile's columns
 
@@ -649,7 +654,7 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
           }
         }
         // Two chunks side by side leave as one store of 128-byte rows: half the rows for the TMA unit of stores of 32 columns each,
-        // two of which fitted the staging tile (weight gradients as above 323 -> 311 and 3775 -> 3705 thousand cycles).
+        // two of which fitted the staging tile (weight gradients as above 323 -> 319, 3775 -> 3745 and 795 -> 792 thousand cycles).
         if (EPI == kEpiStore) {
           if (((c - c_begin) & 1) == 0) {
             if (lane == 0) bulk_wait_read();
