@@ -40,7 +40,8 @@ def summarise(t: torch.Tensor) -> dict:
            "gate_wait_us_mean": us(t[:, 1].mean()), "gate_wait_us_max": us(t[:, 1].max()),
            "tiles_per_cta": float(t[:, 7].mean())}
     mma = t[:, 8] > 0
-    if bool(mma.any()):     # shares of the MMA-issuing thread's tile loop (SM cycles)
+    if bool(mma.any()):     # the MMA-issuing thread's tile loop in SM cycles, and shares of it
+        out["mma_loop_kcycles"] = float(t[mma, 8].mean()) / 1e3
         out["mma_wait_operands_frac"] = float((t[mma, 9] / t[mma, 8]).mean())
         out["mma_wait_accumulator_frac"] = float((t[mma, 10] / t[mma, 8]).mean())
     gated = t[:, 2] > 0
@@ -124,7 +125,8 @@ def sweep(args, buf, layers, routes, x, dy, rank, world, local):
 def main():
     ap = argparse.ArgumentParser()
     add_shape_args(ap)
-    ap.add_argument("--steps", type=int, default=6)
+    ap.add_argument("--steps", type=int, default=6, help="stamps are of the last one; hundreds of them show the clock that the power cap leaves")
+    ap.add_argument("--forward-only", action="store_true", help="the forward under torch.no_grad")
     ap.add_argument("--sweep", default="", help="comma-separated push settings 'pairs_per_chunk:push_warps:push_order[:head_pairs:head_chunks[:push_ctas[:bulk[:split_local]]]]' "
                     "(push_warps 0 = all); prints one line per setting and kind, averaged over ranks")
     args = ap.parse_args()
@@ -144,11 +146,12 @@ def main():
         if step == args.steps - 1:
             barrier(world, local)
             stamps = buf.runtime.set_kernel_timing(True)
-        h = x.detach().requires_grad_(True)
-        cur = h
-        for layer, r in zip(layers, routes):
-            cur = layer.experts(cur, *r)
-        cur.backward(dy)
+        with torch.set_grad_enabled(not args.forward_only):
+            cur = x.detach().requires_grad_(not args.forward_only)
+            for layer, r in zip(layers, routes):
+                cur = layer.experts(cur, *r)
+            if not args.forward_only:
+                cur.backward(dy)
         for layer in layers:
             layer.w1.grad = None
             layer.w2.grad = None
