@@ -47,9 +47,9 @@ constexpr bool has_gate_warp(int epi) { return epi == kEpiSwiglu || epi == kEpiD
 // them, so time that the producer spends on anything else is never made up for: a claim (an atomic, a copy to the other CTA, two
 // loads), and each store with release semantics, which waits for the copies in flight.  The other roles therefore report to
 // the scheduler with plain stores (of units with products, see s_q).  Before and after, with the wider stores below, thousand SM cycles of
-// the MMA loop and us of a launch on its own: 32 experts of 512 rows, hidden 3072, ffn 768 425 -> 319, 268 -> 221 us; of 1250 rows, hidden
-// 7168, ffn 2048 4170 -> 3745, 2850 -> 2716; 12 of 440, hidden 1000, ffn 520 48 -> 40, 42 -> 38; 4 of 4096, hidden and ffn 4096 1532 -> 1523,
-// 1156 -> 1160.  Long units beside narrow outputs lose: 8 of 6144, hidden 2048, ffn 1408 783 -> 792, 603 -> 613 us, hidden 4096 1564 -> 1580;
+// the MMA loop and us of a launch on its own: 32 experts of 512 rows, hidden 3072, ffn 768 425 -> 314, 268 -> 219 us; of 1250 rows, hidden
+// 7168, ffn 2048 4170 -> 3725, 2850 -> 2720; 12 of 440, hidden 1000, ffn 520 48 -> 38, 42 -> 37; 4 of 4096, hidden and ffn 4096 1532 -> 1523,
+// 1156 -> 1160.  Long units beside narrow outputs lose: 8 of 6144, hidden 2048, ffn 1408 783 -> 791, 603 -> 613 us, hidden 4096 1564 -> 1580;
 // all pairs then wait alike for operands (322 -> 364 thousand cycles), where claims had set them apart.  The kernels over row tiles,
 // whose order is static, lose by such a queue (Y of 32008 rows 171 -> 187).
 constexpr int base_warps(int epi, bool schedules) { return kGemmWarps + (schedules || has_gate_warp(epi) ? 1 : 0); }
@@ -60,8 +60,7 @@ constexpr int kMaxDevices = 64;  // per-device host-side tables (kernel attribut
 constexpr int kTileQueue = 8;    // tiles the scheduler may be ahead of the epilogue
 // A claimed tile is work that no idle CTA can take any more, so the scheduler claims late: when the producer has this many
 // k-blocks of the tile before left to issue, about the time that a claim takes until its first operands can be requested.  Thousand
-// cycles at 2, 5, 10, 20, 40: 32 experts of 512 rows 358, 323, 319, 319, 319; of 1250 rows 4010, 3780, 3745, 3746, 3747; 8 of 6144
-// 810, 796, 792, 792, 793.
+// cycles more than at 10 with 2, 5, 20 and 40: 32 experts of 512 rows 39, 4, 0, 0; of 1250 rows 265, 35, 1, 2; 8 of 6144 18, 4, 0, 1.
 constexpr int kClaimAhead = 10;
 constexpr int kEpiWarps = 8;     // two threads per accumulator row: each takes half of the tile's columns
 
@@ -205,7 +204,8 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
   // The scheduler's queue.  It overwrites an entry once every role that reads it has reported so.  A unit with products: producers
   // and MMA warp report with plain stores, since the epilogue, whose report is a release, comes after the copies and products
   // that were issued from what they read.  A unit without any (an expert without rows) makes no role wait for another, so each
-  // reports with a release; a later plain store by the same thread to the same counter still carries it.
+  // reports with a release, on a path of its own (chosen at each report, 32 experts of 512 rows took 319 thousand cycles for 314);
+  // a later plain store by the same thread to the same counter still carries it.
   __shared__ TileEntry s_q[kTileQueue];
   __shared__ int s_q_head, s_q_tail;       // ... how many tiles were queued, how many the epilogue has finished
   __shared__ int s_q_read, s_q_prod;       // ... how many entries the MMA warp has read, how many the producer is (nearly) done with
@@ -344,12 +344,12 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
           lin = e.lin;
           t = unit_coord<CG>(p, e, half_of_pair);
           if (lin >= total_tiles) break;
-          // (see s_q: only the report of a unit without products has to order the read of its entry)
-          if (CG == 2 && !leader) {
-            if (t.k_blocks == 0) st_release_cluster(cluster_map(&s_q_read_peer, 0), it + 1);
-            else st_cluster(cluster_map(&s_q_read_peer, 0), it + 1);
+          if (t.k_blocks == 0) {      // nothing to load (see s_q: only this report has to order the read of the entry)
+            if (CG == 2 && !leader) st_release_cluster(cluster_map(&s_q_read_peer, 0), it + 1);
+            else st_release_cta_shared(&s_q_prod, it + 1);
+            continue;
           }
-          if (leader && t.k_blocks == 0) st_release_cta_shared(&s_q_prod, it + 1);
+          if (CG == 2 && !leader) st_cluster(cluster_map(&s_q_read_peer, 0), it + 1);
         } else {
           lin = first_lin + it * lin_stride;
           if (lin >= total_tiles || lin < 0) break;
@@ -452,10 +452,11 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
         const TileEntry e = s_q[it % kTileQueue];
         if (e.lin >= total_tiles) break;
         __syncwarp();
-        if (lane == 0) {
-          if (e.k_blocks == 0) st_release_cta_shared(&s_q_read, it + 1);
-          else st_volatile_shared(&s_q_read, it + 1);
+        if (e.k_blocks == 0) {        // an expert without rows: the epilogue writes zeros on its own
+          if (lane == 0) st_release_cta_shared(&s_q_read, it + 1);
+          continue;
         }
+        if (lane == 0) st_volatile_shared(&s_q_read, it + 1);
         t = unit_coord<CG>(p, e, 0);
       } else {
         const int lin = first_lin + it * lin_stride;
@@ -463,7 +464,6 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
         t = decode_tile<CG>(p, lin, num_m, 0);
       }
       const uint32_t idesc = idesc0 | (static_cast<uint32_t>(tile_cols<BN>(t.prob ? p.N2 : p.N, t.n_tile * BN) >> 3) << 17);
-      if (t.k_blocks == 0) continue;   // empty expert: the epilogue writes zeros on its own
       // all 32 lanes wait; the outcome is made warp-uniform so that no lane leaves ahead of elect_one / __syncwarp
       long long c_acc = 0;
       if constexpr (stamp) c_acc = clock64();
@@ -654,7 +654,7 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
           }
         }
         // Two chunks side by side leave as one store of 128-byte rows: half the rows for the TMA unit of stores of 32 columns each,
-        // two of which fitted the staging tile (weight gradients as above 323 -> 319, 3775 -> 3745 and 795 -> 792 thousand cycles).
+        // two of which fitted the staging tile (weight gradients of 32 x 512, 32 x 1250 and 8 x 6144 rows: 4, 30 and 3 thousand cycles less).
         if (EPI == kEpiStore) {
           if (((c - c_begin) & 1) == 0) {
             if (lane == 0) bulk_wait_read();
