@@ -823,8 +823,8 @@ cudaError_t launch_dispatch_push(const PushParams& p, int num_blocks, cudaStream
 // Pull combine
 // =============================================================================================
 // 16-byte loads in flight per lane and contributing rank, and threads of a block: one rank alone has no round trip over
-// NVLink to hide behind the other ranks' loads, so it takes a row in larger pieces and twice the warps (the caller's SM
-// budget sets the blocks).  4096 tokens, hidden 7168, 80 blocks, one rank: 84 -> 34 us.  With 8 loads a lane's first reduction
+// NVLink to hide behind the other ranks' loads, so it takes a row in larger pieces and twice the warps (num_blocks
+// is the caller's, 80 by default).  4096 tokens, hidden 7168, 80 blocks, one rank: 84 -> 34 us.  With 8 loads a lane's first reduction
 // waits for all of them, so that width pays only where warps take several pieces; where every piece of 4 loads finds a warp
 // of its own, 4 are faster.  us at 4 / 8 loads, hidden 2048: 256 tokens 12.4 / 13.9, 1000 tokens (2000 pieces for 2560 warps)
 // 13.1 / 14.4, 4096 tokens 20.8 / 19.3; hidden 7168: 256 tokens (1792 pieces) 13.3 / 14.4, 1000 tokens 18.2 / 17.8.
